@@ -107,8 +107,9 @@ int grand_engine_kernel_times(GrandEngine *engine, void *stream, float *reset_ms
 
 /* Work statistics of the last device decode on `stream` (after
  * grand_engine_sync_status): out[0] shots settled by classification (empty
- * syndromes, one-position weight-1 matches), out[1] shots that took the
- * per-shot path, out[2] Jobs published, out[3] search tiles of those Jobs,
+ * syndromes, one-position weight-1 matches), out[1] shots that were searched one
+ * by one, out[2] shots with an iteration past the light budget (each of them a Job
+ * unless the guided search finished it), out[3] search tiles of the Jobs,
  * out[4] scratch words staged for them.  With GRAND_PROFILE=1 in the
  * environment when the engine was created, out[5..8] are the warp-nanoseconds
  * the decode kernel's warps spent classifying, on the per-shot path, on search

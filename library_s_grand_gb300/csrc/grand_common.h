@@ -52,9 +52,27 @@ constexpr int kMaxIters = 3;              // upstream threshold iterations (gran
 constexpr int kMaxSegsPerIter = 15;       // 3 phases x 5 weights
 constexpr int kMaxSegs = kMaxIters * kMaxSegsPerIter;
 
+// Codes the guided search takes (grand_guided_tables.h).
+constexpr int kGuidedMaxRows = 256;
+constexpr int kGuidedMaxCols = 1024;
+constexpr int kGuidedMaxColWeight = 7;
+constexpr int kGuidedMaxDegree = 64;
+constexpr int kGuidedF = 15;            // filter bits, log2 (4 KB)
+// Launch slots per chunk at most (one lane each), and the ballot words of a chunk's records
+// (8192 int32 entries): what keeps a warp's shared memory small enough that half of the
+// SM's storage stays L1 for the code tables.
+constexpr int kMaxChunk = 16;
+constexpr int kFastBallots = 256;
+constexpr int kGuidedItems = 344;       // partial sets a search holds (all its levels)
+constexpr unsigned kNoCol = 0xffffu;    // no column (adjacency padding, empty table slot)
+
 enum Family { kCss = 0, kDem = 1 };
 enum Variant { kUniform = 0, kProb = 1, kMl = 2 };
 enum InputKind { kInSyndromes = 0, kInErrors = 1, kInDetectors = 2 };
+// Who decodes a batch: the general kernel alone; the chunk kernel with the guided search,
+// then the general kernel for what that leaves in the slow queue; or the chunk
+// kernel alone (every search of every code fits, guided_closed).
+enum GuidedMode { kGuidedNone = 0, kGuidedFirst = 1, kGuidedAll = 2 };
 enum Branch { kBranchGpu = 0, kBranchCpu = 1 };
 
 // Status bits raised by the kernels (read back after every launch).
@@ -85,13 +103,14 @@ enum Counter {
   kCtrNextTile = 12,      // next search tile to draw (tiles numbered over all Jobs)
   kCtrScratchTop = 2,     // words of the scratch arena in use
   kCtrNextChunk = 3,      // next 32-slot classification chunk to draw
-  kCtrQueueReserved = 4,  // slow-queue entries reserved (each is written right after)
+  kCtrChunks = 4,         // (classification chunks finished << 32) | slow-queue entries
+                          // reserved (each is written right after)
   kCtrQueueHead = 5,      // slow-queue tickets drawn (a ticket past the reserved
                           // count is held until its entry exists or the batch ends)
-  kCtrChunksDone = 6,     // classification chunks finished
   kCtrSlowDone = 7,       // per-shot-path shots finished (their Jobs published)
   kCtrWarpsDone = 8,      // warps that left the kernel (the last advances the epoch)
-  kCtrSettled = 10,       // shots settled by classification (statistics)
+  kCtrSettled = 10,       // statistics: shots settled without a search (word 0), by the
+                          // guided search (1), and those of the latter past the light budget (2)
   kCtrProfSums = 11,      // profile (DevBatch::profile): warp-ns per kind of work, steps
   kCtrProfEnds = 13,      // profile: latest end per kind of work, ~(first warp start)
   kCtrProfMore = 14,      // profile: the Job publication's steps (kProfPub*)
@@ -156,6 +175,12 @@ struct DevCode {
   const uint32_t *solo_keys; // solo columns (nonzero, containing no other nonzero column)
   const int *solo_cols;      //   by sketch: open addressing, column -1 = empty slot
   uint32_t solo_mask;        //   (solo_cols nullptr: no table)
+  // guided search (grand_guided_tables.h); g_gs = 0: the code has none
+  int g_gs, g_deg, g_max_cw; // words per packed column, largest row degree, largest column weight
+  uint32_t g_tab_mask;
+  unsigned long long g_magic;  // ceil(2^32 / g_deg)
+  const uint32_t *g_rows, *g_cw, *g_cols, *g_filt, *g_tab;
+  const uint16_t *g_adj;
 };
 
 // One searched weight block of one threshold iteration.
@@ -250,7 +275,9 @@ struct DevBatch {
                                  // shot that needs the per-shot path
   unsigned *epoch;               // the workspace's launch epoch (kCtlAllocBytes layout)
   int profile;                   // 1: record per-phase times in the profile lines
-  int fast;                      // 1: settle shots 32 at a time first (empty syndromes, and
+  int chunk;                     // launch slots per chunk (1 .. kMaxChunk; 0: kMaxChunk)
+  int guided;                    // the chunk kernel runs first (enum GuidedMode)
+  int fast;                      // 1: settle shots a chunk at a time first (empty syndromes, and
                                  //    weight-1 matches of a one-position first iteration)
   int light_max_log2;            // light-path budget (candidates, log2)
   int tile_k;                    // prefixes per lane per colex tile (weights <= 2)

@@ -1,8 +1,10 @@
-// grand_decode.cuh -- the persistent decode kernel (sm_103a): one launch per batch.
+// grand_decode.cuh -- the persistent decode kernel (sm_103a): one launch per batch, for the
+// codes and shots the guided search does not take (grand_chunk.cuh).
 //
 // Every warp of the grid loops over whatever work the batch has left, in this
 // order of preference:
-//   1. classification chunks: 32 launch slots, one lane per shot; empty
+//   1. classification chunks (batches without a guided code; otherwise the chunk
+//      kernel ran before this one): launch slots, one lane per shot; empty
 //      syndromes and weight-1 matches of a one-position first iteration (a
 //      syndrome equal to a solo column, found by one sketch lookup) are settled
 //      there, the other shots go to the slow queue (classify_chunk);
@@ -30,6 +32,7 @@
 // every Job's tiles are drawn.  The last warp to leave advances the launch epoch.
 #pragma once
 
+#include "grand_chunk.cuh"
 #include "grand_search.cuh"
 #include "grand_triage.cuh"
 
@@ -56,13 +59,16 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
   // changes only once every warp of the launch has left)
   const unsigned epoch = *reinterpret_cast<volatile unsigned *>(b.epoch);
   const unsigned tag = epoch + 1u;
+  const int chunk = b.chunk > 0 ? b.chunk : kMaxChunk;
+  // after the chunk kernel only its slow queue is left
   const unsigned long long nchunks =
-      b.fast ? (unsigned long long)((b.num_shots + kChunkShots - 1) / kChunkShots) : 0ull;
+      b.fast && !b.guided ? ((unsigned long long)b.num_shots + (unsigned)chunk - 1ull) / (unsigned)chunk : 0ull;
   const unsigned long long nwarps = (unsigned long long)gridDim.x * kDecodeWarps;
   constexpr unsigned long long kTileMask = (1ull << 40) - 1ull;
   unsigned long long ticket = kNone;            // lane 0: a slow-queue ticket not yet used
   unsigned long long held_lo = 0, held_hi = 0;  // lane 0: tiles drawn and not yet run
   int polls = 0;
+  ChunkStats st{0, 0, 0};
   // profile (b.profile): lane 0 adds the time of each step to its kind's total
   unsigned long long *psum = ctr_ptr(b.counters, kCtrProfSums);
   unsigned long long *pend = ctr_ptr(b.counters, kCtrProfEnds);
@@ -84,7 +90,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
       // 2. the per-shot path
       if (step == kStepWait) {
         const unsigned long long reserved =
-            b.fast ? ld_ctr(b, kCtrQueueReserved) : (unsigned long long)b.num_shots;
+            b.fast ? ld_ctr(b, kCtrChunks) & 0xffffffffull : (unsigned long long)b.num_shots;
         if (ticket == kNone && ld_ctr(b, kCtrQueueHead) < reserved)
           ticket = atomicAdd(ctr_ptr(b.counters, kCtrQueueHead), 1ull);
         if (ticket != kNone && ticket < reserved) {
@@ -136,10 +142,10 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
         }
       }
       // 4. done, or wait for the warps still producing work
-      if (step == kStepWait && ld_ctr(b, kCtrChunksDone) >= nchunks) {
-        __threadfence();
+      const unsigned long long chunks = ld_ctr(b, kCtrChunks);
+      if (step == kStepWait && (chunks >> 32) >= nchunks) {
         const unsigned long long reserved =
-            b.fast ? ld_ctr(b, kCtrQueueReserved) : (unsigned long long)b.num_shots;
+            b.fast ? chunks & 0xffffffffull : (unsigned long long)b.num_shots;
         if (ld_ctr(b, kCtrSlowDone) >= reserved) {
           // every slow shot is done and its Job written (a ticket past the
           // entries will never be filled); once the front has passed every Job,
@@ -176,12 +182,8 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
     const unsigned long long t_step = b.profile ? global_ns() : 0ull;
     a0 = __shfl_sync(kFull, a0, 0);
     if (step == kStepChunk) {
-      classify_chunk<MLK>(b, (int)a0, A, tag);
+      classify_chunk<MLK, false>(b, (int)a0, chunk, *reinterpret_cast<FastArea *>(&A), nullptr, st, tag);
       cache.stage_lost();
-      if (lane == 0) {
-        __threadfence();
-        atomicAdd(ctr_ptr(b.counters, kCtrChunksDone), 1ull);
-      }
     } else if (step == kStepShot) {
       a1 = __shfl_sync(kFull, a1, 0);
       triage_shot<MLK>(b, (int)a0, A, plans[wib], tag, a1 != 0ull);
@@ -218,10 +220,24 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
   // the last warp to leave advances the epoch for the next launch
   __syncwarp();
   if (lane == 0) {
-    __threadfence();
+    add_stats(b, st);
     if (atomicAdd(ctr_ptr(b.counters, kCtrWarpsDone), 1ull) + 1ull == nwarps)
       *reinterpret_cast<volatile unsigned *>(b.epoch) = tag;
   }
 }
+
+#ifndef GRAND_HOST_EMULATION
+// The kernels of one batch: the chunk kernel (a warp per chunk) where codes of the batch
+// have a guided search, the decode kernel (grid blocks) unless that leaves it nothing.
+template <bool MLK>
+inline cudaError_t launch_kernels(const DevBatch &b, int grid, cudaStream_t s) {
+  if (b.guided) {
+    const int chunks = (b.num_shots - 1) / b.chunk + 1;
+    chunk_kernel<MLK><<<(chunks + kChunkWarps - 1) / kChunkWarps, kChunkWarps * 32, 0, s>>>(b);
+  }
+  if (b.guided != kGuidedAll) decode_kernel<MLK><<<grid, kDecodeWarps * 32, 0, s>>>(b);
+  return cudaGetLastError();
+}
+#endif
 
 }  // namespace grand

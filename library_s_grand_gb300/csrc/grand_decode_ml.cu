@@ -7,8 +7,7 @@ namespace grand {
 
 #ifndef GRAND_HOST_EMULATION
 cudaError_t launch_decode_ml(const DevBatch &b, int grid, cudaStream_t s) {
-  decode_kernel<true><<<grid, kDecodeWarps * 32, 0, s>>>(b);
-  return cudaGetLastError();
+  return launch_kernels<true>(b, grid, s);
 }
 
 cudaError_t decode_occupancy_ml(int *blocks_per_sm) {

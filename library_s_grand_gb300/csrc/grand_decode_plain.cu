@@ -10,10 +10,11 @@ namespace grand {
 cudaError_t launch_decode_ml(const DevBatch &b, int grid, cudaStream_t s);
 cudaError_t decode_occupancy_ml(int *blocks_per_sm);
 
+int chunk_warps_per_sm() { return kChunkMinBlocks * kChunkWarps; }
+
 cudaError_t launch_decode(const DevBatch &b, int grid, cudaStream_t s) {
   if (b.has_ml) return launch_decode_ml(b, grid, s);
-  decode_kernel<false><<<grid, kDecodeWarps * 32, 0, s>>>(b);
-  return cudaGetLastError();
+  return launch_kernels<false>(b, grid, s);
 }
 
 // Resident blocks per SM both builds reach (the grid is sized for the smaller).

@@ -273,7 +273,7 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   b.profile = e->tn.profile;
   b.light_max_log2 = e->tn.light_max_log2;
   b.tile_k = e->tn.tile_k;
-  for (const DevCode &c : e->codes) b.has_ml |= c.variant == kMl;
+  plan_batch(b, e->codes.data(), (int)e->codes.size(), e->ctx->sm_count, e->tn);
   if (!use_graph) {
     cudaEventRecord(slot->ev[0], s);
     r = launch_pipeline(e->ctx, b, e->tn, s, slot->ev[1]);
@@ -336,7 +336,7 @@ int grand_engine_sync_status(GrandEngine *e, void *stream) {
     set_error("grand: an active-position set exceeded GRAND_MAX_TAM=%d", kMaxTam);
     return GRAND_ERR_LIMIT;
   }
-  if (st & kStatusCasLimit) return GRAND_ERR_CUDA;
+  if (st & (kStatusCasLimit | kStatusWaitLimit)) return GRAND_ERR_CUDA;
   return 0;
 }
 
@@ -349,8 +349,8 @@ int grand_engine_launch_stats(GrandEngine *e, void *stream, long long *out) {
   if (cudaMemcpy(c.data(), it->second->d_small, kCtlBytes, cudaMemcpyDeviceToHost) != cudaSuccess)
     return GRAND_ERR_CUDA;
   out[0] = (long long)c[kCtrSettled * kCtrStride];
-  out[1] = (long long)c[kCtrSlowDone * kCtrStride];
-  out[2] = (long long)(c[kCtrJobs * kCtrStride] >> 40);
+  out[1] = (long long)(c[kCtrSlowDone * kCtrStride] + c[kCtrSettled * kCtrStride + 1]);
+  out[2] = (long long)((c[kCtrJobs * kCtrStride] >> 40) + c[kCtrSettled * kCtrStride + 2]);
   out[3] = (long long)(c[kCtrJobs * kCtrStride] & ((1ull << 40) - 1ull));
   out[4] = (long long)c[kCtrScratchTop * kCtrStride];
   // phase profile (GRAND_PROFILE=1): times in ns from the first warp's start

@@ -9,12 +9,14 @@
 #include <vector>
 
 #include "grand_common.h"
+#include "grand_guided_tables.h"
 
 namespace grand {
 
 // Kernel launchers (grand_decode_plain.cu, grand_decode_ml.cu, grand_sample.cu).
 cudaError_t launch_decode(const DevBatch &b, int grid, cudaStream_t s);
 cudaError_t decode_occupancy(int *blocks_per_sm);
+int chunk_warps_per_sm();  // resident warps of the chunk kernel the launch plan counts on
 cudaError_t launch_sample(const DevCode &cd, const float *d_p, unsigned long long seed,
                           unsigned long long first_shot, int num_shots, int *d_records,
                           int sm_count, cudaStream_t s);
@@ -38,6 +40,8 @@ struct CodeTables {
   uint32_t *solo_keys = nullptr;  // solo-column table (grand_solo.h): sketches
   int *solo_cols = nullptr;        //   and columns per slot (-1: empty)
   uint32_t solo_mask = 0;
+  GuidedTables guided;        // guided-search tables (grand_guided_tables.h): layout,
+  uint32_t *d_guided = nullptr;  //   and their device copy (nullptr: none)
   std::vector<int> key;  // exact content the tables were built from
   size_t bytes = 0;
   ~CodeTables();
@@ -165,6 +169,10 @@ Tuning &tuning();  // process defaults (GRAND_LIGHT_LOG2, GRAND_TILE_K, GRAND_SE
 // Runs the batch; returns 0 or a GRAND_ERR_* code.
 int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming *timing,
               const Tuning *tn = nullptr);
+
+// Which kernels decode the batch, and its chunks: b.has_ml, b.guided, b.chunk, from its
+// codes, b.num_shots and b.shot_map.
+void plan_batch(DevBatch &b, const DevCode *codes, int ncodes, int sm_count, const Tuning &tn);
 
 // Enqueue one decoding launch (control-word reset, decode kernel) on s.
 cudaError_t launch_pipeline(const Context *ctx, const DevBatch &b, const Tuning &tn,

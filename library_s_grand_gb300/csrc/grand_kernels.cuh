@@ -19,9 +19,6 @@ constexpr int kLightWords = kLightTam * 8;      // its staged column words (nwp 
 // end (the rest of the warp's area holds the syndrome and the degeneracy delta)
 constexpr int kWarpStage = 2720;
 constexpr int kTilesPerFetch = 16;  // most tiles a search warp draws at once
-// Launch slots per classification chunk (one lane each): fewer than 32 spreads a
-// batch's classification over more warps, so it ends sooner.
-constexpr int kChunkShots = 32;
 constexpr int kRunKKLight = 4;  // prefixes per lane in a run tile of the triage warp's light search
 
 // Per-warp shared memory of the decode kernel.  A warp does one kind of work at
@@ -73,6 +70,16 @@ __device__ __forceinline__ void nap(int polls) {
 
 __device__ __forceinline__ unsigned long long ld_ctr(const DevBatch &b, int ctr) {
   return *reinterpret_cast<volatile unsigned long long *>(ctr_ptr(b.counters, ctr));
+}
+
+// A code's descriptor into the warp's shared copy, one round trip for the whole of it.
+__device__ __forceinline__ void load_code(DevCode &dst, const DevCode *src) {
+  static_assert(sizeof(DevCode) % 8 == 0, "whole words");
+  __syncwarp();  // every lane is done with the code before
+  for (int i = threadIdx.x & 31; i < (int)(sizeof(DevCode) / 8); i += 32)
+    reinterpret_cast<unsigned long long *>(&dst)[i] =
+        __ldg(reinterpret_cast<const unsigned long long *>(src) + i);
+  __syncwarp();
 }
 
 // Profile (DevBatch::profile): lane 0 adds the time since t0 to profile sums

@@ -183,7 +183,7 @@ cudaError_t start_slot(GrandServer *S, SrvSlot *sl) {
   b.fast = e->tn.fast;
   b.light_max_log2 = e->tn.light_max_log2;
   b.tile_k = e->tn.tile_k;
-  for (const DevCode &c : e->codes) b.has_ml |= c.variant == kMl;
+  plan_batch(b, e->codes.data(), (int)e->codes.size(), e->ctx->sm_count, e->tn);
   // each slot's persistent grid takes its share of the resident blocks, so the
   // slots' kernels are resident together and their batches overlap on the GPU
   Tuning tn = e->tn;

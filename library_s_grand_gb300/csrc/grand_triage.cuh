@@ -1,13 +1,6 @@
 // grand_triage.cuh -- the per-shot work of a decoding launch (sm_103a), run by
 // the warps of the persistent decode kernel (grand_decode.cuh).
 //
-// classify_chunk (kChunkShots launch slots, one lane per shot)
-//   packs the 32 shots' records with coalesced ballots, forms each syndrome and
-//   settles the common shots outright: an empty syndrome (grand_decoder.cu:1223-1241),
-//   and a first threshold iteration with one active position whose column equals
-//   the syndrome (weight-1 match, 1 candidate tested).  The others go to the slow
-//   queue.
-//
 // triage_shot (one warp per shot)
 //   packs the shot's record into bits, forms the syndrome, computes the
 //   flagged-check count of every column (popc(col & s), upstream
@@ -870,424 +863,6 @@ __device__ void triage_shot(const DevBatch &b, int slot, WarpArea &A, PlanState 
     prof_lap(b, kProfPubReady, tq, kCtrProfMore);
     prof_lap(b, kProfShotPublish, tp);
   }
-}
-
-// ---------------------------------------------------------------------------
-// Classification of 32 launch slots, one lane per shot.
-// ---------------------------------------------------------------------------
-constexpr int kFastWords = 4;       // syndrome / logical words a lane keeps (R, n_logicos <= 128)
-constexpr int kFastErrWords = 16;   // error-record words a lane walks (m <= 512)
-constexpr int kFastBallots = 512;   // ballot words of a chunk's records (16384 int32 entries)
-constexpr int kFastLogBallots = 128;  // ballot words of a chunk's separate logical entries
-
-// classify_chunk's part of the WarpArea.
-struct FastArea {
-  uint32_t bits[kFastBallots + 1];      // bit e: entry e of the chunk's records (flat)
-  uint32_t lbits[kFastLogBallots + 1];  // the same for DEM logicals kept in their own array
-  uint32_t res[32][18];                 // result words, one row per lane
-};
-static_assert(sizeof(FastArea) <= sizeof(WarpArea), "FastArea must fit the warp's area");
-
-// Bits b0..b7 of x moved to bits 0, 4, .., 28.
-__device__ __forceinline__ uint32_t spread4(uint32_t x) {
-  x &= 0xffu;
-  x = (x | (x << 12)) & 0x000F000Fu;
-  x = (x | (x << 6)) & 0x03030303u;
-  x = (x | (x << 3)) & 0x11111111u;
-  return x;
-}
-
-// bits[k] = the nonzero flags of p[32k .. 32k + 31] for the n entries at p (bits
-// past n are 0); bits[ceil(n/32)] = 0.  The entries are read once and kept out
-// of L1 (the per-shot path may read them again from L2).  With p 16-byte
-// aligned, lanes read four entries at a time, eight 16-byte loads each in
-// flight (records read in place from host memory need the bytes in flight): a
-// row of 32 lanes is 128 entries, and its four words are four ballots (ballot
-// c holds entry 4l + c in bit l) interleaved by four lanes.  Otherwise, and for
-// the last n % 128 entries, one entry per lane per ballot.
-__device__ __forceinline__ void flat_ballots(const int *p, int n, uint32_t *bits) {
-  const int lane = threadIdx.x & 31;
-  const int nwords = (n + 31) >> 5;
-  int done = 0;  // entries handled by the 16-byte path (a multiple of 128)
-  if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0u) {
-    const int4 *p4 = reinterpret_cast<const int4 *>(p);
-    const int rows = n >> 7;  // full rows of 128 entries
-    for (int r0 = 0; r0 < rows; r0 += 8) {
-      int4 v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        v[u] = r0 + u < rows ? __ldcg(p4 + (r0 + u) * 32 + lane) : make_int4(0, 0, 0, 0);
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (r0 + u < rows) {
-          const uint32_t b0 = __ballot_sync(kFull, v[u].x != 0);
-          const uint32_t b1 = __ballot_sync(kFull, v[u].y != 0);
-          const uint32_t b2 = __ballot_sync(kFull, v[u].z != 0);
-          const uint32_t b3 = __ballot_sync(kFull, v[u].w != 0);
-          if (lane < 4) {
-            const int sh = 8 * lane;
-            bits[(r0 + u) * 4 + lane] = spread4(b0 >> sh) | (spread4(b1 >> sh) << 1) |
-                                        (spread4(b2 >> sh) << 2) | (spread4(b3 >> sh) << 3);
-          }
-        }
-      }
-    }
-    done = rows << 7;
-  }
-  for (int k0 = done >> 5; k0 < nwords; k0 += 16) {
-    int v[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int e = (k0 + u) * 32 + lane;
-      v[u] = e < n ? __ldcg(p + e) : 0;
-    }
-    uint32_t mine = 0u;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const uint32_t w = __ballot_sync(kFull, v[u] != 0);
-      mine = lane == u ? w : mine;
-    }
-    if (lane < 16 && k0 + lane < nwords) bits[k0 + lane] = mine;
-  }
-  if (lane == 0) bits[nwords] = 0u;
-}
-
-// Word q of the nbits-entry bit vector that starts at entry `off` of a flat
-// ballot array (entries past nbits masked off).
-__device__ __forceinline__ uint32_t flat_word(const uint32_t *bits, int off, int q, int nbits) {
-  const int e = off + 32 * q;
-  uint32_t w = __funnelshift_r(bits[e >> 5], bits[(e >> 5) + 1], e & 31);
-  const int rem = nbits - 32 * q;
-  if (rem < 32) w &= (1u << rem) - 1u;
-  return w;
-}
-
-// Upstream's planner (grand_decoder.cu:1284-1296, 1550-1554, 754-786) for a first
-// threshold iteration with one active position: is it searched, and with a
-// weight-1 block (its only candidate)?  *gpu: the branch upstream takes.
-__device__ __forceinline__ bool one_position_searched(const DevCode &cd, bool *gpu) {
-  if (cd.family == kDem && 1 > cd.cap) return false;  // the cap replaces the set by an empty one
-  const bool g = (1 > cd.thr && 1 <= cd.cap && cd.mode == 1) || cd.mode == 0;
-  const bool c = !g && ((1 <= cd.thr && cd.mode == 1) || cd.mode == -1);
-  if (!g && !c) return false;
-  *gpu = g;
-  if (cd.variant != kProb) return true;  // weights 1..min(W, 1)
-  int mi = cd.n_masks - 1;
-  for (int q = 0; q < cd.n_masks; ++q)
-    if (1 <= cd.mask_tam_upper[q]) {
-      mi = q;
-      break;
-    }
-  for (int k = 0; k < cd.num_phases; ++k)
-    if (cd.mask_order[mi][k] == 0) return true;  // phase 0 lists weight 1
-  return false;
-}
-
-// Settles the shots of launch slots kChunkShots*chunk + [0, kChunkShots) that need no search
-// -- an empty syndrome, or a first iteration with one active position whose
-// column equals the syndrome -- and appends the others to the slow queue.  The
-// results are exactly those of triage_shot: the one position is the only
-// candidate of the iteration (found at weight 1, rank 0; one candidate counted
-// on either branch, hibrido 0 / -1), and its active set is the set of nonzero
-// columns contained in the syndrome (flagged-check count = column weight, for
-// 0/1 matrices regular or not), found through the columns grouped by their
-// lowest row.  Shots the lanes cannot settle here (ML codes, supplied errors
-// that differ from the match, wide codes, records that are not back to back)
-// take the slow path: they are appended to the slow queue with tag (the launch
-// epoch + 1).
-template <bool MLK>
-__device__ void classify_chunk(const DevBatch &b, int chunk, WarpArea &A, unsigned tag) {
-  FastArea &F = *reinterpret_cast<FastArea *>(&A);
-  const int lane = threadIdx.x & 31;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  const int slot = chunk * kChunkShots + lane;
-  const bool valid = lane < kChunkShots && slot < b.num_shots;
-  const unsigned long long t_start = global_ns();
-  unsigned long long tp = b.profile ? t_start : 0ull;
-  const int shot = valid ? (b.shot_map ? b.shot_map[slot] : slot) : 0;
-  const int ci = (valid && b.shot_code) ? b.shot_code[shot] : 0;
-  const DevCode &cd = b.codes[ci];
-  const bool errs = cd.input_kind == kInErrors;
-  const bool dem = cd.family == kDem;
-  const int nbits = errs ? cd.m : cd.R;       // entries of the record's leading bit vector
-  const int nwords = (nbits + 31) >> 5;
-  bool ok = valid && cd.nw <= kFastWords && (!errs || nwords <= kFastErrWords) &&
-            (!dem || cd.nlw <= kFastWords);
-  const long long rbase = valid ? (b.in_off ? b.in_off[shot] : (long long)shot * cd.rec_len) : 0;
-
-  uint32_t s[kFastWords] = {0u, 0u, 0u, 0u};
-  uint32_t lg[kFastWords] = {0u, 0u, 0u, 0u};
-  int ow = 0, epos = -1;
-
-  // ---- the records: int32 entries through coalesced ballots over runs of
-  //      back-to-back records, bit-packed words read directly ------------------
-  const bool packed = cd.packed != 0;
-  bool extracted = false;  // this lane's record bits are in rec_cache
-  const bool any_int = __any_sync(kFull, valid && !packed);
-  if (any_int) {
-    const int rlen = (dem && !b.in_log) ? cd.R + cd.n_logicos : nbits;
-    // this lane's bits from a ballot array over the entries starting at `first`
-    // (and, for DEM logicals kept in their own array, from `lfirst` there)
-    // (and its words into rec_cache, for the per-shot path if the shot goes there)
-    uint32_t *cache = b.rec_cache ? b.rec_cache + (size_t)slot * kRecCacheWords : nullptr;
-    auto extract = [&](long long first, long long lfirst, long long lbase) {
-      const int off = (int)(rbase - first);
-      if (errs) {
-        for (int q = 0; q < nwords; ++q) {
-          uint32_t w = flat_word(F.bits, off, q, nbits);
-          if (cache) cache[q] = w;
-          ow += __popc(w);
-          while (w) {
-            const int c = q * 32 + __ffs(w) - 1;
-            w &= w - 1u;
-            epos = c;
-#pragma unroll
-            for (int k = 0; k < kFastWords; ++k)
-              if (k < cd.nw) s[k] ^= __ldg(cd.cols + (size_t)c * cd.nwp + k);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < kFastWords; ++k)
-          if (k < cd.nw) {
-            s[k] = flat_word(F.bits, off, k, cd.R);
-            if (cache) cache[k] = s[k];
-          }
-        if (dem) {
-#pragma unroll
-          for (int k = 0; k < kFastWords; ++k)
-            if (k < cd.nlw) {
-              lg[k] = b.in_log ? flat_word(F.lbits, (int)(lbase - lfirst), k, cd.n_logicos)
-                               : flat_word(F.bits, off + cd.R, k, cd.n_logicos);
-              if (cache) cache[cd.nw + k] = lg[k];
-            }
-        }
-      }
-      extracted = cache != nullptr;
-    };
-    const bool sep_log = dem && b.in_log && valid;
-    if (__any_sync(kFull, sep_log)) {
-      // DEM logicals in their own array: both arrays back to back over the chunk
-      const long long nb = __shfl_down_sync(kFull, rbase, 1);
-      const bool nv = __shfl_down_sync(kFull, valid ? 1 : 0, 1) != 0;
-      const bool joined = !valid || lane == 31 || !nv || nb == rbase + rlen;
-      const long long first = __shfl_sync(kFull, rbase, 0);
-      long long end = valid ? rbase + rlen : first;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const long long u = __shfl_xor_sync(kFull, end, o);
-        end = u > end ? u : end;
-      }
-      bool flat = __all_sync(kFull, joined && !(valid && packed)) && end - first <= 32ll * kFastBallots;
-      const long long lbase = sep_log ? (long long)shot * cd.n_logicos : 0;
-      const long long lnb = __shfl_down_sync(kFull, lbase, 1);
-      const bool ljoined = !valid || lane == 31 || !nv || lnb == lbase + cd.n_logicos;
-      const long long lfirst = __shfl_sync(kFull, lbase, 0);
-      long long lend = valid ? lbase + cd.n_logicos : lfirst;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const long long u = __shfl_xor_sync(kFull, lend, o);
-        lend = u > lend ? u : lend;
-      }
-      flat = flat && __all_sync(kFull, ljoined && sep_log == (valid && dem)) &&
-             lend - lfirst <= 32ll * kFastLogBallots;
-      if (flat) {
-        flat_ballots(b.in + first, (int)(end - first), F.bits);
-        flat_ballots(b.in_log + lfirst, (int)(lend - lfirst), F.lbits);
-        __syncwarp();
-        if (ok) extract(first, lfirst, lbase);
-      } else {
-        ok = ok && packed;  // records that are not back to back: slow path
-      }
-    } else {
-      // Runs of consecutive lanes whose int32 records lie back to back (one run
-      // for a batch packed in slot order; a few where requests' records sit in
-      // separate buffers): each run's entries through one pass of ballots.
-      const bool mine = valid && !packed;
-      const long long pend = __shfl_up_sync(kFull, rbase + rlen, 1);
-      const bool pint = __shfl_up_sync(kFull, mine ? 1 : 0, 1) != 0;
-      const unsigned members_all = __ballot_sync(kFull, mine);
-      unsigned starts = __ballot_sync(kFull, mine && (lane == 0 || !pint || pend != rbase));
-      while (starts) {
-        const int l0 = __ffs(starts) - 1;
-        starts &= starts - 1u;
-        const int lnext = starts ? __ffs(starts) - 1 : 32;
-        const unsigned span = (lnext == 32 ? kFull : ((1u << lnext) - 1u)) & ~((1u << l0) - 1u);
-        const unsigned members = members_all & span;  // l0 .. the run's last lane, no gaps
-        const int llast = 31 - __clz(members);
-        const long long first = __shfl_sync(kFull, rbase, l0);
-        const long long end = __shfl_sync(kFull, rbase + rlen, llast);
-        const bool in_run = (members >> lane) & 1u;
-        if (end - first > 32ll * kFastBallots) {
-          if (in_run) ok = false;  // longer than the chunk's ballot area: slow path
-          continue;
-        }
-        flat_ballots(b.in + first, (int)(end - first), F.bits);
-        __syncwarp();
-        if (in_run && ok) extract(first, 0, 0);
-        __syncwarp();  // every lane has read the run's bits before the next run's
-      }
-    }
-  }
-  if (ok && packed) {
-    const uint32_t *rw = reinterpret_cast<const uint32_t *>(b.in) + rbase;
-    if (errs) {
-      for (int q = 0; q < nwords; ++q) {
-        uint32_t w = __ldcg(rw + q);
-        if (q == nwords - 1 && (nbits & 31)) w &= (1u << (nbits & 31)) - 1u;
-        ow += __popc(w);
-        while (w) {
-          const int c = q * 32 + __ffs(w) - 1;
-          w &= w - 1u;
-          epos = c;
-#pragma unroll
-          for (int k = 0; k < kFastWords; ++k)
-            if (k < cd.nw) s[k] ^= __ldg(cd.cols + (size_t)c * cd.nwp + k);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < kFastWords; ++k)
-        if (k < cd.nw) {
-          uint32_t w = __ldcg(rw + k);
-          if (k == cd.nw - 1 && (cd.R & 31)) w &= (1u << (cd.R & 31)) - 1u;
-          s[k] = w;
-        }
-      if (dem) {
-        const uint32_t *lw = b.in_log ? reinterpret_cast<const uint32_t *>(b.in_log) + (size_t)shot * cd.nlw
-                                      : rw + cd.nw;
-#pragma unroll
-        for (int k = 0; k < kFastWords; ++k)
-          if (k < cd.nlw) {
-            uint32_t w = __ldcg(lw + k);
-            if (k == cd.nlw - 1 && (cd.n_logicos & 31)) w &= (1u << (cd.n_logicos & 31)) - 1u;
-            lg[k] = w;
-          }
-      }
-    }
-  }
-  if (!errs) ow = 0;
-  tp = prof_lap(b, kProfChunkRead, tp);
-
-  // ---- settle: empty syndrome, or a one-position first iteration matched ----
-  const bool empty = ok && (s[0] | s[1] | s[2] | s[3]) == 0u;
-  bool found = false, gpu = false;
-  int pos = -1, deg = 0, iseq = 0;
-  if (ok && !empty && cd.variant != kMl && cd.solo_cols && cd.binary && cd.max_soma >= 1 &&
-      one_position_searched(cd, &gpu)) {
-    // the first iteration's active set is the nonzero columns contained in s:
-    // it is one column whose only candidate matches exactly when s equals a
-    // solo column, found by s's sketch in the solo table
-    uint32_t hs = 0u;
-#pragma unroll
-    for (int q = 0; q < kFastWords; ++q)
-      for (uint32_t rows = q < cd.nw ? s[q] : 0u; rows; rows &= rows - 1u)
-        hs ^= row_hash(q * 32 + __ffs(rows) - 1);
-    uint32_t i = hs & cd.solo_mask;
-    for (uint32_t probe = 0; probe <= cd.solo_mask && !found; ++probe) {
-      const int c = __ldg(cd.solo_cols + i);
-      if (c < 0) break;
-      if (__ldg(cd.solo_keys + i) == hs) {
-        bool eq = true;
-#pragma unroll
-        for (int k = 0; k < kFastWords; ++k)
-          if (k < cd.nw) eq = eq && __ldg(cd.cols + (size_t)c * cd.nwp + k) == s[k];
-        if (eq) {
-          found = true;
-          pos = c;
-        }
-      }
-      i = (i + 1u) & cd.solo_mask;
-    }
-    if (found) {
-      if (!dem && errs) {
-        iseq = (ow == 1 && epos == pos) ? 1 : 0;
-        deg = 1;
-        found = iseq != 0;  // a different supplied error needs the degeneracy test
-      } else if (dem) {
-        deg = 1;
-#pragma unroll
-        for (int k = 0; k < kFastWords; ++k)
-          if (k < cd.nlw && __ldg(cd.lcols + (size_t)pos * cd.nlw + k) != lg[k]) deg = 0;
-      }
-    }
-  }
-  const bool done = empty || found;
-  if (!found) pos = -1;
-  tp = prof_lap(b, kProfChunkTest, tp);
-
-  // ---- results of the settled shots ----------------------------------------
-  if (done) {
-    const unsigned long long now = global_ns();
-    uint32_t *r = F.res[lane];
-#pragma unroll
-    for (int w = 0; w < 18; ++w) r[w] = 0u;
-    r[2] = (uint32_t)ow;
-    if (empty) {
-      r[8] = (uint32_t)-2;
-    } else {
-      const unsigned long long half = t_start + (now - t_start) / 2;  // counts ~ half the time
-      const double t_sum = 1e-6 * (double)(half - t_start);
-      const double t_search = 1e-6 * (double)(now - half);
-      const double t_all = 1e-6 * (double)(now - t_start);
-      r[0] = 1u;
-      r[1] = 1u;
-      r[3] = (uint32_t)deg;
-      r[4] = (uint32_t)iseq;
-      r[5] = 1u;
-      r[6] = 1u;
-      r[8] = gpu ? 0u : (uint32_t)-1;
-      r[9] = 1u;
-      const unsigned long long a = (unsigned long long)__double_as_longlong(t_sum);
-      const unsigned long long bb = (unsigned long long)__double_as_longlong(t_search);
-      const unsigned long long d = (unsigned long long)__double_as_longlong(t_all);
-      r[10] = (uint32_t)a;
-      r[11] = (uint32_t)(a >> 32);
-      r[12] = (uint32_t)bb;
-      r[13] = (uint32_t)(bb >> 32);
-      r[16] = (uint32_t)d;
-      r[17] = (uint32_t)(d >> 32);
-    }
-    if (b.ml_cost) b.ml_cost[shot] = 0.0f;
-    if (b.deferred) b.deferred[shot] = 0;
-  }
-  __syncwarp();
-  const unsigned settled = __ballot_sync(kFull, done);
-  if (lane == 0 && settled)
-    atomicAdd(ctr_ptr(b.counters, kCtrSettled), (unsigned long long)__popc(settled));
-  for (unsigned mm = settled; mm; mm &= mm - 1u) {
-    const int j = __ffs(mm) - 1;
-    const int sj = __shfl_sync(kFull, shot, j);
-    if (lane < 18) reinterpret_cast<uint32_t *>(b.results + sj)[lane] = F.res[j][lane];
-    if (b.dec_err || b.dec_log) {
-      const int cj = __shfl_sync(kFull, ci, j);
-      const int pj = __shfl_sync(kFull, pos, j);
-      const DevCode &cdj = b.codes[cj];
-      if (b.dec_err)
-        for (int c = lane; c < cdj.m; c += 32) b.dec_err[(size_t)sj * cdj.m + c] = c == pj ? 1 : 0;
-      if (b.dec_log && cdj.family == kDem)
-        for (int c = lane; c < cdj.n_logicos; c += 32)
-          b.dec_log[(size_t)sj * cdj.n_logicos + c] =
-              pj >= 0 ? (unsigned char)((__ldg(cdj.lcols + (size_t)pj * cdj.nlw + (c >> 5)) >> (c & 31)) & 1u)
-                      : 0;
-    }
-  }
-
-  // ---- the others: appended to the slow queue --------------------------------
-  const bool slow = valid && !done;
-  const unsigned sm = __ballot_sync(kFull, slow);
-  if (sm) {
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(ctr_ptr(b.counters, kCtrQueueReserved), (unsigned long long)__popc(sm));
-    base = __shfl_sync(kFull, base, 0);
-    // the entry carries this launch's tag: a ticket holder that reads it knows it
-    // is not a leftover of an earlier launch
-    if (slow)
-      *reinterpret_cast<volatile unsigned long long *>(b.queue + base + __popc(sm & lt_mask)) =
-          ((unsigned long long)tag << 32) | (unsigned)slot | (extracted && ok ? 0x80000000u : 0u);
-  }
-  __syncwarp();
-  prof_lap(b, kProfChunkWrite, tp);
 }
 
 }  // namespace grand

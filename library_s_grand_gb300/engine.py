@@ -155,8 +155,8 @@ class Engine:
                                             d_records, stream or None)
 
     def launch_stats(self, stream=0):
-        """(settled by classification, per-shot path, Jobs, tiles, scratch words) of the
-        last device decode on `stream`."""
+        """(settled by classification, searched one by one, past the light budget, Job
+        tiles, Job scratch words) of the last device decode on `stream`."""
         out = (ctypes.c_longlong * 31)()
         rc = self.lib.grand_engine_launch_stats(self.h, stream or None, out)
         return tuple(out[:5]) if rc == 0 else None
