@@ -33,8 +33,8 @@ constexpr int kFastLogBallots = kMaxChunk * kFastLogWords;  // ballot words of s
 // classify_chunk's part of a warp's shared memory.  A shot's row holds its syndrome
 // (words 0 .. 7), sketch (8), supplied weight (9) and logical words (10 .. 13) while it is open, and its result's 18 words once it is settled.
 struct FastArea {
-  uint32_t bits[kFastBallots + 1];      // bit e: entry e of the run's records (flat)
-  uint32_t lbits[kFastLogBallots + 1];  // the same for DEM logicals kept in their own array
+  uint32_t bits[kFastBallots + 8];      // the run's records, entry after entry (flat_ballots)
+  uint32_t lbits[kFastLogBallots + 8];  // the same for DEM logicals kept in their own array
   uint32_t row[kMaxChunk][18];
   int shot[kMaxChunk];
 };
@@ -49,70 +49,48 @@ struct ChunkArea {
   DevCode code;  // the code being searched
 };
 
-// Bits b0..b7 of x moved to bits 0, 4, .., 28.
-__device__ __forceinline__ uint32_t spread4(uint32_t x) {
-  x &= 0xffu;
-  x = (x | (x << 12)) & 0x000F000Fu;
-  x = (x | (x << 6)) & 0x03030303u;
-  x = (x | (x << 3)) & 0x11111111u;
-  return x;
-}
-
-// bits[k] = the nonzero flags of p[32k .. 32k + 31] for the n entries at p (bits
-// past n are 0); bits[ceil(n/32)] = 0.  The entries are read once and kept out
-// of L1 (the per-shot path may read them again from L2).  With p 16-byte
-// aligned, lanes read four entries at a time, eight 16-byte loads each in
-// flight (records read in place from host memory need the bytes in flight): a
-// row of 32 lanes is 128 entries, and its four words are four ballots (ballot
-// c holds entry 4l + c in bit l) interleaved by four lanes.  Otherwise, and for
-// the last n % 128 entries, one entry per lane per ballot.
-static __device__ __noinline__ void flat_ballots(const int *p, int n, uint32_t *bits) {
+// The nonzero flags of the n entries at p as a bit vector: entry e is bit pad + e, with
+// pad (returned, 0 .. 3) the entries between p and the 16-byte boundary below it; other
+// bits are arbitrary.  Lanes read four entries at a time, eight 16-byte loads each in
+// flight (records read in place from host memory need the bytes in flight), kept out of
+// L1; two lanes' flags make a byte.  The groups of four that p and the end cut are
+// read entry by entry.  Writes whole rows of 128 entries (16 bytes).
+static __device__ __noinline__ int flat_ballots(const int *p, int n, uint32_t *bits) {
   const int lane = threadIdx.x & 31;
-  const int nwords = (n + 31) >> 5;
-  int done = 0;  // entries handled by the 16-byte path (a multiple of 128)
-  if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0u) {
-    const int4 *p4 = reinterpret_cast<const int4 *>(p);
-    const int rows = n >> 7;  // full rows of 128 entries
+  const int pad = (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 3u);
+  p -= pad;
+  n += pad;
+  uint8_t *bytes = reinterpret_cast<uint8_t *>(bits);
+  const int4 *p4 = reinterpret_cast<const int4 *>(p);
+  const int first = pad ? 1 : 0, full = n >> 2;  // whole groups: first .. full - 1
 #pragma unroll 1
-    for (int r0 = 0; r0 < rows; r0 += 8) {
-      int4 v[8];
+  for (int r0 = 0; r0 * 128 < n; r0 += 8) {
+    int4 v[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        v[u] = r0 + u < rows ? __ldcg(p4 + (r0 + u) * 32 + lane) : make_int4(0, 0, 0, 0);
+    for (int u = 0; u < 8; ++u) {
+      const int i = (r0 + u) * 32 + lane;
+      v[u] = i >= first && i < full ? __ldcg(p4 + i) : make_int4(0, 0, 0, 0);
+    }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        if (r0 + u < rows) {
-          const uint32_t b0 = __ballot_sync(kFull, v[u].x != 0);
-          const uint32_t b1 = __ballot_sync(kFull, v[u].y != 0);
-          const uint32_t b2 = __ballot_sync(kFull, v[u].z != 0);
-          const uint32_t b3 = __ballot_sync(kFull, v[u].w != 0);
-          if (lane < 4) {
-            const int sh = 8 * lane;
-            bits[(r0 + u) * 4 + lane] = spread4(b0 >> sh) | (spread4(b1 >> sh) << 1) |
-                                        (spread4(b2 >> sh) << 2) | (spread4(b3 >> sh) << 3);
-          }
-        }
+    for (int u = 0; u < 8; ++u) {
+      if ((r0 + u) * 128 < n) {
+        const unsigned nib = (v[u].x ? 1u : 0u) | (v[u].y ? 2u : 0u) | (v[u].z ? 4u : 0u) | (v[u].w ? 8u : 0u);
+        const unsigned next = __shfl_down_sync(kFull, nib, 1);
+        if (!(lane & 1)) bytes[((r0 + u) * 32 + lane) >> 1] = (uint8_t)(nib | (next << 4));
       }
     }
-    done = rows << 7;
   }
+  if (pad | (n & 3)) {
+    __syncwarp();
+    if (lane == 0) {
 #pragma unroll 1
-  for (int k0 = done >> 5; k0 < nwords; k0 += 16) {
-    int v[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const int e = (k0 + u) * 32 + lane;
-      v[u] = e < n ? __ldcg(p + e) : 0;
+      for (int e = pad; e < n; ++e) {
+        if (e >= 4 * first && e < 4 * full) e = 4 * full;
+        if (e < n && __ldcg(p + e)) bytes[e >> 3] |= (uint8_t)(1u << (e & 7));
+      }
     }
-    uint32_t mine = 0u;
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const uint32_t w = __ballot_sync(kFull, v[u] != 0);
-      mine = lane == u ? w : mine;
-    }
-    if (lane < 16 && k0 + lane < nwords) bits[k0 + lane] = mine;
   }
-  if (lane == 0) bits[nwords] = 0u;
+  return pad;
 }
 
 // Word q of the nbits-entry bit vector that starts at entry `off` of a flat
@@ -123,29 +101,6 @@ __device__ __forceinline__ uint32_t flat_word(const uint32_t *bits, int off, int
   const int rem = nbits - 32 * q;
   if (rem < 32) w &= (1u << rem) - 1u;
   return w;
-}
-
-// Upstream's planner (grand_decoder.cu:1284-1296, 1550-1554, 754-786) for a first
-// threshold iteration with one active position: is it searched, and with a
-// weight-1 block (its only candidate)?  *gpu: the branch upstream takes.
-static __device__ __noinline__ bool one_position_searched(const DevCode &cd, bool *gpu) {
-  if (cd.family == kDem && 1 > cd.cap) return false;  // the cap replaces the set by an empty one
-  const bool g = (1 > cd.thr && 1 <= cd.cap && cd.mode == 1) || cd.mode == 0;
-  const bool c = !g && ((1 <= cd.thr && cd.mode == 1) || cd.mode == -1);
-  if (!g && !c) return false;
-  *gpu = g;
-  if (cd.variant != kProb) return true;  // weights 1..min(W, 1)
-  int mi = cd.n_masks - 1;
-#pragma unroll 1
-  for (int q = 0; q < cd.n_masks; ++q)
-    if (1 <= cd.mask_tam_upper[q]) {
-      mi = q;
-      break;
-    }
-#pragma unroll 1
-  for (int k = 0; k < cd.num_phases; ++k)
-    if (cd.mask_order[mi][k] == 0) return true;  // phase 0 lists weight 1
-  return false;
 }
 
 // Statistics of a warp, added to the control block when it leaves: shots settled without
@@ -206,11 +161,9 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
   //      back-to-back records, bit-packed words read directly ------------------
   int ow = 0, epos = -1;
   uint32_t hs = 0u;
-  uint32_t s[kFastWords];
-#pragma unroll
-  for (int k = 0; k < kFastWords; ++k) s[k] = 0u;
   bool log_ok = true;
   const bool sep = b.in_log != nullptr;
+  int lpad = 0;
   if (sep) {
     // the chunk's logicals lie back to back unless the shots are mapped (a single-code
     // call: every lane has the same code)
@@ -218,10 +171,13 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
     if (__any_sync(kFull, ok && dem && log_ok)) {
       const int first = chunk * size;
       const int cnt = b.num_shots - first < size ? b.num_shots - first : size;
-      flat_ballots(b.in_log + (long long)first * cd.n_logicos, cnt * cd.n_logicos, F.lbits);
+      lpad = flat_ballots(b.in_log + (long long)first * cd.n_logicos, cnt * cd.n_logicos, F.lbits);
       __syncwarp();
     }
   }
+  const uint32_t *cols = cd.g_gs ? cd.g_cols : cd.cols;
+  const uint32_t *hcol = cd.g_gs ? cd.g_hcol : cd.hcol;
+  const int stride = cd.g_gs ? cd.g_gs : cd.nwp;  // words per column
   // this lane's record out of ballots of the entries from `first` on (or its packed words)
   auto take = [&](int at, const uint32_t *rw) {
     auto word = [&](int q) {
@@ -231,6 +187,8 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
       return rem < 32 ? w & ((1u << rem) - 1u) : w;
     };
     if (errs) {
+      Resid s;
+      s.a = s.b = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll 1
       for (int q = 0; q < nwords; ++q) {
         uint32_t w = word(q);
@@ -239,15 +197,23 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
         for (; w; w &= w - 1u) {
           const int c = q * 32 + __ffs((int)w) - 1;
           epos = c;
-          hs ^= __ldg(cd.hcol + c);
-          const uint32_t *col = cd.cols + (size_t)c * cd.nwp;
-#pragma unroll
-          for (int k = 0; k < kFastWords; ++k)
-            if (k < nw) s[k] ^= __ldg(col + k);
+          hs ^= __ldg(hcol + c);
+          if (stride >= 4) {
+            xor_col(cols, stride == 8, (unsigned)c, s);
+          } else {
+            s.a.x ^= __ldg(cols + c * stride);
+            if (stride == 2) s.a.y ^= __ldg(cols + c * 2 + 1);
+          }
         }
       }
-#pragma unroll
-      for (int k = 0; k < kFastWords; ++k) row[k] = s[k];
+      row[0] = s.a.x;
+      row[1] = s.a.y;
+      row[2] = s.a.z;
+      row[3] = s.a.w;
+      row[4] = s.b.x;
+      row[5] = s.b.y;
+      row[6] = s.b.z;
+      row[7] = s.b.w;
     } else {
 #pragma unroll 1
       for (int k = 0; k < kFastWords; ++k) {
@@ -266,7 +232,7 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
           uint32_t w = 0u;
           if (k < cd.nlw) {
             if (lw) w = __ldcg(lw + k) & (rem < 32 ? (1u << rem) - 1u : kFull);
-            else if (sep) w = flat_word(F.lbits, lane * cd.n_logicos, k, cd.n_logicos);
+            else if (sep) w = flat_word(F.lbits, lpad + lane * cd.n_logicos, k, cd.n_logicos);
             else w = flat_word(F.bits, at + cd.R, k, cd.n_logicos);
           }
           row[kRowLog + k] = w;
@@ -307,9 +273,9 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
         if (in_run) ok = false;  // longer than the chunk's ballot area: slow path
         continue;
       }
-      flat_ballots(b.in + first, (int)(end - first), F.bits);
+      const int pad = flat_ballots(b.in + first, (int)(end - first), F.bits);
       __syncwarp();
-      at = in_run ? (int)(rbase - first) : at;
+      at = in_run ? (int)(rbase - first) + pad : at;
     } else {
       words = false;
       rw = reinterpret_cast<const uint32_t *>(b.in) + rbase;
@@ -323,27 +289,32 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
   bool empty = ok;
 #pragma unroll 1
   for (int k = 0; k < nw && empty; ++k) empty = row[k] == 0u;
-  bool found = false, gpu = false;
+  bool found = false;
   int pos = -1, deg = 0, iseq = 0;
-  if (ok && !empty && cd.solo_cols && cd.binary && cd.max_soma >= 1 && one_position_searched(cd, &gpu)) {
+  if (ok && !empty && cd.solo_branch) {
     // the first iteration's active set is the nonzero columns contained in s:
     // it is one column whose only candidate matches exactly when s equals a
-    // solo column, found by s's sketch in the solo table
-    uint32_t i = hs & cd.solo_mask;
+    // solo column, found by s's sketch (in the guided search's table, or in one of the
+    // solo columns alone)
+    const uint32_t mask = cd.g_gs ? cd.g_tab_mask : cd.solo_mask;
+    uint32_t i = hs & mask;
 #pragma unroll 1
-    for (uint32_t probe = 0; probe <= cd.solo_mask && !found; ++probe) {
-      const int c = __ldg(cd.solo_cols + i);
-      if (c < 0) break;
-      if (__ldg(cd.solo_keys + i) == hs) {
+    for (uint32_t probe = 0; probe <= mask && !found; ++probe) {
+      uint2 e;
+      if (cd.g_gs) e = __ldg(reinterpret_cast<const uint2 *>(cd.g_tab) + i);
+      else e = make_uint2(__ldg(cd.solo_keys + i), (unsigned)__ldg(cd.solo_cols + i) | kSoloFlag);
+      const int c = (int)(e.y & 0xffffu);
+      if (c == (int)kNoCol) break;
+      if (e.x == hs && (e.y & kSoloFlag)) {
         bool eq = true;
 #pragma unroll 1
-        for (int k = 0; k < nw && eq; ++k) eq = __ldg(cd.cols + (size_t)c * cd.nwp + k) == row[k];
+        for (int k = 0; k < nw && eq; ++k) eq = __ldg(cols + c * stride + k) == row[k];
         if (eq) {
           found = true;
           pos = c;
         }
       }
-      i = (i + 1u) & cd.solo_mask;
+      i = (i + 1u) & mask;
     }
     if (found) {
       if (!dem && errs) {
@@ -374,23 +345,22 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
       if (empty) {
         row[8] = (uint32_t)-2;
       } else {
-        const unsigned long long half = t_start + (now - t_start) / 2;  // counts ~ half the time
+        // the times: counts and search half each, and the whole
+        const unsigned long long dt = now - t_start;
+        const unsigned long long h = (unsigned long long)__double_as_longlong(1e-6 * (double)(dt >> 1));
+        const unsigned long long t = (unsigned long long)__double_as_longlong(1e-6 * (double)dt);
+        row[10] = row[12] = (uint32_t)h;
+        row[11] = row[13] = (uint32_t)(h >> 32);
+        row[16] = (uint32_t)t;
+        row[17] = (uint32_t)(t >> 32);
         row[0] = 1u;
         row[1] = 1u;
         row[3] = (uint32_t)deg;
         row[4] = (uint32_t)iseq;
         row[5] = 1u;
         row[6] = 1u;
-        row[8] = gpu ? 0u : (uint32_t)-1;
+        row[8] = cd.solo_branch == kSoloGpu ? 0u : (uint32_t)-1;
         row[9] = 1u;
-#pragma unroll 1
-        for (int k = 0; k < 3; ++k) {  // the times: counts, search, whole shot
-          const unsigned long long dt = k == 0 ? half - t_start : (k == 1 ? now - half : now - t_start);
-          const unsigned long long a = (unsigned long long)__double_as_longlong(1e-6 * (double)dt);
-          const int w = k == 2 ? 16 : 10 + 2 * k;
-          row[w] = (uint32_t)a;
-          row[w + 1] = (uint32_t)(a >> 32);
-        }
       }
       if (b.ml_cost)
         b.ml_cost[shot] = MLK && found && cd.variant == kMl ? __fadd_rn(0.0f, __ldg(cd.llr + pos)) : 0.0f;
@@ -445,8 +415,7 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
         if (lane < code.nlw) eb = rj[kRowLog + lane];
       } else if (code.input_kind == kInErrors) {
         if (!code.packed && !one_run) {  // a later run took its bits' place
-          flat_ballots(b.in + rb_j, code.m, F.bits);
-          at_j = 0;
+          at_j = flat_ballots(b.in + rb_j, code.m, F.bits);
           __syncwarp();
         }
         const int rem = code.m - 32 * lane;
@@ -495,6 +464,18 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
   __syncwarp();
 }
 
+// A load whose value nothing uses, for the line it brings into L1.
+__device__ __forceinline__ void touch_line(const void *p) {
+#ifdef GRAND_HOST_EMULATION
+  (void)p;
+#else
+  unsigned x;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(x) : "l"(p));
+#endif
+}
+constexpr int kWarmCodes = 8;   // codes whose tables are fetched ahead (about 60 KB for the BB codes)
+constexpr int kWarmTam = 192;   // active sets whose binomials are
+
 // One warp per chunk of the batch.
 constexpr int kChunkWarps = 4;
 // Resident blocks per SM: 5 leave a thread 96 registers and the SM about 130 KB of L1.
@@ -509,6 +490,18 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
   const int wib = threadIdx.x >> 5;
   const unsigned long long chunk = (unsigned long long)blockIdx.x * kChunkWarps + (unsigned)wib;
   if (chunk * (unsigned)b.chunk >= (unsigned long long)b.num_shots) return;
+  // The first blocks of an SM find its L1 empty: one load per 128-byte line of the codes'
+  // tables, and of the binomials of small sets, starts them on their way together, in
+  // place of one miss after another along the search's chains.
+  {
+    const int stride = kChunkWarps * 32;
+    for (int k = 0; k < b.num_codes && k < kWarmCodes; ++k) {
+      const DevCode &cd = b.codes[k];
+      const int lines = cd.g_gs ? (cd.g_words + 31) >> 5 : 0;
+      for (int i = threadIdx.x; i < lines; i += stride) touch_line(cd.g_rows + 32 * i);
+    }
+    for (int i = threadIdx.x; i < kWarmTam * (kMaxW + 1) / 16; i += stride) touch_line(b.ncr + 16 * i);
+  }
   const unsigned tag = *reinterpret_cast<volatile unsigned *>(b.epoch) + 1u;
   const unsigned long long t_enter = b.profile ? global_ns() : 0ull;
   ChunkStats st{0, 0, 0};

@@ -53,7 +53,7 @@ constexpr int kMaxSegsPerIter = 15;       // 3 phases x 5 weights
 constexpr int kMaxSegs = kMaxIters * kMaxSegsPerIter;
 
 // Codes the guided search takes (grand_guided_tables.h).
-constexpr int kGuidedMaxRows = 256;
+constexpr int kGuidedMaxRows = 255;     // (row numbers and the row of zeros behind them: a byte)
 constexpr int kGuidedMaxCols = 1024;
 constexpr int kGuidedMaxColWeight = 7;
 constexpr int kGuidedMaxDegree = 64;
@@ -65,6 +65,7 @@ constexpr int kMaxChunk = 16;
 constexpr int kFastBallots = 256;
 constexpr int kGuidedItems = 344;       // partial sets a search holds (all its levels)
 constexpr unsigned kNoCol = 0xffffu;    // no column (adjacency padding, empty table slot)
+constexpr unsigned kSoloFlag = 0x10000u;
 
 enum Family { kCss = 0, kDem = 1 };
 enum Variant { kUniform = 0, kProb = 1, kMl = 2 };
@@ -175,11 +176,13 @@ struct DevCode {
   const uint32_t *solo_keys; // solo columns (nonzero, containing no other nonzero column)
   const int *solo_cols;      //   by sketch: open addressing, column -1 = empty slot
   uint32_t solo_mask;        //   (solo_cols nullptr: no table)
+  int solo_branch;           // how a first iteration of one position is searched (solo_branch_of)
   // guided search (grand_guided_tables.h); g_gs = 0: the code has none
   int g_gs, g_deg, g_max_cw; // words per packed column, largest row degree, largest column weight
   uint32_t g_tab_mask;
+  int g_words;                 // the tables lie in one block of g_words words from g_rows on
   unsigned long long g_magic;  // ceil(2^32 / g_deg)
-  const uint32_t *g_rows, *g_cw, *g_cols, *g_filt, *g_tab;
+  const uint32_t *g_rows, *g_cw, *g_cols, *g_filt, *g_tab, *g_hcol;
   const uint16_t *g_adj;
 };
 
@@ -244,6 +247,31 @@ struct alignas(128) Job {
   alignas(16) unsigned long long mlkey[kMaxIters][kMaxW + 1][2]; // ML: {cost key, lex rank} minima
 };
 static_assert(sizeof(Job) % 128 == 0, "Job must fill whole 128-byte lines in arrays");
+
+// A first threshold iteration with one active position, as upstream's planner treats it
+// (grand_decoder.cu:1284-1296, 1550-1554, 754-786): not searched with a weight-1 block (its
+// only candidate), or searched on the CPU or the GPU branch.  (kSoloNone as well for a
+// code without a solo table, or whose flagged-check counts are not column overlaps.)
+enum SoloBranch { kSoloNone = 0, kSoloCpu = 1, kSoloGpu = 2 };
+inline int solo_branch_of(const DevCode &cd) {
+  if (!cd.solo_cols || !cd.binary || cd.max_soma < 1) return kSoloNone;
+  if (cd.family == kDem && 1 > cd.cap) return kSoloNone;  // the cap replaces the set by an empty one
+  const bool g = (1 > cd.thr && 1 <= cd.cap && cd.mode == 1) || cd.mode == 0;
+  const bool c = !g && ((1 <= cd.thr && cd.mode == 1) || cd.mode == -1);
+  if (!g && !c) return kSoloNone;
+  const int branch = g ? kSoloGpu : kSoloCpu;
+  if (cd.variant != kProb) return cd.Wc >= 1 ? branch : kSoloNone;  // weights 1..min(W, 1)
+  if (cd.n_masks < 1) return kSoloNone;
+  int mi = cd.n_masks - 1;
+  for (int q = 0; q < cd.n_masks; ++q)
+    if (1 <= cd.mask_tam_upper[q]) {
+      mi = q;
+      break;
+    }
+  for (int k = 0; k < cd.num_phases; ++k)
+    if (cd.mask_order[mi][k] == 0) return branch;  // phase 0 lists weight 1
+  return kSoloNone;
+}
 
 // Everything one batched launch needs.
 struct DevBatch {

@@ -52,7 +52,7 @@ struct alignas(16) GuidedArea {
   uint2 item[kGuidedItems];
   uint32_t sw[8];                // the syndrome, zero past nw
   uint32_t am[32];               // the searched iteration's active columns
-  uint8_t rows[kGuidedMaxRows];  // the syndrome's set rows, ascending
+  uint8_t rows[kGuidedMaxRows + 4];  // the syndrome's set rows, ascending, padded with R
 };
 constexpr unsigned kNoRow = 1023u;
 static_assert(kGuidedItems <= 1024 && kGuidedMaxCols <= 1024 && kGuidedMaxRows < (int)kNoRow,
@@ -73,22 +73,6 @@ __device__ __forceinline__ int warp_add(int v) {
 #else
   return __reduce_add_sync(kFull, v);
 #endif
-}
-
-// C(n, k) for n <= 1024, k <= 6: exact, the small weights in 32 bits.
-static __device__ __noinline__ unsigned long long binom_small(int n, int k) {
-  if (k < 0 || n < k) return 0ull;
-  const unsigned u = (unsigned)n;
-  if (k == 0) return 1ull;
-  if (k == 1) return u;
-  unsigned r = u * (u - 1u) >> 1;
-  if (k == 2) return r;
-  r = r * (u - 2u) / 3u;  // at most 1024 * 1023 * 1022 / 2 < 2^32
-  if (k == 3) return r;
-  unsigned long long q = (unsigned long long)r * (u - 3u) >> 2;
-  if (k >= 5) q = q * (u - 4u) / 5ull;
-  if (k >= 6) q = q * (u - 5u) / 6ull;
-  return q;
 }
 
 // One code's tables and the search's state, uniform over the warp.
@@ -246,9 +230,10 @@ __device__ __forceinline__ void guided_probe(const GuidedArea &G, const GuidedVi
 #pragma unroll 1
   for (uint32_t guard = 0; guard <= v.tab_mask; ++guard) {
     const uint2 e = __ldg(reinterpret_cast<const uint2 *>(v.tab) + i);
-    if (e.y == kNoCol) return;
-    if (e.x == h && e.y != c && !in_path(p, e.y) && ((G.am[e.y >> 5] >> (e.y & 31u)) & 1u))
-      best = guided_match<MLK>(G.sw, v.cols, v.wide, v.llr, p, d, c, e.y, best);
+    const unsigned j = e.y & 0xffffu;
+    if (j == kNoCol) return;
+    if (e.x == h && j != c && !in_path(p, j) && ((G.am[j >> 5] >> (j & 31u)) & 1u))
+      best = guided_match<MLK>(G.sw, v.cols, v.wide, v.llr, p, d, c, j, best);
     i = (i + 1u) & v.tab_mask;
   }
 }
@@ -415,6 +400,14 @@ __device__ __forceinline__ bool guided_search(GuidedArea &G, const GuidedView &v
   return true;
 }
 
+// x added to the counters of each bit position.
+__device__ __forceinline__ void add_bits(uint32_t x, uint32_t &c0, uint32_t &c1, uint32_t &c2) {
+  const uint32_t t = c0 & x;
+  c0 ^= x;
+  c2 ^= c1 & t;
+  c1 ^= t;
+}
+
 // Exclusive prefix sum over the lanes.
 __device__ __forceinline__ int lanes_before(int v) {
   const int lane = threadIdx.x & 31;
@@ -489,39 +482,53 @@ __device__ __forceinline__ int guided_shot(const DevBatch &b, const DevCode &cd,
     if ((word >> lane) & 1u) G.rows[ones + __popc(word & ((1u << lane) - 1u))] = (uint8_t)(32 * k + lane);
     ones += __popc(word);
   }
+  if (lane < 4) G.rows[ones + lane] = (uint8_t)cd.R;  // the row of zeros behind the table's
   __syncwarp();
 
   // ---- counts, bit-sliced: lane q the columns of mask word q ----------------------
   const int L = cd.max_soma < kMaxIters ? cd.max_soma : kMaxIters;
   uint32_t am0 = 0u, am1 = 0u, am2 = 0u;
-  if (lane < mw) {
-    const uint32_t *rows = cd.g_rows + lane;
+  {
+    // up to 8 mask words: four groups of lanes share the rows and add their counts up;
+    // up to 16: two groups; the list ends with rows of zeros
+    const int split = mw <= 8 ? 4 : (mw <= 16 ? 2 : 1);
+    const int q = lane & (32 / split - 1);
+    const int step = 4 * split, part = lane / (32 / split);
+    const uint32_t *rows = cd.g_rows + (q < mw ? q : 0);
     uint32_t c0 = 0u, c1 = 0u, c2 = 0u;
 #pragma unroll 1
-    for (int i = 0; i < ones; i += 8) {
-      uint32_t x[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) x[u] = i + u < ones ? __ldg(rows + (int)G.rows[i + u] * mw) : 0u;
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const uint32_t t = c0 & x[u];
-        c0 ^= x[u];
-        c2 ^= c1 & t;
-        c1 ^= t;
-      }
+    for (int i = 4 * part; i < ones; i += step) {
+      const uchar4 r = *reinterpret_cast<const uchar4 *>(G.rows + i);
+      const uint32_t x0 = __ldg(rows + (int)r.x * mw), x1 = __ldg(rows + (int)r.y * mw),
+                     x2 = __ldg(rows + (int)r.z * mw), x3 = __ldg(rows + (int)r.w * mw);
+      add_bits(x0, c0, c1, c2);
+      add_bits(x1, c0, c1, c2);
+      add_bits(x2, c0, c1, c2);
+      add_bits(x3, c0, c1, c2);
     }
-    const uint32_t w0 = __ldg(cd.g_cw + lane), w1 = __ldg(cd.g_cw + mw + lane),
-                   w2 = __ldg(cd.g_cw + 2 * mw + lane);
-    // missing = weight - count, bit by bit; zero columns are never active
-    const uint32_t nz = w0 | w1 | w2;
-    const uint32_t m0 = w0 ^ c0, b0 = ~w0 & c0;
-    const uint32_t m1 = w1 ^ c1 ^ b0, b1 = (~w1 & c1) | (~(w1 ^ c1) & b0);
-    const uint32_t m2 = w2 ^ c2 ^ b1;
-    am0 = nz & ~(m0 | m1 | m2);
-    am1 = nz & ~(m1 | m2);
-    am2 = nz & ~(m2 | (m1 & m0));
+    __syncwarp();
+#pragma unroll 1
+    for (int o = 32 / split; o < 32; o <<= 1) {
+      const uint32_t y0 = __shfl_xor_sync(kFull, c0, o), y1 = __shfl_xor_sync(kFull, c1, o),
+                     y2 = __shfl_xor_sync(kFull, c2, o);
+      const uint32_t t0 = c0 & y0, t1 = (c1 & y1) | (t0 & (c1 ^ y1));
+      c2 ^= y2 ^ t1;
+      c1 ^= y1 ^ t0;
+      c0 ^= y0;
+    }
+    if (lane < mw) {
+      const uint32_t w0 = __ldg(cd.g_cw + lane), w1 = __ldg(cd.g_cw + mw + lane),
+                     w2 = __ldg(cd.g_cw + 2 * mw + lane);
+      // missing = weight - count, bit by bit; zero columns are never active
+      const uint32_t nz = w0 | w1 | w2;
+      const uint32_t m0 = w0 ^ c0, b0 = ~w0 & c0;
+      const uint32_t m1 = w1 ^ c1 ^ b0, b1 = (~w1 & c1) | (~(w1 ^ c1) & b0);
+      const uint32_t m2 = w2 ^ c2 ^ b1;
+      am0 = nz & ~(m0 | m1 | m2);
+      am1 = nz & ~(m1 | m2);
+      am2 = nz & ~(m2 | (m1 & m0));
+    }
   }
-  __syncwarp();
   const unsigned long long t_counts = global_ns();
   tp = prof_lap(b, kProfShotCounts, tp);
 
@@ -530,7 +537,7 @@ __device__ __forceinline__ int guided_shot(const DevBatch &b, const DevCode &cd,
   v.filt = cd.g_filt;
   v.tab = cd.g_tab;
   v.adj = cd.g_adj;
-  v.hcol = cd.hcol;
+  v.hcol = cd.g_hcol;
   v.llr = ml ? cd.llr : nullptr;
   v.tab_mask = cd.g_tab_mask;
   v.deg = cd.g_deg;
@@ -575,7 +582,7 @@ __device__ __forceinline__ int guided_shot(const DevBatch &b, const DevCode &cd,
     __syncwarp();
 
     // candidate counts: lane w holds those of weights 1 .. w
-    unsigned long long upto = lane >= 1 && lane <= kMaxW ? binom_small(tam, lane) : 0ull;
+    unsigned long long upto = lane >= 1 ? ncr(b.ncr, tam, lane) : 0ull;
 #pragma unroll 1
     for (int o = 1; o < 8; o <<= 1) {
       const unsigned long long u = __shfl_up_sync(kFull, upto, o);
@@ -654,7 +661,7 @@ __device__ __forceinline__ int guided_shot(const DevBatch &b, const DevCode &cd,
       const int pre = lanes_before(__popc(am));
       const unsigned c = lane < wn.w ? set_col(wn.key, wn.w, lane) : 0u;
       const int idx = __shfl_sync(kFull, pre, (int)(c >> 5)) + __popc(G.am[c >> 5] & ((1u << (c & 31u)) - 1u));
-      unsigned long long after = lane < wn.w ? binom_small(tam - 1 - idx, wn.w - lane) : 0ull;
+      unsigned long long after = lane < wn.w ? ncr(b.ncr, tam - 1 - idx, wn.w - lane) : 0ull;
 #pragma unroll 1
       for (int o = 4; o > 0; o >>= 1) after += __shfl_xor_sync(kFull, after, o);
       tested += __shfl_sync(kFull, upto, wn.w) - __shfl_sync(kFull, upto, wn.w - 1) -

@@ -1,7 +1,8 @@
 // grand_guided_tables.h -- a code's tables for the guided search (host side, built
 // with the code tables; the search itself is grand_guided.cuh).
 //
-//   rows   R rows of H packed into mw = ceil(m/32) words (bit c of row r)
+//   rows   R rows of H packed into mw = ceil(m/32) words (bit c of row r), then one of
+//          zeros
 //   cw     the column weights bit-sliced: bit c of cw[b * mw + (c >> 5)] is bit b of
 //          column c's weight, b < 3
 //   adj    the columns of each row, ascending, deg u16 per row (kNoCol past the
@@ -9,9 +10,11 @@
 //   cols   m columns packed into gs = 4 or 8 words
 //   filt   a 2^kGuidedF-bit filter of the column sketches (one bit per column)
 //   tab    the columns by sketch: open addressing, linear probing, {sketch, column}
-//          pairs (column kNoCol = empty slot), at most half full
+//          pairs (column kNoCol = empty slot; kSoloFlag set for a solo column,
+//          grand_solo.h), at most half full
+//   hcol   the column sketches
 //
-// A code has them when its matrix is 0/1, with at most 256 rows, 1024 columns, 7
+// A code has them when its matrix is 0/1, with at most 255 rows, 1024 columns, 7
 // ones per column and 64 per row: the search keeps a residual syndrome in 4 or 8
 // registers and one mask word per lane, counts in 3 bits, and gains from rows
 // that meet few columns.
@@ -24,6 +27,7 @@
 #include <vector>
 
 #include "grand_common.h"
+#include "grand_solo.h"
 
 namespace grand {
 
@@ -31,13 +35,15 @@ struct GuidedTables {
   int gs = 0, deg = 0, max_cw = 0;
   uint32_t tab_mask = 0;
   // one block of words; the parts start at these word offsets (16-byte aligned)
-  size_t o_rows = 0, o_cw = 0, o_adj = 0, o_cols = 0, o_filt = 0, o_tab = 0;
+  size_t total = 0, o_rows = 0, o_cw = 0, o_adj = 0, o_cols = 0, o_filt = 0, o_tab = 0, o_hcol = 0;
   std::vector<uint32_t> words;  // empty: the code has no guided search
 };
 
-// cols: m columns of nwp words; hcol: their sketches; binary: every entry of H is 0 or 1.
+// cols: m columns of nwp words; hcol: their sketches; binary: every entry of H is 0 or 1;
+// solo: the code's solo columns.
 inline GuidedTables build_guided_tables(const std::vector<uint32_t> &cols, int nwp, int R, int m,
-                                        const std::vector<uint32_t> &hcol, bool binary) {
+                                        const std::vector<uint32_t> &hcol, bool binary,
+                                        const SoloTable &solo) {
   GuidedTables g;
   if (!binary || R > kGuidedMaxRows || m > kGuidedMaxCols) return g;
   const int mw = (m + 31) / 32, nw = (R + 31) / 32;
@@ -62,12 +68,14 @@ inline GuidedTables build_guided_tables(const std::vector<uint32_t> &cols, int n
     top += (n + 3) & ~(size_t)3;
     return at;
   };
-  g.o_rows = part((size_t)R * mw);
+  g.o_rows = part((size_t)(R + 1) * mw);
   g.o_cw = part((size_t)3 * mw);
   g.o_adj = part(((size_t)R * g.deg + 1) / 2);
   g.o_cols = part((size_t)m * g.gs);
   g.o_filt = part((size_t)1 << (kGuidedF - 5));
   g.o_tab = part((size_t)2 * slots);
+  g.o_hcol = part((size_t)m);
+  g.total = top;
   g.words.assign(top, 0u);
   uint32_t *w = g.words.data();
   std::vector<uint16_t> a((size_t)R * g.deg, (uint16_t)kNoCol);
@@ -91,6 +99,13 @@ inline GuidedTables build_guided_tables(const std::vector<uint32_t> &cols, int n
     w[g.o_tab + 2 * i] = hcol[c];
     w[g.o_tab + 2 * i + 1] = (uint32_t)c;
   }
+  memcpy(w + g.o_hcol, hcol.data(), sizeof(uint32_t) * m);
+  for (size_t k = 0; k < solo.cols.size(); ++k) {
+    if (solo.cols[k] < 0) continue;
+    uint32_t i = solo.keys[k] & g.tab_mask;
+    while (w[g.o_tab + 2 * i + 1] != (uint32_t)solo.cols[k]) i = (i + 1) & g.tab_mask;
+    w[g.o_tab + 2 * i + 1] |= kSoloFlag;
+  }
   return g;
 }
 
@@ -108,6 +123,8 @@ inline void set_guided(DevCode &d, const GuidedTables &g, const uint32_t *base) 
   d.g_cols = base + g.o_cols;
   d.g_filt = base + g.o_filt;
   d.g_tab = base + g.o_tab;
+  d.g_hcol = base + g.o_hcol;
+  d.g_words = (int)g.total;
 }
 
 // Does every search of this code fit the chunk kernel, whatever the syndrome?  Its records

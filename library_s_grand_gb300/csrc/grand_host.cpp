@@ -297,7 +297,7 @@ std::shared_ptr<CodeTables> Context::tables(int family, const int *H, const int 
   if (e == cudaSuccess) e = upload(&t->hcol, hcol);
   if (e == cudaSuccess) e = upload(&t->solo_keys, solo.keys);
   if (e == cudaSuccess) e = upload(&t->solo_cols, solo.cols);
-  t->guided = build_guided_tables(cols, t->nwp, n, m, hcol, t->binary != 0);
+  t->guided = build_guided_tables(cols, t->nwp, n, m, hcol, t->binary != 0, solo);
   if (e == cudaSuccess && !t->guided.words.empty()) {
     e = upload(&t->d_guided, t->guided.words);
     std::vector<uint32_t>().swap(t->guided.words);  // only the layout is needed from here on
@@ -379,6 +379,7 @@ DevCode make_devcode(const CodeTables &t, const CallParams &p) {
   d.solo_cols = t.solo_cols;
   d.solo_mask = t.solo_mask;
   set_guided(d, t.guided, t.d_guided);
+  d.solo_branch = solo_branch_of(d);
   return d;
 }
 

@@ -61,12 +61,13 @@ int main(int argc, char **argv) {
   const std::string dir = argv[1];
   Code k;
   if (!load_code(dir, k)) return 2;
-  const GuidedTables g = build_guided_tables(k.cols, k.d.nwp, k.n, k.m, k.hcol, k.d.binary != 0);
+  const GuidedTables g = build_guided_tables(k.cols, k.d.nwp, k.n, k.m, k.hcol, k.d.binary != 0, k.solo);
   std::vector<uint32_t> aligned(g.words.size() + 4);
   uint32_t *base = aligned.data();
   while (reinterpret_cast<uintptr_t>(base) & 15u) ++base;
   std::copy(g.words.begin(), g.words.end(), base);
   set_guided(k.d, g, g.words.empty() ? nullptr : base);
+  k.d.solo_branch = solo_branch_of(k.d);
   const int N = k.N, m = k.m, nl = k.nl;
   const bool dem = k.family == kDem;
   const std::vector<int> rec = read_ints(dir + "/rec.bin", (size_t)N * k.rec_len);
