@@ -1,27 +1,39 @@
-// grand_chunk.cuh -- the chunk step of a decoding launch (sm_103a), and the chunk kernel
-// that runs it with the guided search.
+// grand_chunk.cuh -- the chunk step of a decoding launch (sm_103a): up to kMaxChunk launch slots
+// by one warp, one lane per shot.
 //
-// classify_chunk (up to kMaxChunk launch slots, one lane per shot)
-//   packs the shots' records with coalesced ballots, forms each syndrome and
-//   settles the common shots outright: an empty syndrome (grand_decoder.cu:1223-1241),
-//   and a first threshold iteration with one active position whose column equals
-//   the syndrome (weight-1 match, 1 candidate tested).
+// classify_chunk
+//   packs the shots' records with coalesced loads, forms each syndrome and settles the
+//   common shots outright: an empty syndrome (grand_decoder.cu:1223-1241), and a first
+//   threshold iteration with one active position whose column equals the syndrome
+//   (weight-1 match, 1 candidate tested).  The others stay open: their syndromes wait in
+//   the chunk's rows.
+// write_chunk
+//   writes the results of the chunk's settled shots, and appends those still open to
+//   the slow queue of the decode kernel.
 //
-// chunk_kernel
-//   takes the remaining shots of a chunk one after another through the guided search
-//   (grand_guided.cuh), by the warp that holds their syndromes and record bits.  One
-//   warp per chunk, blocks scheduled by the hardware: nothing waits.  It is a kernel of
-//   its own, not a step of the persistent decode kernel, for its working set: there
-//   (46 KB of shared memory per block, 128 registers, 650 KB of code) the same search
-//   ran at 16 warps per SM out of 28 KB of L1 and missed the instruction caches
-//   (headline 80 us, mix 178 us, noisy [[288]] 164 us); here 48, 125 and 92 us.
+// The chunk kernel (grand_front.cuh) runs the guided search on the open shots in between;
+// the decode kernel runs the two back to back for batches without a guided code.
 #pragma once
 
-#include "grand_guided.cuh"
 #include "grand_kernels.cuh"
 
 namespace grand {
 
+// A syndrome: the second half is used by codes of more than 128 rows (wide).
+struct Resid {
+  uint4 a, b;
+};
+__device__ __forceinline__ void xor_into(uint4 &r, const uint4 w) {
+  r.x ^= w.x;
+  r.y ^= w.y;
+  r.z ^= w.z;
+  r.w ^= w.w;
+}
+__device__ __forceinline__ void xor_col(const uint32_t *cols, bool wide, unsigned c, Resid &r) {
+  const uint4 *p = reinterpret_cast<const uint4 *>(cols) + (c << (wide ? 1 : 0));
+  xor_into(r.a, __ldg(p));
+  if (wide) xor_into(r.b, __ldg(p + 1));
+}
 // ---------------------------------------------------------------------------
 // Chunks of up to kMaxChunk launch slots, one lane per shot.
 // ---------------------------------------------------------------------------
@@ -30,24 +42,21 @@ constexpr int kFastLogWords = 4;      // DEM logical words (n_logicos <= 128)
 constexpr int kFastErrWords = 32;     // error-record words (m <= 1024)
 constexpr int kFastLogBallots = kMaxChunk * kFastLogWords;  // ballot words of separate logical entries
 
-// classify_chunk's part of a warp's shared memory.  A shot's row holds its syndrome
-// (words 0 .. 7), sketch (8), supplied weight (9) and logical words (10 .. 13) while it is open, and its result's 18 words once it is settled.
-struct FastArea {
+// A chunk in its warp's shared memory.  A shot's row holds its syndrome (words 0 .. 7),
+// sketch (8), supplied weight (9) and logical words (10 .. 13) while it is open, and its
+// result's 18 words once it is settled.
+struct alignas(16) FastArea {
+  uint32_t row[kMaxChunk][18];
+  unsigned long long key[kMaxChunk];    // settled shots: the decoded columns (set_col), row[1] of them
+  int shot[kMaxChunk], code[kMaxChunk];
+  int at[kMaxChunk];                    // where its record starts in bits (-1: elsewhere)
+  uint8_t state[kMaxChunk];             // 0: open, 1: settled
   uint32_t bits[kFastBallots + 8];      // the run's records, entry after entry (flat_ballots)
   uint32_t lbits[kFastLogBallots + 8];  // the same for DEM logicals kept in their own array
-  uint32_t row[kMaxChunk][18];
-  int shot[kMaxChunk];
 };
 constexpr int kRowSketch = kFastWords, kRowWeight = kFastWords + 1, kRowLog = kFastWords + 2;
 static_assert(kRowLog + kFastLogWords <= 18, "an open shot's words fit its row");
 static_assert(sizeof(FastArea) <= sizeof(WarpArea), "FastArea must fit the decode kernel's area");
-
-// The chunk kernel's shared memory of one warp.
-struct ChunkArea {
-  GuidedArea guided;
-  FastArea fast;
-  DevCode code;  // the code being searched
-};
 
 // The nonzero flags of the n entries at p as a bit vector: entry e is bit pad + e, with
 // pad (returned, 0 .. 3) the entries between p and the 16-byte boundary below it; other
@@ -115,28 +124,46 @@ __device__ __forceinline__ void add_stats(const DevBatch &b, const ChunkStats &s
   if (st.heavy) atomicAdd(w + 2, (unsigned long long)st.heavy);
 }
 
-// Settles the shots of launch slots size * chunk + [0, size), size <= kMaxChunk.
+// Column e (of w, in list order) of a column set: 10 bits each, the first on top.
+__device__ __forceinline__ unsigned set_col(unsigned long long key, int w, int e) {
+  return (unsigned)(key >> (10 * (w - 1 - e))) & 1023u;
+}
+
+// Word `lane` of the column set `key` (w columns).
+__device__ __forceinline__ uint32_t set_word(unsigned long long key, int w) {
+  const int lane = threadIdx.x & 31;
+  uint32_t e = 0u;
+#pragma unroll 1
+  for (int k = 0; k < w; ++k) {
+    const unsigned c = set_col(key, w, k);
+    if ((int)(c >> 5) == lane) e |= 1u << (c & 31u);
+  }
+  return e;
+}
+
+// out[0 .. n) = the bits of word `lane` of a vector, one byte each.
+__device__ __forceinline__ void bits_to_bytes(unsigned char *out, int n, uint32_t word) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int c0 = 0; c0 < n; c0 += 32) {
+    const uint32_t w = __shfl_sync(kFull, word, c0 >> 5);
+    if (c0 + lane < n) out[c0 + lane] = (unsigned char)((w >> lane) & 1u);
+  }
+}
+
+// Classifies the shots of launch slots size * chunk + [0, size), size <= kMaxChunk, into F.
+// hot: the block's copies of the codes (nullptr: none).  Returns the mask of the lanes whose
+// shots the guided search takes: open, with their syndrome, sketch, supplied weight and
+// logical words in their row.
 //
-// One lane per shot forms the syndromes and settles the shots that need no search: an
-// empty syndrome, or a first iteration with one active position whose column equals
-// the syndrome.  The results are exactly those of the general path: the one position
+// The results of the settled shots are exactly those of the general path: the one position
 // is the only candidate of the iteration (found at weight 1, rank 0; one candidate
 // counted on either branch, hibrido 0 / -1), and its active set is the set of nonzero
 // columns contained in the syndrome (flagged-check count = column weight, for
 // 0/1 matrices regular or not), a solo column found by the syndrome's sketch.
-//
-// GUIDED: the warp then takes the other shots one after another through the guided
-// search, from the syndromes and record bits it holds (area: the warp's search area
-// and code copy).  What is left -- codes without the search's tables, records too wide
-// for a lane, levels that do not fit -- is appended to the slow queue with tag (the
-// launch epoch + 1).
-//
-// kCtrChunks counts the chunks done (high half) and the queue entries reserved (low
-// half) in one word, so that a warp that sees every chunk done sees every
-// reservation too, with no fence in between.
-template <bool MLK, bool GUIDED>
-__device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int size, FastArea &F,
-                                               ChunkArea *area, ChunkStats &st, unsigned tag) {
+template <bool MLK>
+__device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotCode *hot, int chunk,
+                                                   int size, FastArea &F, ChunkStats &st) {
   const int lane = threadIdx.x & 31;
   const int slot = chunk * size + lane;
   const bool valid = lane < size && slot < b.num_shots;
@@ -144,7 +171,8 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
   unsigned long long tp = b.profile ? t_start : 0ull;
   const int shot = valid ? (b.shot_map ? b.shot_map[slot] : slot) : 0;
   const int ci = (valid && b.shot_code) ? b.shot_code[shot] : 0;
-  const DevCode &cd = b.codes[ci];
+  const DevCode &full = b.codes[ci];
+  const HotCode &cd = hot && ci < kHotCodes ? hot[ci] : static_cast<const HotCode &>(full);
   const bool errs = cd.input_kind == kInErrors;
   const bool dem = cd.family == kDem;
   const bool packed = cd.packed != 0;
@@ -155,7 +183,10 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
             (!dem || cd.nlw <= kFastLogWords);
   const long long rbase = valid ? (b.in_off ? b.in_off[shot] : (long long)shot * cd.rec_len) : 0;
   uint32_t *row = F.row[valid ? lane : 0];
-  if (valid) F.shot[lane] = shot;
+  if (valid) {
+    F.shot[lane] = shot;
+    F.code[lane] = ci;
+  }
 
   // ---- the records: int32 entries through coalesced ballots over runs of
   //      back-to-back records, bit-packed words read directly ------------------
@@ -175,8 +206,8 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
       __syncwarp();
     }
   }
-  const uint32_t *cols = cd.g_gs ? cd.g_cols : cd.cols;
-  const uint32_t *hcol = cd.g_gs ? cd.g_hcol : cd.hcol;
+  const uint32_t *cols = cd.g_gs ? cd.g_cols : full.cols;
+  const uint32_t *hcol = cd.g_gs ? cd.g_hcol : full.hcol;
   const int stride = cd.g_gs ? cd.g_gs : cd.nwp;  // words per column
   // this lane's record out of ballots of the entries from `first` on (or its packed words)
   auto take = [&](int at, const uint32_t *rw) {
@@ -296,13 +327,13 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
     // it is one column whose only candidate matches exactly when s equals a
     // solo column, found by s's sketch (in the guided search's table, or in one of the
     // solo columns alone)
-    const uint32_t mask = cd.g_gs ? cd.g_tab_mask : cd.solo_mask;
+    const uint32_t mask = cd.g_gs ? cd.g_tab_mask : full.solo_mask;
     uint32_t i = hs & mask;
 #pragma unroll 1
     for (uint32_t probe = 0; probe <= mask && !found; ++probe) {
       uint2 e;
       if (cd.g_gs) e = __ldg(reinterpret_cast<const uint2 *>(cd.g_tab) + i);
-      else e = make_uint2(__ldg(cd.solo_keys + i), (unsigned)__ldg(cd.solo_cols + i) | kSoloFlag);
+      else e = make_uint2(__ldg(full.solo_keys + i), (unsigned)__ldg(full.solo_cols + i) | kSoloFlag);
       const int c = (int)(e.y & 0xffffu);
       if (c == (int)kNoCol) break;
       if (e.x == hs && (e.y & kSoloFlag)) {
@@ -364,96 +395,87 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
       }
       if (b.ml_cost)
         b.ml_cost[shot] = MLK && found && cd.variant == kMl ? __fadd_rn(0.0f, __ldg(cd.llr + pos)) : 0.0f;
-      if (b.deferred) b.deferred[shot] = 0;
-    }
-    __syncwarp();
-    // one coalesced pass over the rows: word i belongs to lane i / 18's shot
-#pragma unroll 1
-    for (int i = lane; i < size * 18; i += 32) {
-      const int j = (i * 3641) >> 16;  // i / 18 for i < 18 * kMaxChunk
-      if ((settled >> j) & 1u)
-        reinterpret_cast<uint32_t *>(b.results + F.shot[j])[i - 18 * j] = F.row[j][i - 18 * j];
-    }
-    if (b.dec_err || b.dec_log) {
-#pragma unroll 1
-      for (unsigned mm = settled; mm; mm &= mm - 1u) {
-        const int j = __ffs((int)mm) - 1;
-        const int sj = F.shot[j];
-        const int cj = __shfl_sync(kFull, ci, j);
-        const int pj = __shfl_sync(kFull, pos, j);
-        const DevCode &cdj = b.codes[cj];
-        if (b.dec_err)
-          bits_to_bytes(b.dec_err + (size_t)sj * cdj.m, cdj.m,
-                        pj >= 0 && (pj >> 5) == lane ? 1u << (pj & 31) : 0u);
-        if (b.dec_log && cdj.family == kDem)
-          bits_to_bytes(b.dec_log + (size_t)sj * cdj.n_logicos, cdj.n_logicos,
-                        pj >= 0 && lane < cdj.nlw ? __ldg(cdj.lcols + (size_t)pj * cdj.nlw + lane) : 0u);
-      }
     }
   }
-  tp = prof_lap(b, kProfChunkWrite, tp);
+  if (valid) {
+    F.state[lane] = done ? 1 : 0;
+    F.key[lane] = found ? (unsigned long long)pos : 0ull;
+    // (one run: its bits stay; a later run takes an earlier one's place)
+    F.at[lane] = ok && !packed && one_run ? at : -1;
+  }
+  __syncwarp();
+  prof_lap(b, kProfChunkWrite, tp);
+  return __ballot_sync(kFull, ok && !done && cd.g_gs);
+}
 
-  unsigned slow = __ballot_sync(kFull, valid && !done);
-
-  // ---- the others: the guided search ------------------------------------------
-  if constexpr (GUIDED) {
-    DevCode &code = area->code;
-    int loaded = -1;
+// The chunk's results, and its open shots into the slow queue with tag (the launch
+// epoch + 1).
+//
+// kCtrChunks counts the chunks done (high half) and the queue entries reserved (low
+// half) in one word, so that a warp that sees every chunk done sees every
+// reservation too, with no fence in between.
+__device__ __forceinline__ void write_chunk(const DevBatch &b, const HotCode *hot, int chunk, int size,
+                                            const FastArea &F, unsigned tag) {
+  const int lane = threadIdx.x & 31;
+  const int slot = chunk * size + lane;
+  const bool valid = lane < size && slot < b.num_shots;
+  const bool open = valid && F.state[valid ? lane : 0] == 0;
+  const unsigned settled = __ballot_sync(kFull, valid && !open);
+  const unsigned slow = __ballot_sync(kFull, open);
+  // one coalesced pass over the rows: word i belongs to lane i / 18's shot
 #pragma unroll 1
-    for (unsigned mm = __ballot_sync(kFull, ok && !done && cd.g_gs); mm; mm &= mm - 1u) {
+  for (int i = lane; i < size * 18; i += 32) {
+    const int j = (i * 3641) >> 16;  // i / 18 for i < 18 * kMaxChunk
+    if ((settled >> j) & 1u)
+      reinterpret_cast<uint32_t *>(b.results + F.shot[j])[i - 18 * j] = F.row[j][i - 18 * j];
+  }
+  if (b.deferred && valid && !open) b.deferred[F.shot[lane]] = 0;
+  if (b.dec_err || b.dec_log) {
+#pragma unroll 1
+    for (unsigned mm = settled; mm; mm &= mm - 1u) {
       const int j = __ffs((int)mm) - 1;
-      const int cj = __shfl_sync(kFull, ci, j);
-      int at_j = __shfl_sync(kFull, at, j);
-      const long long rb_j = __shfl_sync(kFull, rbase, j);
-      if (loaded != cj) {
-        load_code(code, b.codes + cj);
-        loaded = cj;
+      const int sj = F.shot[j], w = (int)F.row[j][1];
+      const unsigned long long key = F.key[j];
+      const HotCode &cd = b.codes[F.code[j]];
+      if (b.dec_err && cd.m <= kGuidedMaxCols) {
+        bits_to_bytes(b.dec_err + (size_t)sj * cd.m, cd.m, set_word(key, w));
+      } else if (b.dec_err) {  // one column at most: only the solo test settles such a code's shots
+#pragma unroll 1
+        for (int c = lane; c < cd.m; c += 32)
+          b.dec_err[(size_t)sj * cd.m + c] = w && c == (int)key ? 1 : 0;
       }
-      const uint32_t *rj = F.row[j];
-      uint32_t eb = 0u;
-      if (code.family == kDem) {
-        if (lane < code.nlw) eb = rj[kRowLog + lane];
-      } else if (code.input_kind == kInErrors) {
-        if (!code.packed && !one_run) {  // a later run took its bits' place
-          at_j = flat_ballots(b.in + rb_j, code.m, F.bits);
-          __syncwarp();
-        }
-        const int rem = code.m - 32 * lane;
-        if (rem > 0)
-          eb = code.packed ? __ldcg(reinterpret_cast<const uint32_t *>(b.in) + rb_j + lane) &
-                                 (rem < 32 ? (1u << rem) - 1u : kFull)
-                           : flat_word(F.bits, at_j, lane, code.m);
+      if (b.dec_log && cd.family == kDem) {
+        uint32_t le = 0u;
+#pragma unroll 1
+        for (int k = 0; k < w && lane < cd.nlw; ++k)
+          le ^= __ldg(cd.lcols + (w == 1 ? (unsigned)key : set_col(key, w, k)) * (unsigned)cd.nlw +
+                      (unsigned)lane);
+        bits_to_bytes(b.dec_log + (size_t)sj * cd.n_logicos, cd.n_logicos, le);
       }
-      const int r = guided_shot<MLK>(b, code, F.shot[j], area->guided, lane < kFastWords ? rj[lane] : 0u,
-                                     rj[kRowSketch], eb, (int)rj[kRowWeight], global_ns());
-      if (r) {
-        slow &= ~(1u << j);
-        ++st.guided;
-        st.heavy += r - 1;
-      }
-    }
-    if (b.guided == kGuidedAll) {
-      if (slow && lane == 0) atomicOr(b.status, kStatusWaitLimit);  // never: see guided_closed
-      return;
     }
   }
-
-  // ---- what is left: the slow queue -------------------------------------------
+  if (b.guided == kGuidedAll) {
+    if (slow && lane == 0) atomicOr(b.status, kStatusWaitLimit);  // never: see guided_closed
+    return;
+  }
   unsigned long long base = 0;
   if (lane == 0)
     base = atomicAdd(ctr_ptr(b.counters, kCtrChunks), (1ull << 32) + (unsigned long long)__popc(slow));
   if (slow) {
     base = __shfl_sync(kFull, base, 0) & 0xffffffffull;
-    if ((slow >> lane) & 1u) {
+    if (open) {
       // its record's bits for the per-shot path, in place of a second read of the caller's
-      const bool cache = b.rec_cache && ok && !packed && one_run &&
-                         nwords + (dem ? cd.nlw : 0) <= kRecCacheWords;
+      const int ci = F.code[lane];
+      const HotCode &cd = hot && ci < kHotCodes ? hot[ci] : static_cast<const HotCode &>(b.codes[ci]);
+      const int nbits = cd.input_kind == kInErrors ? cd.m : cd.R, nwords = (nbits + 31) >> 5;
+      const int nlw = cd.family == kDem ? cd.nlw : 0, at = F.at[lane];
+      const bool cache = b.rec_cache && at >= 0 && nwords + nlw <= kRecCacheWords;
       if (cache) {
         uint32_t *cp = b.rec_cache + (size_t)slot * kRecCacheWords;
 #pragma unroll 1
         for (int q = 0; q < nwords; ++q) cp[q] = flat_word(F.bits, at, q, nbits);
 #pragma unroll 1
-        for (int k = 0; k < cd.nlw && dem; ++k) cp[nwords + k] = row[kRowLog + k];
+        for (int k = 0; k < nlw; ++k) cp[nwords + k] = F.row[lane][kRowLog + k];
       }
       // the entry carries this launch's tag: a ticket holder that reads it knows it
       // is not a leftover of an earlier launch
@@ -462,61 +484,6 @@ __device__ __forceinline__ void classify_chunk(const DevBatch &b, int chunk, int
     }
   }
   __syncwarp();
-}
-
-// A load whose value nothing uses, for the line it brings into L1.
-__device__ __forceinline__ void touch_line(const void *p) {
-#ifdef GRAND_HOST_EMULATION
-  (void)p;
-#else
-  unsigned x;
-  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(x) : "l"(p));
-#endif
-}
-constexpr int kWarmCodes = 8;   // codes whose tables are fetched ahead (about 60 KB for the BB codes)
-constexpr int kWarmTam = 192;   // active sets whose binomials are
-
-// One warp per chunk of the batch.
-constexpr int kChunkWarps = 4;
-// Resident blocks per SM: 5 leave a thread 96 registers and the SM about 130 KB of L1.
-// Measured (4 / 5 / 6 / 8 blocks): headline batch 47.8 / 48.4 / 52.2 / 59.2 us, noisy
-// [[288]] 103 / 92 / 101 / 122 us, ML DEM 279 / 299 / 309 / 301 us, mix 126 / 125 / 125 /
-// 138 us.
-constexpr int kChunkMinBlocks = 5;
-
-template <bool MLK>
-__global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kernel(const DevBatch b) {
-  __shared__ ChunkArea areas[kChunkWarps];
-  const int wib = threadIdx.x >> 5;
-  const unsigned long long chunk = (unsigned long long)blockIdx.x * kChunkWarps + (unsigned)wib;
-  if (chunk * (unsigned)b.chunk >= (unsigned long long)b.num_shots) return;
-  // The first blocks of an SM find its L1 empty: one load per 128-byte line of the codes'
-  // tables, and of the binomials of small sets, starts them on their way together, in
-  // place of one miss after another along the search's chains.
-  {
-    const int stride = kChunkWarps * 32;
-    for (int k = 0; k < b.num_codes && k < kWarmCodes; ++k) {
-      const DevCode &cd = b.codes[k];
-      const int lines = cd.g_gs ? (cd.g_words + 31) >> 5 : 0;
-      for (int i = threadIdx.x; i < lines; i += stride) touch_line(cd.g_rows + 32 * i);
-    }
-    for (int i = threadIdx.x; i < kWarmTam * (kMaxW + 1) / 16; i += stride) touch_line(b.ncr + 16 * i);
-  }
-  const unsigned tag = *reinterpret_cast<volatile unsigned *>(b.epoch) + 1u;
-  const unsigned long long t_enter = b.profile ? global_ns() : 0ull;
-  ChunkStats st{0, 0, 0};
-  classify_chunk<MLK, true>(b, (int)chunk, b.chunk, areas[wib].fast, &areas[wib], st, tag);
-  if ((threadIdx.x & 31) == 0) {
-    add_stats(b, st);
-    if (b.profile) {
-      const unsigned long long t = global_ns();
-      unsigned long long *ends = ctr_ptr(b.counters, kCtrProfEnds);
-      atomicMax(ends + kProfStart, ~t_enter);
-      atomicMax(ends + kProfChunk, t);
-      atomicAdd(ctr_ptr(b.counters, kCtrProfSums) + kProfChunk, t - t_enter);
-      atomicAdd(ctr_ptr(b.counters, kCtrProfSums) + kProfSteps, 1ull);
-    }
-  }
 }
 
 }  // namespace grand

@@ -58,12 +58,19 @@ constexpr int kGuidedMaxCols = 1024;
 constexpr int kGuidedMaxColWeight = 7;
 constexpr int kGuidedMaxDegree = 64;
 constexpr int kGuidedF = 15;            // filter bits, log2 (4 KB)
-// Launch slots per chunk at most (one lane each), and the ballot words of a chunk's records
-// (8192 int32 entries): what keeps a warp's shared memory small enough that half of the
-// SM's storage stays L1 for the code tables.
-constexpr int kMaxChunk = 16;
+// Launch slots per chunk at most (one lane each; 16 / 24 / 32: mix 79 / 63 / 64 us, sampled
+// ML DEM 231 / 232 / 216 us), and the ballot words of a chunk's records (8192 int32
+// entries): what keeps a warp's shared memory small enough that some of the SM's storage
+// stays L1 for the code tables.
+constexpr int kMaxChunk = 32;
 constexpr int kFastBallots = 256;
-constexpr int kGuidedItems = 344;       // partial sets a search holds (all its levels)
+constexpr int kGuidedLanes = 8;         // lanes that search a shot (a warp searches 32 / 8 at once)
+constexpr int kGuidedItems = 512;       // partial sets a warp's searches hold (a shot: 1/4 of them, or
+                                        // all when the warp searches it alone)
+constexpr int kHotCodes = 8;            // codes a block of the chunk kernel copies to shared memory
+constexpr int kChunkWarps = 4;          // warps per block of the chunk kernel
+constexpr int kChunkMinBlocks = 4;      // its resident blocks per SM (3 / 4 / 5: mix 93 / 77 / 81 us,
+                                        // noisy [[288]] 60 / 52 / 61 us)
 constexpr unsigned kNoCol = 0xffffu;    // no column (adjacency padding, empty table slot)
 constexpr unsigned kSoloFlag = 0x10000u;
 
@@ -148,42 +155,51 @@ GRAND_HD inline unsigned long long *ctr_ptr(unsigned long long *counters, int k)
   return counters + k * kCtrStride;
 }
 
-// Immutable per-code tables plus the per-call search parameters.
-struct DevCode {
-  int R, m, nw, nwp, mw;
-  int max_soma, regular;
+// What the chunk step and the guided search read of a code (their blocks keep a copy in
+// shared memory).
+struct HotCode {
+  int R, m, nw, mw;
+  int max_soma;
   int family, variant, input_kind;
-  int W, Wc;                 // configured weight and min(W, 6)
+  int Wc;                    // min(configured weight, 6)
   int mode, thr, cap;        // mode_of_search, threshold_for_hybrid, max_size_active_positions
   int num_phases, n_masks;
-  int mask_tam_upper[kMaxMasks];
-  int mask_order[kMaxMasks][3];
   int n_logicos, nlw;
-  int rank;                  // rank of RREF(H_other), CSS
   int rec_len;               // int32 entries (or packed words) per shot record
   int packed;                // 1: records are bit-packed uint32 words (bit i of word k =
                              // entry 32k + i): ceil(R/32) syndrome / detector words (then
                              // ceil(n_logicos/32) logical words for DEM), ceil(m/32) error words
-  const uint32_t *cols;      // m * nwp
-  const int *colw;           // m
-  const uint32_t *rows;      // R * mw (CSS, errors input)
-  const uint32_t *rref;      // rank * mw
-  const int *pivrow;         // m: RREF row whose pivot is column c, or -1
-  const uint32_t *lcols;     // m * nlw
-  const float *llr;          // m
-  const uint32_t *hcol;      // m column sketches
-  int binary;                // every entry of H is 0 or 1 (column weights are popcounts)
-  const uint32_t *solo_keys; // solo columns (nonzero, containing no other nonzero column)
-  const int *solo_cols;      //   by sketch: open addressing, column -1 = empty slot
-  uint32_t solo_mask;        //   (solo_cols nullptr: no table)
+  int nwp;                   // words per column of cols
   int solo_branch;           // how a first iteration of one position is searched (solo_branch_of)
   // guided search (grand_guided_tables.h); g_gs = 0: the code has none
   int g_gs, g_deg, g_max_cw; // words per packed column, largest row degree, largest column weight
+  int g_odd;                 // every nonzero column has odd weight
   uint32_t g_tab_mask;
   int g_words;                 // the tables lie in one block of g_words words from g_rows on
   unsigned long long g_magic;  // ceil(2^32 / g_deg)
   const uint32_t *g_rows, *g_cw, *g_cols, *g_filt, *g_tab, *g_hcol;
   const uint16_t *g_adj;
+  const uint32_t *lcols;     // m * nlw
+  const float *llr;          // m
+};
+
+// Immutable per-code tables plus the per-call search parameters.
+struct DevCode : HotCode {
+  int regular;
+  int W;                     // configured weight
+  int mask_tam_upper[kMaxMasks];
+  int mask_order[kMaxMasks][3];
+  int rank;                  // rank of RREF(H_other), CSS
+  const uint32_t *cols;      // m * nwp
+  const int *colw;           // m
+  const uint32_t *rows;      // R * mw (CSS, errors input)
+  const uint32_t *rref;      // rank * mw
+  const int *pivrow;         // m: RREF row whose pivot is column c, or -1
+  const uint32_t *hcol;      // m column sketches
+  int binary;                // every entry of H is 0 or 1 (column weights are popcounts)
+  const uint32_t *solo_keys; // solo columns (nonzero, containing no other nonzero column)
+  const int *solo_cols;      //   by sketch: open addressing, column -1 = empty slot
+  uint32_t solo_mask;        //   (solo_cols nullptr: no table)
 };
 
 // One searched weight block of one threshold iteration.
@@ -289,6 +305,7 @@ struct DevBatch {
   unsigned char *dec_log;        // num_shots x n_logicos or nullptr
   float *ml_cost;                // num_shots or nullptr
   const unsigned long long *ncr; // (kMaxTam + 1) x (kMaxW + 1)
+  const unsigned long long *upto; // (kGuidedMaxCols + 1) x 8: C(n, 1) + .. + C(n, k) at [8n + k], k <= 6
   Job *jobs;
   int max_jobs;
   unsigned long long *counters;  // control words (enum Counter)

@@ -182,7 +182,9 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
     const unsigned long long t_step = b.profile ? global_ns() : 0ull;
     a0 = __shfl_sync(kFull, a0, 0);
     if (step == kStepChunk) {
-      classify_chunk<MLK, false>(b, (int)a0, chunk, *reinterpret_cast<FastArea *>(&A), nullptr, st, tag);
+      FastArea &F = *reinterpret_cast<FastArea *>(&A);
+      classify_chunk<MLK>(b, nullptr, (int)a0, chunk, F, st);
+      write_chunk(b, nullptr, (int)a0, chunk, F, tag);
       cache.stage_lost();
     } else if (step == kStepShot) {
       a1 = __shfl_sync(kFull, a1, 0);
@@ -225,19 +227,5 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
       *reinterpret_cast<volatile unsigned *>(b.epoch) = tag;
   }
 }
-
-#ifndef GRAND_HOST_EMULATION
-// The kernels of one batch: the chunk kernel (a warp per chunk) where codes of the batch
-// have a guided search, the decode kernel (grid blocks) unless that leaves it nothing.
-template <bool MLK>
-inline cudaError_t launch_kernels(const DevBatch &b, int grid, cudaStream_t s) {
-  if (b.guided) {
-    const int chunks = (b.num_shots - 1) / b.chunk + 1;
-    chunk_kernel<MLK><<<(chunks + kChunkWarps - 1) / kChunkWarps, kChunkWarps * 32, 0, s>>>(b);
-  }
-  if (b.guided != kGuidedAll) decode_kernel<MLK><<<grid, kDecodeWarps * 32, 0, s>>>(b);
-  return cudaGetLastError();
-}
-#endif
 
 }  // namespace grand

@@ -1,6 +1,7 @@
 // grand_decode_ml.cu -- the decode kernel built with the ML (cost-ordered)
 // search paths, for batches with an ML code.
 #include "grand_decode.cuh"
+#include "grand_front.cuh"
 #include "grand_host.h"
 
 namespace grand {

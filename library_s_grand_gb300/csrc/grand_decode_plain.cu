@@ -2,6 +2,7 @@
 // code, fewer registers), for batches without an ML code; and the launcher that
 // picks the build.
 #include "grand_decode.cuh"
+#include "grand_front.cuh"
 #include "grand_host.h"
 
 namespace grand {
@@ -9,8 +10,6 @@ namespace grand {
 #ifndef GRAND_HOST_EMULATION
 cudaError_t launch_decode_ml(const DevBatch &b, int grid, cudaStream_t s);
 cudaError_t decode_occupancy_ml(int *blocks_per_sm);
-
-int chunk_warps_per_sm() { return kChunkMinBlocks * kChunkWarps; }
 
 cudaError_t launch_decode(const DevBatch &b, int grid, cudaStream_t s) {
   if (b.has_ml) return launch_decode_ml(b, grid, s);

@@ -257,6 +257,7 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   b.shot_code = d_shot_code;
   b.results = d_results;
   b.ncr = e->ctx->d_ncr;
+  b.upto = e->ctx->d_upto;
   b.jobs = (Job *)slot->d_jobs;
   b.max_jobs = max_jobs;
   b.counters = (unsigned long long *)slot->d_small;

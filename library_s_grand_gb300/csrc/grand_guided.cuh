@@ -1,4 +1,4 @@
-// grand_guided.cuh -- the guided search of one shot by one warp (sm_103a).
+// grand_guided.cuh -- the guided search, four shots to a warp (sm_103a).
 //
 // A set S of active columns matches when the XOR of its columns is the syndrome
 // s.  Take any set row r of s: an odd number of S's columns hold r, so at least
@@ -19,89 +19,57 @@
 // LLR then column) with ties to the smaller index set.  Its rank in the enumeration,
 // and with it the number of candidates upstream reports, follow from its positions.
 //
-// Levels.  The partial sets of one size lie side by side in shared memory ("items":
-// the item extended and the column added, the residual's sketch and lowest row).  Level d extends the
-// items of d - 1 columns by one: lanes take (item, neighbour) pairs, so a level
-// of n items is n * deg / 32 steps whatever the shape of the tree; each new set
-// probes the sketch filter for its last column (weight d + 1) and, while larger
-// weights remain, is kept for the next level.  A level that outgrows the area
-// gives the shot to the general path.
+// Levels.  The partial sets of one size, of all the warp's shots, lie side by side in
+// shared memory ("items": the item extended and the column added, the residual's sketch
+// and lowest row, the shot).  Level d extends the items of d - 1 columns by one: the
+// warp's lanes take (item, neighbour) pairs, so a level of n items is n * deg / 32
+// steps whatever the shape of the trees; each new set probes the sketch filter for its
+// last column (weight d + 1) and, while larger weights remain, is kept for the next
+// level.  Shots whose levels together outgrow the items are searched again one by one;
+// one that outgrows them alone takes the general path.
 //
 // The flagged-check counts (upstream grand_decoder.cu:67-81, 406-416) are formed
-// from the rows: lane q holds mask word q of the columns, the rows of H selected by
+// from the rows: a lane holds a mask word of the columns, the rows of H selected by
 // the syndrome are added into 3-bit counters kept as bit slices, and a column is
 // active in iteration i when at most i of its rows are missing from the syndrome
 // (its count, with the irregular offset, reaches max_soma - i).
 //
-// What bounds it: latency and the instruction caches.  A shot's work is some hundred
-// instructions in a chain of L1 round trips (row words, adjacency, columns, filter),
-// run once per shot by warps that are all somewhere else in it, so the code is
-// kept small: loops stay rolled, column widths are a run-time choice and the rare
-// parts are out of line.  Against the prefix-lookup search in Jobs (grand_lookup.cuh)
-// that did this before: 20000 noisy [[288]] shots, W = 4, 957 -> 92 us; 8192 random
-// detector records of the 120 x 720 DEM 562 -> 40 us.
+// What bounds it: the instruction chain (some 11 cycles an instruction per warp, L1 round
+// trips among them) and the instruction caches.  Most of a shot's instructions are
+// uniform -- planning, loop control, reductions -- so eight lanes take a shot and a
+// warp takes four, in step; the code is kept small: loops stay rolled, column widths
+// are a run-time choice and the rare parts are out of line.  TIMES
 #pragma once
 
-#include "grand_kernels.cuh"
+#include "grand_chunk.cuh"
 
 namespace grand {
 
-// x: the residual's sketch; y: the item it extends (10 bits), the column added (10) and
-// the residual's lowest row (10, kNoRow: zero).
+// One shot of the warp: its syndrome, the active columns of its iterations, and what the
+// lanes that extend its sets read of its code.
+struct alignas(16) GuidedGroup {
+  uint32_t sw[8];                    // the syndrome, zero past nw
+  uint32_t am[kMaxIters][32];        // the iterations' active columns
+  const uint32_t *cols, *hcol, *filt, *tab;
+  const uint16_t *adj;
+  const float *llr;                  // nullptr: first-hit search
+  uint32_t tab_mask;
+  int deg, m;
+  int limit;                         // most set rows a residual of this level may have
+  int wide;                          // more than 128 rows: columns of eight words
+  alignas(4) uint8_t rows[kGuidedMaxRows + 5];  // the syndrome's set rows, ascending, padded with R
+};
+// An item: x: the residual's sketch; y: the item it extends (10 bits), the column added
+// (10), the residual's lowest row (10, kNoRow: zero) and the group (2).
 struct alignas(16) GuidedArea {
   uint2 item[kGuidedItems];
-  uint32_t sw[8];                // the syndrome, zero past nw
-  uint32_t am[32];               // the searched iteration's active columns
-  uint8_t rows[kGuidedMaxRows + 4];  // the syndrome's set rows, ascending, padded with R
+  GuidedGroup group[32 / kGuidedLanes];
 };
 constexpr unsigned kNoRow = 1023u;
-static_assert(kGuidedItems <= 1024 && kGuidedMaxCols <= 1024 && kGuidedMaxRows < (int)kNoRow,
-              "an item's fields have 10 bits each");
+static_assert(kGuidedItems <= 1024 && kGuidedMaxCols <= 1024 && kGuidedMaxRows < (int)kNoRow &&
+                  32 / kGuidedLanes <= 4,
+              "an item's fields have 10 bits each, its group 2");
 
-__device__ __forceinline__ uint32_t warp_xor(uint32_t v) {
-#ifdef GRAND_HOST_EMULATION
-  for (int o = 16; o > 0; o >>= 1) v ^= __shfl_xor_sync(kFull, v, o);
-  return v;
-#else
-  return __reduce_xor_sync(kFull, v);
-#endif
-}
-__device__ __forceinline__ int warp_add(int v) {
-#ifdef GRAND_HOST_EMULATION
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-  return v;
-#else
-  return __reduce_add_sync(kFull, v);
-#endif
-}
-
-// One code's tables and the search's state, uniform over the warp.
-struct GuidedView {
-  const uint32_t *cols, *filt, *tab;
-  const uint16_t *adj;
-  const uint32_t *hcol;
-  const float *llr;          // nullptr: first-hit search
-  uint32_t tab_mask;
-  unsigned long long magic;  // ceil(2^32 / deg): p * magic >> 32 = p / deg for p < 2^26
-  int deg, max_cw, m;
-  bool wide;                 // more than 128 rows: columns of eight words
-};
-
-// A residual syndrome: the second half is used by codes of more than 128 rows (wide).
-struct Resid {
-  uint4 a, b;
-};
-__device__ __forceinline__ void xor_into(uint4 &r, const uint4 w) {
-  r.x ^= w.x;
-  r.y ^= w.y;
-  r.z ^= w.z;
-  r.w ^= w.w;
-}
-__device__ __forceinline__ void xor_col(const uint32_t *cols, bool wide, unsigned c, Resid &r) {
-  const uint4 *p = reinterpret_cast<const uint4 *>(cols) + (c << (wide ? 1 : 0));
-  xor_into(r.a, __ldg(p));
-  if (wide) xor_into(r.b, __ldg(p + 1));
-}
 // The columns of a partial set, 16 bits each from the lowest up (the rest kNoCol).
 struct Path {
   uint32_t lo, hi;
@@ -155,10 +123,6 @@ struct GuidedBest {
   unsigned long long key;
   uint32_t cost;
 };
-
-__device__ __forceinline__ unsigned set_col(unsigned long long key, int w, int e) {
-  return (unsigned)(key >> (10 * (w - 1 - e))) & 1023u;
-}
 
 // ML: is index set a before b in the enumeration (both in list order)?
 __device__ __forceinline__ bool ml_set_before(const float *llr, unsigned long long a,
@@ -222,23 +186,24 @@ __device__ __noinline__ GuidedBest guided_match(const uint32_t *sw, const uint32
 // The active columns outside the set whose sketch is h, each tested as the last
 // column of the set {the d columns of p, c}.
 template <bool MLK>
-__device__ __forceinline__ void guided_probe(const GuidedArea &G, const GuidedView &v, const Path &p,
+__device__ __forceinline__ void guided_probe(const GuidedGroup &S, const uint32_t *am, const Path &p,
                                              int d, unsigned c, uint32_t h, GuidedBest &best) {
   const uint32_t f = h >> (32 - kGuidedF);
-  if (!((__ldg(v.filt + (f >> 5)) >> (f & 31u)) & 1u)) return;
-  uint32_t i = h & v.tab_mask;
+  if (!((__ldg(S.filt + (f >> 5)) >> (f & 31u)) & 1u)) return;
+  const uint32_t mask = S.tab_mask;
+  uint32_t i = h & mask;
 #pragma unroll 1
-  for (uint32_t guard = 0; guard <= v.tab_mask; ++guard) {
-    const uint2 e = __ldg(reinterpret_cast<const uint2 *>(v.tab) + i);
+  for (uint32_t guard = 0; guard <= mask; ++guard) {
+    const uint2 e = __ldg(reinterpret_cast<const uint2 *>(S.tab) + i);
     const unsigned j = e.y & 0xffffu;
     if (j == kNoCol) return;
-    if (e.x == h && j != c && !in_path(p, j) && ((G.am[j >> 5] >> (j & 31u)) & 1u))
-      best = guided_match<MLK>(G.sw, v.cols, v.wide, v.llr, p, d, c, j, best);
-    i = (i + 1u) & v.tab_mask;
+    if (e.x == h && j != c && !in_path(p, j) && ((am[j >> 5] >> (j & 31u)) & 1u))
+      best = guided_match<MLK>(S.sw, S.cols, S.wide != 0, MLK ? S.llr : nullptr, p, d, c, j, best);
+    i = (i + 1u) & mask;
   }
 }
 
-// What the search found (uniform over the warp).
+// What the search found for a group's shot.
 struct GuidedWinner {
   int w;                    // 0: nothing
   unsigned long long key;   // its columns, in list order
@@ -246,178 +211,12 @@ struct GuidedWinner {
   int w_done;               // ML: last weight searched (the bound may stop it early)
 };
 
-// FP32 sum of the w smallest LLRs of the active columns (the bound of weight w):
-// upstream's prefix sums add them in ascending order.
-static __device__ __noinline__ float ml_prefix(const uint32_t *am, const float *llr, int m, int w) {
-  const int lane = threadIdx.x & 31;
-  float sum = 0.0f;
-  unsigned long long last = 0ull;  // {LLR key, column} of the smallest taken so far, plus one
-#pragma unroll 1
-  for (int e = 0; e < w; ++e) {
-    unsigned long long best = kNone;
-#pragma unroll 1
-    for (int c0 = 0; c0 < m; c0 += 32) {
-      const int c = c0 + lane;
-      if ((am[c0 >> 5] >> lane) & 1u) {  // bits past m are 0
-        const uint32_t u = __float_as_uint(__ldg(llr + c));
-        const uint32_t k = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-        const unsigned long long x = ((unsigned long long)k << 32) | (unsigned)c;
-        if (x >= last && x < best) best = x;
-      }
-    }
-    best = warp_min_u64(best);
-    if (best == kNone) break;
-    const uint32_t k = (uint32_t)(best >> 32);
-    sum = __fadd_rn(sum, __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k));
-    last = best + 1ull;
-  }
-  return sum;
-}
-
-// Weights w_first .. w_last of the active set G.am in ascending order, to the first
-// weight with a match (ML: to the bound).  hs: the syndrome's sketch, ones / row0: its
-// number of set rows and its lowest.  Returns false when a level does not fit.
-//
-// Weight w is searched while its level is formed: every item of w - 2 columns is
-// extended by one (items lo .. hi), each new set probes for its last column, and,
-// while larger weights remain, sets that can still reach weight w_last are kept from
-// index hi on.
-template <bool MLK>
-__device__ __forceinline__ bool guided_search(GuidedArea &G, const GuidedView &v, uint32_t hs,
-                                              int ones, unsigned row0, int w_first, int w_last,
-                                              GuidedWinner &wn) {
-  const int lane = threadIdx.x & 31;
-  const bool ml = MLK && v.llr != nullptr;
-  wn.w = 0;
-  wn.key = kNone;
-  wn.cost = 0xffffffffu;
-  wn.w_done = w_last;
-  if (ones > v.max_cw * w_last) return true;  // no w_last columns hold that many rows
-  const Path none{0xffffffffu, 0xffffffffu};
-  if (lane == 0) G.item[0] = make_uint2(hs, row0);
-  __syncwarp();
-  int lo = 0, hi = 1;
-#pragma unroll 1
-  for (int w = 1; w <= w_last; ++w) {
-    if (MLK && ml && wn.w && ml_prefix(G.am, v.llr, v.m, w) >= key_cost(wn.cost)) {
-      wn.w_done = w - 1;
-      return true;
-    }
-    GuidedBest best;
-    best.key = kNone;
-    best.cost = 0xffffffffu;
-    const int d = w - 1;  // columns of the sets formed
-    const bool probe = w >= w_first, push = w < w_last;
-    if (d == 0) {
-      if (probe && lane == 0) guided_probe<MLK>(G, v, none, 0, kNoCol, hs, best);
-    } else {
-      const int pairs = (hi - lo) * v.deg;
-      int top = hi;
-      int z = -1;  // an item of residual zero being extended (by every active column), -1: none yet
-      unsigned zeros = 0u;
-      // steps of 32 (item, neighbour) pairs, then, for each item without a row to
-      // follow, steps of 32 columns
-#pragma unroll 1
-      for (int p0 = 0;; p0 += 32) {
-        int i = lo;
-        unsigned c = kNoCol;
-        uint2 it = make_uint2(0u, 0u);
-        if (z < 0 && p0 < pairs) {
-          const int p = p0 + lane;
-          if (p < pairs) {
-            const int q = (int)(((unsigned long long)(unsigned)p * v.magic) >> 32);
-            i = lo + q;
-            it = G.item[i];
-            const unsigned row = it.y & 1023u;
-            if (row != kNoRow) c = __ldg(v.adj + row * (unsigned)v.deg + (unsigned)(p - q * v.deg));
-            else zeros = 1u;
-          }
-        } else {
-          if (z < 0 || p0 >= v.m) {
-            if (z < 0 && !__any_sync(kFull, zeros != 0u)) break;  // (ML, or weights out of order)
-            z = z < 0 ? lo : z + 1;
-            while (z < hi && (G.item[z].y & 1023u) != kNoRow) ++z;
-            if (z >= hi) break;
-            p0 = 0;
-          }
-          i = z;
-          it = G.item[z];
-          if (p0 + lane < v.m) c = (unsigned)(p0 + lane);
-        }
-        // one child per lane: column c after item i, if active and not in it
-        bool live = c != kNoCol && ((G.am[(c >> 5) & 31u] >> (c & 31u)) & 1u);
-        Path path = none;
-        if (live) {
-          it.x ^= __ldg(v.hcol + c);
-          uint32_t up = it.y;
-#pragma unroll 1
-          for (int e = d - 1; e > 0; --e) {
-            push_col(path, (up >> 10) & 1023u);
-            up = G.item[up >> 20].y;
-          }
-          live = !in_path(path, c);
-          if (live && probe) guided_probe<MLK>(G, v, path, d - 1, c, it.x, best);
-        }
-        if (push) {
-          if (live) {
-            const Resid r = residual(G.sw, v.cols, v.wide, path, d - 1, c);
-            it.y = ((unsigned)i << 20) | (c << 10) | lowest_row(r);
-            live = ones_of(r) <= v.max_cw * (w_last - d);
-          }
-          const unsigned keep = __ballot_sync(kFull, live);
-          const int at = top + __popc(keep & ((1u << lane) - 1u));
-          top += __popc(keep);
-          if (top > kGuidedItems) return false;
-          if (live) G.item[at] = it;
-        }
-      }
-      __syncwarp();
-      lo = hi;
-      hi = top;
-    }
-    if (__any_sync(kFull, best.key != kNone)) {
-      if (!ml) {
-        wn.w = w;
-        wn.key = warp_min_u64(best.key);
-        return true;
-      }
-      const uint32_t o = __reduce_min_sync(kFull, best.cost);
-      unsigned who = __ballot_sync(kFull, best.key != kNone && best.cost == o);
-      unsigned long long key = __shfl_sync(kFull, best.key, __ffs((int)who) - 1);
-#pragma unroll 1
-      for (who &= who - 1u; who; who &= who - 1u) {
-        const unsigned long long k2 = __shfl_sync(kFull, best.key, __ffs((int)who) - 1);
-        if (ml_set_before(v.llr, k2, key, w)) key = k2;
-      }
-      if (!wn.w || o < wn.cost) {
-        wn.w = w;
-        wn.key = key;
-        wn.cost = o;
-      }
-    }
-    if (lo == hi && w > 1 && !wn.w) break;  // nothing left to extend
-  }
-  return true;
-}
-
 // x added to the counters of each bit position.
 __device__ __forceinline__ void add_bits(uint32_t x, uint32_t &c0, uint32_t &c1, uint32_t &c2) {
   const uint32_t t = c0 & x;
   c0 ^= x;
   c2 ^= c1 & t;
   c1 ^= t;
-}
-
-// Exclusive prefix sum over the lanes.
-__device__ __forceinline__ int lanes_before(int v) {
-  const int lane = threadIdx.x & 31;
-  int sum = v;
-#pragma unroll 1
-  for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(kFull, sum, o);
-    if (lane >= o) sum += u;
-  }
-  return sum - v;
 }
 
 // Are the bits of delta (word `lane` of the difference of two errors with one syndrome)
@@ -448,272 +247,557 @@ static __device__ __noinline__ bool in_row_space(const DevCode &cd, uint32_t del
   return __all_sync(kFull, acc == delta);
 }
 
-// out[0 .. n) = the bits of word `lane` of a vector, one byte each.
-__device__ __forceinline__ void bits_to_bytes(unsigned char *out, int n, uint32_t word) {
+// Word `lane` of a supplied error (CSS): from its chunk's ballots (at >= 0) or from the
+// record itself.
+static __device__ __noinline__ uint32_t error_word(const DevBatch &b, const HotCode &cd, const FastArea &F,
+                                                   int at, int shot) {
   const int lane = threadIdx.x & 31;
+  const int rem = cd.m - 32 * lane;
+  if (at >= 0) return rem > 0 ? flat_word(F.bits, at, lane, cd.m) : 0u;
+  const int *rec = b.in + (b.in_off ? b.in_off[shot] : (long long)shot * cd.rec_len);
+  if (cd.packed)
+    return rem > 0 ? (unsigned)__ldcg(rec + lane) & (rem < 32 ? (1u << rem) - 1u : kFull) : 0u;
+  uint32_t mine = 0u;
 #pragma unroll 1
-  for (int c0 = 0; c0 < n; c0 += 32) {
-    const uint32_t w = __shfl_sync(kFull, word, c0 >> 5);
-    if (c0 + lane < n) out[c0 + lane] = (unsigned char)((w >> lane) & 1u);
+  for (int q = 0; 32 * q < cd.m; ++q) {
+    const uint32_t w = __ballot_sync(kFull, 32 * q + lane < cd.m && __ldcg(rec + 32 * q + lane) != 0);
+    if (q == lane) mine = w;
   }
+  return mine;
 }
 
-// One shot, start to finish, by one warp: the threshold iterations in upstream's order
-// (grand_decoder.cu:1284-1343) until one has a match, and the shot's result.
-// s_lane: syndrome word `lane` (0 past nw), not all zero; hs: its sketch; eb_lane: word
-// `lane` of the supplied error (CSS) or of the true logical flips (DEM), 0 past the
-// last.  Returns 1 when done, 2 when done and past the light budget, 0 when the shot
-// needs the general path (nothing has been written).
+// cnt (1 .. 4) open shots of the block: the threshold iterations in upstream's order
+// (grand_decoder.cu:1284-1343) until one has a match, and the shot's result into its row.
+// An entry is (warp of the block << 8) | lane of its chunk.  Returns the mask of the shots
+// finished (bit k: entry k; none of them when the levels do not fit), and in bits 8 .. those
+// past the light budget.
+//
+// Eight lanes (a group) count, plan and report for one shot; the sets are extended by
+// all lanes for all of them.  The groups run in step: every loop goes on while some group
+// needs it, and a collective of the warp serves all of them.
 template <bool MLK>
-__device__ __forceinline__ int guided_shot(const DevBatch &b, const DevCode &cd, int shot, GuidedArea &G,
-                                        uint32_t s_lane, uint32_t hs, uint32_t eb_lane,
-                                        int original_weight, unsigned long long t_start) {
+__device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, GuidedArea &A,
+                                        FastArea *areas, size_t area_step, const uint16_t *list,
+                                        int cnt) {
+  constexpr int G = kGuidedLanes;
+  constexpr unsigned kGroup = (1u << G) - 1u;
   const int lane = threadIdx.x & 31;
+  const int g = lane / G, gl = lane & (G - 1), gb = g * G;
+  GuidedGroup &S = A.group[g];
+  uint2 *item = A.item;
+  const unsigned long long t_start = global_ns();
+  unsigned long long tp = b.profile ? t_start : 0ull;
+  bool live = g < cnt;
+  const int entry = live ? (int)list[g] : 0;
+  FastArea &F = *reinterpret_cast<FastArea *>(reinterpret_cast<char *>(areas) + (entry >> 8) * area_step);
+  const int j = entry & 255;
+  uint32_t *row = F.row[j];
+  const int ci = F.code[j];
+  const DevCode &full = b.codes[ci];
+  const HotCode &cd = hot && ci < kHotCodes ? hot[ci] : static_cast<const HotCode &>(full);
   const bool ml = MLK && cd.variant == kMl;
-  const int mw = cd.mw;
-  unsigned long long tp = b.profile ? global_ns() : 0ull;
-
-  // ---- the syndrome and its rows ------------------------------------------------
-  if (lane < 8) G.sw[lane] = s_lane;
-  int ones = 0;
-#pragma unroll 1
-  for (int k = 0; k < cd.nw; ++k) {
-    const uint32_t word = __shfl_sync(kFull, s_lane, k);
-    if ((word >> lane) & 1u) G.rows[ones + __popc(word & ((1u << lane) - 1u))] = (uint8_t)(32 * k + lane);
-    ones += __popc(word);
+  const bool prob = cd.variant == kProb;
+  const int mw = cd.mw, max_cw = cd.g_max_cw;
+  const float *llr = ml ? cd.llr : nullptr;
+  const uint32_t hs = row[kRowSketch];
+  if (gl == 0) {
+    S.cols = cd.g_cols;
+    S.hcol = cd.g_hcol;
+    S.filt = cd.g_filt;
+    S.tab = cd.g_tab;
+    S.adj = cd.g_adj;
+    S.llr = llr;
+    S.tab_mask = cd.g_tab_mask;
+    S.deg = cd.g_deg;
+    S.m = cd.m;
+    S.wide = cd.g_gs == 8 ? 1 : 0;
   }
-  if (lane < 4) G.rows[ones + lane] = (uint8_t)cd.R;  // the row of zeros behind the table's
-  __syncwarp();
+  // the largest row degree of the warp's codes: the pairs an item is given
+  int deg = cd.g_deg;
+  unsigned long long magic = cd.g_magic;
+#pragma unroll 1
+  for (int o = G; o < 32; o <<= 1) {
+    const int d2 = __shfl_xor_sync(kFull, deg, o);
+    const unsigned long long m2 = __shfl_xor_sync(kFull, magic, o);
+    if (d2 > deg) {
+      deg = d2;
+      magic = m2;
+    }
+  }
 
-  // ---- counts, bit-sliced: lane q the columns of mask word q ----------------------
-  const int L = cd.max_soma < kMaxIters ? cd.max_soma : kMaxIters;
-  uint32_t am0 = 0u, am1 = 0u, am2 = 0u;
+  // ---- the syndrome and its rows: lane gl the rows of word gl ----------------------
+  int ones;
   {
-    // up to 8 mask words: four groups of lanes share the rows and add their counts up;
-    // up to 16: two groups; the list ends with rows of zeros
-    const int split = mw <= 8 ? 4 : (mw <= 16 ? 2 : 1);
-    const int q = lane & (32 / split - 1);
-    const int step = 4 * split, part = lane / (32 / split);
-    const uint32_t *rows = cd.g_rows + (q < mw ? q : 0);
-    uint32_t c0 = 0u, c1 = 0u, c2 = 0u;
+    uint32_t word = gl < kFastWords && live ? row[gl] : 0u;
+    if (gl < kFastWords) S.sw[gl] = word;
+    int sum = __popc(word);
+    const int mine = sum;
 #pragma unroll 1
-    for (int i = 4 * part; i < ones; i += step) {
-      const uchar4 r = *reinterpret_cast<const uchar4 *>(G.rows + i);
-      const uint32_t x0 = __ldg(rows + (int)r.x * mw), x1 = __ldg(rows + (int)r.y * mw),
-                     x2 = __ldg(rows + (int)r.z * mw), x3 = __ldg(rows + (int)r.w * mw);
-      add_bits(x0, c0, c1, c2);
-      add_bits(x1, c0, c1, c2);
-      add_bits(x2, c0, c1, c2);
-      add_bits(x3, c0, c1, c2);
+    for (int o = 1; o < kFastWords; o <<= 1) {
+      const int u = __shfl_sync(kFull, sum, lane - o);
+      if (gl >= o) sum += u;
     }
-    __syncwarp();
+    ones = __shfl_sync(kFull, sum, gb + kFastWords - 1);
+    int n = sum - mine;
 #pragma unroll 1
-    for (int o = 32 / split; o < 32; o <<= 1) {
-      const uint32_t y0 = __shfl_xor_sync(kFull, c0, o), y1 = __shfl_xor_sync(kFull, c1, o),
-                     y2 = __shfl_xor_sync(kFull, c2, o);
-      const uint32_t t0 = c0 & y0, t1 = (c1 & y1) | (t0 & (c1 ^ y1));
-      c2 ^= y2 ^ t1;
-      c1 ^= y1 ^ t0;
-      c0 ^= y0;
-    }
-    if (lane < mw) {
-      const uint32_t w0 = __ldg(cd.g_cw + lane), w1 = __ldg(cd.g_cw + mw + lane),
-                     w2 = __ldg(cd.g_cw + 2 * mw + lane);
+    for (; word; word &= word - 1u) S.rows[n++] = (uint8_t)(32 * gl + __ffs((int)word) - 1);
+    if (gl < 4) S.rows[ones + gl] = (uint8_t)cd.R;  // the row of zeros behind the table's
+  }
+  __syncwarp();
+  const unsigned row0 = S.rows[0];
+
+  // ---- counts, bit-sliced: lane gl the columns of mask words gl, gl + G, .. ----------
+  const int L = cd.max_soma < kMaxIters ? cd.max_soma : kMaxIters;
+  int t01 = 0, t2 = 0;  // active columns of the iterations (the first two packed)
+#pragma unroll 1
+  for (int q = gl; __any_sync(kFull, live && q < mw); q += G) {
+    if (live && q < mw) {
+      const uint32_t *rows = cd.g_rows + q;
+      uint32_t c0 = 0u, c1 = 0u, c2 = 0u;
+#pragma unroll 1
+      for (int i = 0; i < ones; i += 4) {
+        const uchar4 r = *reinterpret_cast<const uchar4 *>(S.rows + i);
+        const uint32_t x0 = __ldg(rows + (int)r.x * mw), x1 = __ldg(rows + (int)r.y * mw),
+                       x2 = __ldg(rows + (int)r.z * mw), x3 = __ldg(rows + (int)r.w * mw);
+        add_bits(x0, c0, c1, c2);
+        add_bits(x1, c0, c1, c2);
+        add_bits(x2, c0, c1, c2);
+        add_bits(x3, c0, c1, c2);
+      }
+      const uint32_t w0 = __ldg(cd.g_cw + q), w1 = __ldg(cd.g_cw + mw + q), w2 = __ldg(cd.g_cw + 2 * mw + q);
       // missing = weight - count, bit by bit; zero columns are never active
       const uint32_t nz = w0 | w1 | w2;
       const uint32_t m0 = w0 ^ c0, b0 = ~w0 & c0;
       const uint32_t m1 = w1 ^ c1 ^ b0, b1 = (~w1 & c1) | (~(w1 ^ c1) & b0);
       const uint32_t m2 = w2 ^ c2 ^ b1;
-      am0 = nz & ~(m0 | m1 | m2);
-      am1 = nz & ~(m1 | m2);
-      am2 = nz & ~(m2 | (m1 & m0));
+      const uint32_t a0 = nz & ~(m0 | m1 | m2), a1 = nz & ~(m1 | m2), a2 = nz & ~(m2 | (m1 & m0));
+      S.am[0][q] = a0;
+      S.am[1][q] = a1;
+      S.am[2][q] = a2;
+      t01 += __popc(a0) | (__popc(a1) << 16);
+      t2 += __popc(a2);
     }
   }
+#pragma unroll 1
+  for (int o = 1; o < G; o <<= 1) {
+    t01 += __shfl_xor_sync(kFull, t01, o);
+    t2 += __shfl_xor_sync(kFull, t2, o);
+  }
+  __syncwarp();
   const unsigned long long t_counts = global_ns();
   tp = prof_lap(b, kProfShotCounts, tp);
 
-  GuidedView v;
-  v.cols = cd.g_cols;
-  v.filt = cd.g_filt;
-  v.tab = cd.g_tab;
-  v.adj = cd.g_adj;
-  v.hcol = cd.g_hcol;
-  v.llr = ml ? cd.llr : nullptr;
-  v.tab_mask = cd.g_tab_mask;
-  v.deg = cd.g_deg;
-  v.magic = cd.g_magic;
-  v.max_cw = cd.g_max_cw;
-  v.m = cd.m;
-  v.wide = cd.g_gs == 8;
-
   // ---- the iterations --------------------------------------------------------------
-  const bool prob = cd.variant == kProb;
   GuidedWinner wn;
   wn.w = 0;
+  wn.key = kNone;
   int tam = 0, tam_old = 0, passes = 0, hib = -2, heavy = 0, found = 0;
   unsigned long long tested = 0;
 #pragma unroll 1
-  for (int i = 0; i < L && !found; ++i) {
-    passes = i + 1;
-    uint32_t am = am0;
-    am0 = am1;
-    am1 = am2;
-    const int n_act = warp_add(__popc(am));
-    tam = n_act;
-    if (cd.family == kDem) {  // grand_decoder.cu:1550-1554
-      if (tam > cd.cap) tam = tam_old;
-      else tam_old = tam;
-    }
-    if (tam <= 0) continue;
-    const bool gpu = (tam > cd.thr && tam <= cd.cap && cd.mode == 1) || cd.mode == 0;
-    const bool cpu = !gpu && ((tam <= cd.thr && cd.mode == 1) || cd.mode == -1);
-    if (!gpu && !cpu) continue;
-    if (tam < n_act) {  // the first tam columns of the larger set (the cap rule)
-      int left = tam - lanes_before(__popc(am));
-      uint32_t rest = am;
-      am = 0u;
-#pragma unroll 1
-      for (; rest && left > 0; --left) {
-        am |= rest & (0u - rest);
-        rest &= rest - 1u;
+  for (int i = 0; i < kMaxIters; ++i) {
+    bool on = live && !found && i < L;
+    if (!__any_sync(kFull, on)) break;
+    const int n_act = i == 0 ? t01 & 0xffff : (i == 1 ? t01 >> 16 : t2);
+    uint32_t *am = S.am[i];
+    if (on) {
+      passes = i + 1;
+      tam = n_act;
+      if (cd.family == kDem) {  // grand_decoder.cu:1550-1554
+        if (tam > cd.cap) tam = tam_old;
+        else tam_old = tam;
       }
     }
-    G.am[lane] = am;
-    __syncwarp();
-
-    // candidate counts: lane w holds those of weights 1 .. w
-    unsigned long long upto = lane >= 1 ? ncr(b.ncr, tam, lane) : 0ull;
+    const bool gpu = (tam > cd.thr && tam <= cd.cap && cd.mode == 1) || cd.mode == 0;
+    const bool cpu = !gpu && ((tam <= cd.thr && cd.mode == 1) || cd.mode == -1);
+    on = on && tam > 0 && (gpu || cpu);
+    if (__any_sync(kFull, on && tam < n_act)) {
+      // the first tam columns of the larger set (the cap rule)
+      int left = on ? tam : n_act;
 #pragma unroll 1
-    for (int o = 1; o < 8; o <<= 1) {
-      const unsigned long long u = __shfl_up_sync(kFull, upto, o);
-      if (lane >= o) upto += u;
+      for (int q0 = 0; __any_sync(kFull, q0 < mw); q0 += G) {
+        const int q = q0 + gl;
+        uint32_t word = q < mw ? am[q] : 0u;
+        int sum = __popc(word);
+        const int mine = sum;
+#pragma unroll 1
+        for (int o = 1; o < G; o <<= 1) {
+          const int u = __shfl_sync(kFull, sum, lane - o);
+          if (gl >= o) sum += u;
+        }
+        int keep = left - (sum - mine);
+        if (keep < mine && q < mw) {
+          uint32_t cut = 0u;
+#pragma unroll 1
+          for (; keep > 0; --keep) {
+            cut |= word & (0u - word);
+            word &= word - 1u;
+          }
+          am[q] = cut;
+        }
+        left -= __shfl_sync(kFull, sum, gb + G - 1);
+      }
+      __syncwarp();
     }
-    const unsigned long long c15 = __shfl_sync(kFull, upto, 5);
-    const unsigned long long c6 = __shfl_sync(kFull, upto, 6) - c15;
+    // candidate counts: lane k of the group holds those of weights 1 .. k
+    const unsigned long long upto = gl < 8 ? __ldg(b.upto + 8 * tam + gl) : 0ull;
+
     // the weights searched (bit w), in one ascending run or weight 6 (run) before the others
-    unsigned long long total = 0;
-    unsigned ws = 0u, run;
-    int mi = 0;
-    if (prob) {
-      mi = cd.n_masks - 1;  // grand_decoder.cu:754-762
+    unsigned ws = 0u, run = 0u;
+    const int *order = full.mask_order[0];
+    int wmax = cd.Wc < tam ? cd.Wc : tam;
+    if (on && prob) {
+      int mi = cd.n_masks - 1;  // grand_decoder.cu:754-762
 #pragma unroll 1
       for (int q = 0; q < cd.n_masks; ++q)
-        if (tam <= cd.mask_tam_upper[q]) {
+        if (tam <= full.mask_tam_upper[q]) {
           mi = q;
           break;
         }
-      run = 0u;
+      order = full.mask_order[mi];
 #pragma unroll 1
       for (int k = 0; k < cd.num_phases; ++k) {
-        const int pid = cd.mask_order[mi][k];
-        if (pid == 0) {
-          total += c15;
-          ws |= (2u << (tam < 5 ? tam : 5)) - 2u;
-        } else if (pid == 1 && tam >= 6) {
-          total += c6;
+        const int pid = order[k];
+        if (pid == 0) ws |= (2u << (tam < 5 ? tam : 5)) - 2u;
+        if (pid == 1 && tam >= 6) {
           if (!ws) run = 64u;
           ws |= 64u;
         }
       }
       if (!run) run = ws;
-    } else {
-      const int wmax = cd.Wc < tam ? cd.Wc : tam;
-      total = __shfl_sync(kFull, upto, wmax);
+    } else if (on) {
       run = ws = (2u << wmax) - 2u;
     }
-    heavy |= total > (1ull << b.light_max_log2) || tam > kLightTam || tam * cd.nwp > kLightWords;
+    unsigned rest = ws & ~run;
 
+    // ---- the search ------------------------------------------------------------------
 #pragma unroll 1
-    for (unsigned rest = ws & ~run; run; run = rest, rest = 0u) {
-      if (!guided_search<MLK>(G, v, hs, ones, G.rows[0], __ffs((int)run) - 1, 31 - __clz((int)run), wn))
-        return 0;
-      if (wn.w) break;
-    }
-    hib = gpu ? (hib == -1 ? 1 : 0) : -1;
-    if (!wn.w) {
-      tested += total;
-      continue;
-    }
-    found = i + 1;
-    // the candidates the winning iteration reports
-    if (ml) {
-      tested += cpu ? __shfl_sync(kFull, upto, wn.w_done) : total;
-    } else if (prob) {
-      // the phases before the winner's, and for the CPU branch the weights before it,
-      // for the GPU branch the whole phase (grand_decoder.cu:1006)
-#pragma unroll 1
-      for (int k = 0; k < cd.num_phases; ++k) {
-        const int pid = cd.mask_order[mi][k];
-        const bool hit = (pid == 0 && wn.w <= 5) || (pid == 1 && wn.w == 6);
-        if (hit && cpu) {
-          if (pid == 0) tested += __shfl_sync(kFull, upto, wn.w - 1);
-          break;
-        }
-        if (pid == 0) tested += c15;
-        if (pid == 1) tested += c6;
-        if (hit) break;
+    while (__any_sync(kFull, run != 0u)) {
+      const int w_first = run ? __ffs((int)run) - 1 : 1;
+      int w_last = run ? 31 - __clz((int)run) : 0;
+      if (run) {
+        wn.w = 0;
+        wn.cost = 0xffffffffu;
+        wn.w_done = w_last;
       }
-    } else {
-      tested += cpu ? __shfl_sync(kFull, upto, wn.w - 1) : total;  // grand_decoder.cu:1303-1304
-    }
-    if (!ml && cpu) {
-      // rank + 1 of the set among its weight's candidates (grand_decoder.cu:547-548)
-      const int pre = lanes_before(__popc(am));
-      const unsigned c = lane < wn.w ? set_col(wn.key, wn.w, lane) : 0u;
-      const int idx = __shfl_sync(kFull, pre, (int)(c >> 5)) + __popc(G.am[c >> 5] & ((1u << (c & 31u)) - 1u));
-      unsigned long long after = lane < wn.w ? ncr(b.ncr, tam - 1 - idx, wn.w - lane) : 0ull;
+      // columns of odd weight only: the weight of a match and the syndrome's are alike
+      // (ML goes on to the last weight for its bound)
+      const bool odd = cd.g_odd != 0;
+      if (odd && !ml && ((w_last ^ ones) & 1)) --w_last;
+      bool go = run != 0u && w_last >= w_first && ones <= max_cw * w_last;
+      // the roots: the empty sets of the groups that search
+      unsigned roots = __ballot_sync(kFull, go && gl == 0);
+      int lo = 0, hi = __popc(roots);
+      if (go && gl == 0)
+        item[__popc(roots & ((1u << lane) - 1u))] = make_uint2(hs, ((unsigned)g << 30) | row0);
+      __syncwarp();
+      float psum = 0.0f;                // ML: sum of the pw smallest LLRs of the active set,
+      unsigned long long plast = 0ull;  //   {LLR key, column} of the last of them, plus one
+      int pw = 0;
 #pragma unroll 1
-      for (int o = 4; o > 0; o >>= 1) after += __shfl_xor_sync(kFull, after, o);
-      tested += __shfl_sync(kFull, upto, wn.w) - __shfl_sync(kFull, upto, wn.w - 1) -
-                __shfl_sync(kFull, after, 0);
+      for (int w = 1; __any_sync(kFull, go && w <= w_last); ++w) {
+        bool act = go && w <= w_last;
+        if (MLK && __any_sync(kFull, act && ml && wn.w)) {
+          // upstream's prefix sums: the w smallest LLRs, added in ascending order
+#pragma unroll 1
+          for (;;) {
+            const bool want = act && ml && wn.w && pw < w;
+            if (!__any_sync(kFull, want)) break;
+            unsigned long long next = kNone;
+            if (want) {
+#pragma unroll 1
+              for (int q = gl; q < mw; q += G)
+#pragma unroll 1
+                for (uint32_t word = am[q]; word; word &= word - 1u) {
+                  const int c = 32 * q + __ffs((int)word) - 1;
+                  const uint32_t u = __float_as_uint(__ldg(llr + c));
+                  const uint32_t k = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+                  const unsigned long long x = ((unsigned long long)k << 32) | (unsigned)c;
+                  if (x >= plast && x < next) next = x;
+                }
+            }
+#pragma unroll 1
+            for (int o = 1; o < G; o <<= 1) {
+              const unsigned long long u = __shfl_xor_sync(kFull, next, o);
+              next = u < next ? u : next;
+            }
+            if (next != kNone) {
+              const uint32_t k = (uint32_t)(next >> 32);
+              psum = __fadd_rn(psum, __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k));
+              plast = next + 1ull;
+            }
+            if (want) ++pw;
+          }
+          if (act && ml && wn.w && psum >= key_cost(wn.cost)) {
+            wn.w_done = w - 1;
+            go = act = false;
+          }
+        }
+        const int d = w - 1;  // columns of the sets formed
+        // bit gb of a mask: the group's
+        const unsigned acts = __ballot_sync(kFull, act);
+        const unsigned probes = __ballot_sync(kFull, act && w >= w_first && !(odd && ((w ^ ones) & 1)));
+        const unsigned pushes = __ballot_sync(kFull, act && w < w_last);
+        if (gl == 0) S.limit = max_cw * (w_last - d);
+        __syncwarp();
+        unsigned long long bkey = kNone;  // the group's best of this weight
+        uint32_t bcost = 0xffffffffu;
+        const Path none{0xffffffffu, 0xffffffffu};
+        const int pairs = d == 0 ? 32 : (hi - lo) * deg;
+        int top = hi;
+        bool zeros = false;
+        int zi = -1;  // an item of residual zero being extended by every active column
+        uint32_t zbits = 0u;
+        // steps of 32 (item, neighbour) pairs (weight 1: one step of the roots); then, for
+        // each item without a row to follow, steps over its group's active columns, a
+        // lane those of its word
+#pragma unroll 1
+        for (int p0 = 0;; p0 += 32) {
+          int from = 0;
+          unsigned c = kNoCol;
+          uint2 it = make_uint2(0u, 0u);
+          bool root = false;
+          if (zi < 0 && p0 < pairs) {
+            const int p = p0 + lane;
+            if (d == 0) {
+              root = lane < hi;
+              if (root) it = item[lane];
+            } else if (p < pairs) {
+              const int n = (int)(((unsigned long long)(unsigned)p * magic) >> 32);
+              const int k = p - n * deg;
+              from = lo + n;
+              it = item[from];
+              const GuidedGroup &T = A.group[it.y >> 30];
+              const unsigned r = it.y & 1023u;
+              if (r == kNoRow) zeros = true;
+              else if (k < T.deg && ((acts >> (G * (it.y >> 30))) & 1u))
+                c = __ldg(T.adj + r * (unsigned)T.deg + (unsigned)k);
+            }
+          } else {
+            if (zi < 0 && !__any_sync(kFull, zeros)) break;  // (zeros: ML, or weights out of order)
+            if (!__any_sync(kFull, zbits != 0u)) {
+              zi = zi < 0 ? lo : zi + 1;
+              while (zi < hi && !((item[zi].y & 1023u) == kNoRow && ((acts >> (G * (item[zi].y >> 30))) & 1u)))
+                ++zi;
+              if (zi >= hi) break;
+              zbits = A.group[item[zi].y >> 30].am[i][lane];
+              const int tail = A.group[item[zi].y >> 30].m - 32 * lane;  // (words past the last are not set)
+              if (tail <= 0) zbits = 0u;
+            }
+            from = zi;
+            it = item[zi];
+            if (zbits) {
+              c = (unsigned)(32 * lane + __ffs((int)zbits) - 1);
+              zbits &= zbits - 1u;
+            }
+          }
+          // one child per lane: column c after the item, if active and not in it
+          const int gid = (int)(it.y >> 30);
+          const GuidedGroup &T = A.group[gid];
+          const uint32_t *tam = T.am[i];
+          GuidedBest best;
+          best.key = kNone;
+          best.cost = 0xffffffffu;
+          Path path = none;
+          bool child = root || (c != kNoCol && ((tam[(c >> 5) & 31u] >> (c & 31u)) & 1u));
+          if (child) {
+            if (!root) {
+              it.x ^= __ldg(T.hcol + c);
+              uint32_t up = it.y;
+#pragma unroll 1
+              for (int e = d - 1; e > 0; --e) {
+                push_col(path, (up >> 10) & 1023u);
+                up = item[(up >> 20) & 1023u].y;
+              }
+              child = !in_path(path, c);
+            }
+            if (child && ((probes >> (G * gid)) & 1u))
+              guided_probe<MLK>(T, tam, path, root ? 0 : d - 1, c, it.x, best);
+          }
+          unsigned hit = __ballot_sync(kFull, best.key != kNone);
+#pragma unroll 1
+          for (; hit; hit &= hit - 1u) {  // rare: each match to its group's lanes
+            const int src = __ffs((int)hit) - 1;
+            const unsigned long long k2 = __shfl_sync(kFull, best.key, src);
+            const uint32_t o2 = __shfl_sync(kFull, best.cost, src);
+            if (__shfl_sync(kFull, gid, src) == g) {
+              const bool less = !ml ? k2 < bkey
+                                    : o2 < bcost || bkey == kNone ||
+                                          (o2 == bcost && ml_set_before(llr, k2, bkey, w));
+              if (less) {
+                bkey = k2;
+                bcost = o2;
+              }
+            }
+          }
+          if (d == 0) continue;
+          const bool push = child && ((pushes >> (G * gid)) & 1u);
+          if (__any_sync(kFull, push)) {
+            bool keep = push;
+            if (keep) {
+              const Resid r = residual(T.sw, T.cols, T.wide != 0, path, d - 1, c);
+              it.y = ((unsigned)gid << 30) | ((unsigned)from << 20) | (c << 10) | lowest_row(r);
+              keep = ones_of(r) <= T.limit;
+            }
+            const unsigned kept = __ballot_sync(kFull, keep);
+            const int at = top + __popc(kept & ((1u << lane) - 1u));
+            top += __popc(kept);
+            if (top > kGuidedItems) return 0;
+            if (keep) item[at] = it;
+          }
+        }
+        __syncwarp();
+        if (d) {
+          lo = hi;
+          hi = top;
+        }
+        if (act && bkey != kNone && (!ml || !wn.w || bcost < wn.cost)) {
+          wn.w = w;
+          wn.key = bkey;
+          wn.cost = bcost;
+          if (!ml) go = false;
+        }
+        if (lo == hi && d && !wn.w) go = false;  // nothing left to extend
+      }
+      run = wn.w ? 0u : rest;
+      rest = 0u;
     }
+
+    // ---- the candidates the iteration reports ------------------------------------------
+    const unsigned long long c15 = __shfl_sync(kFull, upto, gb + 5);
+    const unsigned long long c6 = __shfl_sync(kFull, upto, gb + 6) - c15;
+    const unsigned long long before = __shfl_sync(kFull, upto, gb + (wn.w ? wn.w - 1 : 0));
+    unsigned long long total = __shfl_sync(kFull, upto, gb + wmax);
+    unsigned long long upto_hit = __shfl_sync(kFull, upto, gb + (ml ? wn.w_done & 7 : wn.w));
+    if (prob) {
+      total = 0;
+      bool past = false;  // the winner's phase is behind
+#pragma unroll 1
+      for (int k = 0; on && k < cd.num_phases; ++k) {
+        const int pid = order[k];
+        const unsigned long long n = pid == 0 ? c15 : (pid == 1 && tam >= 6 ? c6 : 0ull);
+        total += n;
+        const bool mine = wn.w && ((pid == 0 && wn.w <= 5) || (pid == 1 && wn.w == 6));
+        // the phases before the winner's, and for the CPU branch the weights before it, for
+        // the GPU branch the whole phase (grand_decoder.cu:1006)
+        if (wn.w && !past) tested += mine && cpu ? (pid == 0 ? before : 0ull) : n;
+        past = past || mine;
+      }
+    }
+    if (on) {
+      heavy |= total > (1ull << b.light_max_log2) || tam > kLightTam || tam * cd.nwp > kLightWords;
+      hib = gpu ? (hib == -1 ? 1 : 0) : -1;
+      if (!wn.w) tested += total;
+      else if (ml) tested += cpu ? upto_hit : total;
+      else if (!prob) tested += cpu ? before : total;  // grand_decoder.cu:1303-1304
+    }
+    const bool ranked = on && wn.w && !ml && cpu;
+    if (__any_sync(kFull, ranked)) {
+      // rank + 1 of the set among its weight's candidates (grand_decoder.cu:547-548)
+      unsigned long long after = 0ull;
+      if (ranked && gl < wn.w) {
+        const unsigned c = set_col(wn.key, wn.w, gl);
+        int idx = __popc(am[c >> 5] & ((1u << (c & 31u)) - 1u));
+#pragma unroll 1
+        for (int q = 0; q < (int)(c >> 5); ++q) idx += __popc(am[q]);
+        const unsigned long long *u = b.upto + 8 * (tam - 1 - idx) + (wn.w - gl);
+        after = __ldg(u) - __ldg(u - 1);
+      }
+#pragma unroll 1
+      for (int o = 1; o < 8; o <<= 1) after += __shfl_xor_sync(kFull, after, o);
+      after = __shfl_sync(kFull, after, gb);
+      if (ranked) tested += upto_hit - before - after;
+    }
+    if (on && wn.w) found = i + 1;
   }
   tp = prof_lap(b, kProfShotLight, tp);
 
   // ---- the result --------------------------------------------------------------------
-  uint32_t e = 0u;   // word `lane` of the decoded error
-  uint32_t le = 0u;  // and of its logical flips (DEM)
   const bool dem = cd.family == kDem;
+  const int shot = F.shot[j];
+  const bool errs = cd.input_kind == kInErrors;
+  bool differs = false;
+  if (live && found) {
+    if (dem) {  // decoded logical flips vs the supplied true flips (grand_decoder.cu:1623-1644)
+      if (gl < cd.nlw) {
+        uint32_t le = 0u;
 #pragma unroll 1
-  for (int k = 0; k < wn.w; ++k) {
-    const unsigned c = set_col(wn.key, wn.w, k);
-    if ((int)(c >> 5) == lane) e |= 1u << (c & 31u);
-    if (dem && lane < cd.nlw) le ^= __ldg(cd.lcols + c * (unsigned)cd.nlw + (unsigned)lane);
+        for (int k = 0; k < wn.w; ++k)
+          le ^= __ldg(cd.lcols + set_col(wn.key, wn.w, k) * (unsigned)cd.nlw + (unsigned)gl);
+        differs = le != row[kRowLog + gl];
+      }
+    } else if (errs) {  // grand_decoder.cu:1362: as many columns, and each of them supplied
+      const int at = F.at[j];
+      differs = at < 0 || (int)row[kRowWeight] != wn.w;
+      if (!differs && gl < wn.w) {
+        const int c = at + (int)set_col(wn.key, wn.w, gl);
+        differs = !((F.bits[c >> 5] >> (c & 31)) & 1u);
+      }
+    }
   }
-  int degenerate = 0, is_equal = 0;
-  if (found && dem) {
-    // decoded logical flips vs the supplied true flips (grand_decoder.cu:1623-1644)
-    degenerate = __all_sync(kFull, le == eb_lane) ? 1 : 0;
-  } else if (found && cd.input_kind == kInErrors) {
-    is_equal = __all_sync(kFull, e == eb_lane) ? 1 : 0;  // grand_decoder.cu:1362
-    degenerate = is_equal || in_row_space(cd, e ^ eb_lane) ? 1 : 0;
+  const bool told = ((__ballot_sync(kFull, differs) >> gb) & kGroup) != 0u;
+  bool is_equal = live && found && !dem && errs && !told;
+  bool degenerate = is_equal || (live && found && dem && !told);
+  {
+    // a supplied error that differs (or whose bits are not at hand): a group at a time, by
+    // the whole warp
+    unsigned todo = __ballot_sync(kFull, gl == 0 && told && !dem);
+#pragma unroll 1
+    for (; todo; todo &= todo - 1u) {
+      const int src = __ffs((int)todo) - 1;
+      const int e2 = __shfl_sync(kFull, entry, src);
+      const int w2 = __shfl_sync(kFull, wn.w, src);
+      const unsigned long long k2 = __shfl_sync(kFull, wn.key, src);
+      const FastArea &F2 =
+          *reinterpret_cast<const FastArea *>(reinterpret_cast<char *>(areas) + (e2 >> 8) * area_step);
+      const int j2 = e2 & 255;
+      const DevCode &cd2 = b.codes[F2.code[j2]];
+      const uint32_t delta = set_word(k2, w2) ^ error_word(b, cd2, F2, F2.at[j2], F2.shot[j2]);
+      const bool eq = __all_sync(kFull, delta == 0u);
+      const bool deg2 = eq || in_row_space(cd2, delta);
+      if (gb == src) {
+        is_equal = eq;
+        degenerate = deg2;
+      }
+    }
   }
-  if (dem && b.dec_log) bits_to_bytes(b.dec_log + (size_t)shot * cd.n_logicos, cd.n_logicos, le);
-  if (b.dec_err) bits_to_bytes(b.dec_err + (size_t)shot * cd.m, cd.m, e);
-  // the 72-byte result as 18 words, one per lane (finish_shot's layout and times)
-  const unsigned long long now = global_ns();
-  const unsigned long long dt = lane < 12 ? t_counts - t_start : lane < 14 ? now - t_counts
-                                : lane < 16 || !found ? 0ull : now - t_start;
-  const unsigned long long bits = (unsigned long long)__double_as_longlong(1e-6 * (double)dt);
-  uint32_t x = (lane & 1) ? (uint32_t)(bits >> 32) : (uint32_t)bits;
-  x = lane == 9 ? (uint32_t)(found ? found : passes) : x;
-  x = lane == 8 ? (uint32_t)hib : x;
-  x = lane == 7 ? (uint32_t)(tested >> 32) : x;
-  x = lane == 6 ? (uint32_t)tested : x;
-  x = lane == 5 ? (uint32_t)tam : x;
-  x = lane == 4 ? (uint32_t)is_equal : x;
-  x = lane == 3 ? (uint32_t)degenerate : x;
-  x = lane == 2 ? (uint32_t)original_weight : x;
-  x = lane == 1 ? (uint32_t)wn.w : x;
-  x = lane == 0 ? (found ? 1u : 0u) : x;
-  if (lane < 18) reinterpret_cast<uint32_t *>(b.results + shot)[lane] = x;
-  if (lane == 0) {
+  const int ow = (int)row[kRowWeight];
+  __syncwarp();  // every lane has read the open shot's words
+  if (live && gl == 0) {
+    const unsigned long long now = global_ns();
+    const unsigned long long a = (unsigned long long)__double_as_longlong(1e-6 * (double)(t_counts - t_start));
+    const unsigned long long s = (unsigned long long)__double_as_longlong(1e-6 * (double)(now - t_counts));
+    const unsigned long long t =
+        found ? (unsigned long long)__double_as_longlong(1e-6 * (double)(now - t_start)) : 0ull;
+    row[0] = found ? 1u : 0u;
+    row[1] = (uint32_t)wn.w;
+    row[2] = (uint32_t)ow;
+    row[3] = degenerate ? 1u : 0u;
+    row[4] = is_equal ? 1u : 0u;
+    row[5] = (uint32_t)tam;
+    row[6] = (uint32_t)tested;
+    row[7] = (uint32_t)(tested >> 32);
+    row[8] = (uint32_t)hib;
+    row[9] = (uint32_t)(found ? found : passes);
+    row[10] = (uint32_t)a;
+    row[11] = (uint32_t)(a >> 32);
+    row[12] = (uint32_t)s;
+    row[13] = (uint32_t)(s >> 32);
+    row[14] = row[15] = 0u;
+    row[16] = (uint32_t)t;
+    row[17] = (uint32_t)(t >> 32);
+    F.key[j] = wn.key;
+    F.state[j] = 1;
     if (b.ml_cost) b.ml_cost[shot] = found && ml ? key_cost(wn.cost) : 0.0f;
-    if (b.deferred) b.deferred[shot] = 0;
   }
   __syncwarp();
   prof_lap(b, kProfShotFinish, tp);
-  return heavy ? 2 : 1;
+  int ret = 0;
+#pragma unroll 1
+  for (int k = 0; k < 32 / G; ++k) {
+    if (k < cnt) ret |= 1 << k;
+    ret |= __shfl_sync(kFull, live && heavy ? 1 : 0, k * G) << (8 + k);
+  }
+  return ret;
 }
 
 }  // namespace grand

@@ -32,7 +32,7 @@
 namespace grand {
 
 struct GuidedTables {
-  int gs = 0, deg = 0, max_cw = 0;
+  int gs = 0, deg = 0, max_cw = 0, odd = 1;
   uint32_t tab_mask = 0;
   // one block of words; the parts start at these word offsets (16-byte aligned)
   size_t total = 0, o_rows = 0, o_cw = 0, o_adj = 0, o_cols = 0, o_filt = 0, o_tab = 0, o_hcol = 0;
@@ -55,7 +55,10 @@ inline GuidedTables build_guided_tables(const std::vector<uint32_t> &cols, int n
         adj[32 * k + __builtin_ctz(w)].push_back(c);
         ++cw[c];
       }
-  for (int c = 0; c < m; ++c) g.max_cw = std::max(g.max_cw, cw[c]);
+  for (int c = 0; c < m; ++c) {
+    g.max_cw = std::max(g.max_cw, cw[c]);
+    if (cw[c] && !(cw[c] & 1)) g.odd = 0;
+  }
   for (int r = 0; r < R; ++r) g.deg = std::max(g.deg, (int)adj[r].size());
   if (g.max_cw < 1 || g.max_cw > kGuidedMaxColWeight || g.deg > kGuidedMaxDegree) return g;
   g.gs = nw <= 4 ? 4 : 8;
@@ -115,6 +118,7 @@ inline void set_guided(DevCode &d, const GuidedTables &g, const uint32_t *base) 
   if (!d.g_gs) return;
   d.g_deg = g.deg;
   d.g_max_cw = g.max_cw;
+  d.g_odd = g.odd;
   d.g_magic = 0xffffffffull / (unsigned)g.deg + 1ull;
   d.g_tab_mask = g.tab_mask;
   d.g_rows = base + g.o_rows;

@@ -105,6 +105,15 @@ static unsigned long long ncr_host(int n, int k) {
   return r;
 }
 
+template <class T>
+static cudaError_t upload(T **d, const std::vector<T> &h) {
+  size_t bytes = std::max<size_t>(h.size() * sizeof(T), 16);
+  cudaError_t e = cudaMalloc(d, bytes);
+  if (e != cudaSuccess) return e;
+  if (h.empty()) return cudaMemset(*d, 0, bytes);
+  return cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+}
+
 Context *Context::get(int *err) {
   static std::mutex mu;
   static Context *ctxs[64] = {};
@@ -148,6 +157,18 @@ Context *Context::get(int *err) {
       cudaMemcpy(c->d_ncr, t.data(), t.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess) {
     set_error("grand: could not upload the binomial table");
     *err = GRAND_ERR_CUDA;
+    delete c;
+    return nullptr;
+  }
+  std::vector<unsigned long long> upto(8 * (kGuidedMaxCols + 1), 0ull);
+  for (int n = 0; n <= kGuidedMaxCols; ++n)
+    for (int k = 1; k < 8; ++k)
+      upto[8 * (size_t)n + k] = upto[8 * (size_t)n + k - 1] + (k <= kMaxW ? ncr_host(n, k) : 0ull);
+  if (upload(&c->d_upto, upto) != cudaSuccess) {
+    set_error("grand: could not upload the candidate counts");
+    *err = GRAND_ERR_CUDA;
+    cudaFree(c->d_ncr);
+    cudaFree(c->d_upto);
     delete c;
     return nullptr;
   }
@@ -209,15 +230,6 @@ static int rref_bits(std::vector<uint32_t> &rows, int n, int mw, int m, std::vec
     ++r;
   }
   return r;
-}
-
-template <class T>
-static cudaError_t upload(T **d, const std::vector<T> &h) {
-  size_t bytes = std::max<size_t>(h.size() * sizeof(T), 16);
-  cudaError_t e = cudaMalloc(d, bytes);
-  if (e != cudaSuccess) return e;
-  if (h.empty()) return cudaMemset(*d, 0, bytes);
-  return cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
 }
 
 std::shared_ptr<CodeTables> Context::tables(int family, const int *H, const int *H_other,
@@ -397,14 +409,13 @@ void plan_batch(DevBatch &b, const DevCode *codes, int ncodes, int sm_count, con
   b.guided = !tn.fast || !any ? kGuidedNone : (all ? kGuidedAll : kGuidedFirst);
   b.chunk = kMaxChunk;
   if (b.guided) {
-    // as many chunks as there are resident warps, up to the chunk's limits: fewer leave
-    // warps idle, more only add the chunks' own cost (their records' round trips), and
-    // past one wave the blocks balance the load.  16384 headline shots: 50.4 us in
-    // chunks of 4, 48.4 of 5 (chosen), 52.7 of 8, 70.2 of 16; the 100000-shot mix: 199,
-    // -, 149 and 124 us (16, chosen)
-    const int warps = sm_count * chunk_warps_per_sm();
-    int c = (b.num_shots + warps - 1) / warps;
-    c = std::min<long long>(std::min(c, (int)kMaxChunk), 32 * kFastBallots / entries);
+    // full waves of the resident warps, in chunks as large as they may be: a chunk costs
+    // its records' round trips whatever its size, a part wave costs a whole one (twice
+    // the chunks in half the size: headline 30.8 -> 40.3 us, noisy [[288]] 52 -> 62)
+    const int warps = sm_count * kChunkMinBlocks * kChunkWarps;
+    const int most = (int)std::min<long long>(kMaxChunk, 32 * kFastBallots / entries);
+    const int waves = (b.num_shots - 1) / (warps * std::max(most, 1)) + 1;
+    const int c = std::min((b.num_shots - 1) / (warps * waves) + 1, most);
     b.chunk = std::max(c, 1);
   }
   if (b.guided == kGuidedAll) b.deferred = nullptr;  // nothing is ever deferred
@@ -517,6 +528,7 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
     b.ml_cost = req.h_cost ? (float *)ws->d_cost : nullptr;
   }
   b.ncr = ctx->d_ncr;
+  b.upto = ctx->d_upto;
   b.jobs = (Job *)ws->d_jobs;
   b.max_jobs = max_jobs;
   b.counters = (unsigned long long *)ws->d_small;

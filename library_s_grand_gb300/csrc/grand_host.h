@@ -16,7 +16,6 @@ namespace grand {
 // Kernel launchers (grand_decode_plain.cu, grand_decode_ml.cu, grand_sample.cu).
 cudaError_t launch_decode(const DevBatch &b, int grid, cudaStream_t s);
 cudaError_t decode_occupancy(int *blocks_per_sm);
-int chunk_warps_per_sm();  // resident warps of the chunk kernel the launch plan counts on
 cudaError_t launch_sample(const DevCode &cd, const float *d_p, unsigned long long seed,
                           unsigned long long first_shot, int num_shots, int *d_records,
                           int sm_count, cudaStream_t s);
@@ -118,6 +117,7 @@ class Context {
   int sm_count = 0;
   int decode_bps = 1;  // resident decode-kernel blocks per SM
   unsigned long long *d_ncr = nullptr;
+  unsigned long long *d_upto = nullptr;  // DevBatch::upto
   int pageable_access = 0;
 
   std::shared_ptr<CodeTables> tables(int family, const int *H, const int *H_other,

@@ -72,16 +72,6 @@ __device__ __forceinline__ unsigned long long ld_ctr(const DevBatch &b, int ctr)
   return *reinterpret_cast<volatile unsigned long long *>(ctr_ptr(b.counters, ctr));
 }
 
-// A code's descriptor into the warp's shared copy, one round trip for the whole of it.
-__device__ __forceinline__ void load_code(DevCode &dst, const DevCode *src) {
-  static_assert(sizeof(DevCode) % 8 == 0, "whole words");
-  __syncwarp();  // every lane is done with the code before
-  for (int i = threadIdx.x & 31; i < (int)(sizeof(DevCode) / 8); i += 32)
-    reinterpret_cast<unsigned long long *>(&dst)[i] =
-        __ldg(reinterpret_cast<const unsigned long long *>(src) + i);
-  __syncwarp();
-}
-
 // Profile (DevBatch::profile): lane 0 adds the time since t0 to profile sums
 // word w; returns the current time (0 when not profiling).
 __device__ __forceinline__ unsigned long long prof_lap(const DevBatch &b, int w,

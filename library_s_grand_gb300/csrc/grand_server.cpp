@@ -170,6 +170,7 @@ cudaError_t start_slot(GrandServer *S, SrvSlot *sl) {
   b.shot_code = sl->d_code;
   b.results = sl->d_res;
   b.ncr = e->ctx->d_ncr;
+  b.upto = e->ctx->d_upto;
   b.jobs = sl->d_jobs;
   b.max_jobs = S->max_shots;
   b.counters = sl->d_small;

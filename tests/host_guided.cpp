@@ -9,6 +9,21 @@
 #define main host_kernels_main
 #include "host_kernels.cpp"
 #undef main
+
+// the block's threads meet; shared-memory atomics
+static std::atomic<int> g_block_count{0}, g_block_gen{0};
+static void __syncthreads() {
+  const int gen = g_block_gen.load();
+  if (g_block_count.fetch_add(1) + 1 == (int)blockDim.x) {
+    g_block_count.store(0);
+    g_block_gen.fetch_add(1);
+    return;
+  }
+  while (g_block_gen.load() == gen) std::this_thread::yield();
+}
+static inline int atomicAdd(int *a, int v) { return __atomic_fetch_add(a, v, __ATOMIC_SEQ_CST); }
+
+#include "grand_front.cuh"
 #include "grand_guided_tables.h"
 
 // The kernels of a batch as the library launches them (launch_kernels).
@@ -25,6 +40,11 @@ static void run_guided_batch(DevBatch &b, int N) {
   std::vector<uint32_t> rec_cache((size_t)N * kRecCacheWords, 0xa5a5a5a5u);
   b.num_shots = N;
   b.ncr = ncr.data();
+  std::vector<unsigned long long> upto(8 * (kGuidedMaxCols + 1), 0ull);
+  for (int n = 0; n <= kGuidedMaxCols; ++n)
+    for (int k = 1; k < 8; ++k)
+      upto[8 * (size_t)n + k] = upto[8 * (size_t)n + k - 1] + (k <= kMaxW ? C(n, k) : 0ull);
+  b.upto = upto.data();
   b.jobs = jobs.data();
   b.max_jobs = N;
   b.counters = small;

@@ -143,18 +143,20 @@ def test_capped_dem_stress(guided, port, tmp_path):
 
 
 def test_levels_that_do_not_fit(guided, port, tmp_path):
-    """Columns of weight 7 on 24 rows: each row meets dozens of them, so the levels of a
-    weight-4 search outgrow the warp's area and the shots take the general path."""
+    """Columns of weight 5 on 24 rows: each row meets dozens of them, so the levels of a
+    weight-4 search outgrow the warp's items (of several shots together, and of one alone)
+    and the shots take the general path."""
     rng = np.random.default_rng(3)
-    h = np.zeros((24, 128), np.int32)
-    for c in range(128):
-        h[rng.choice(24, 7, replace=False), c] = 1
-    e = np.zeros((40, 128), np.int32)
+    h = np.zeros((24, 230), np.int32)
+    for c in range(230):
+        h[rng.choice(24, 5, replace=False), c] = 1
+    assert 40 < h.sum(axis=1).max() <= 64
+    e = np.zeros((40, 230), np.int32)
     for i in range(40):
-        e[i, rng.choice(128, 1 + i % 5, replace=False)] = 1
-    cfg = (4, 256, 0, 128, 10, -1)
+        e[i, rng.choice(230, 1 + i % 5, replace=False)] = 1
+    cfg = (4, 256, 0, 230, 10, -1)
     res, dec, out = _run(guided, str(tmp_path), h, h, e, True, 0, cfg, [], 10)
     prc, pres, pdec = port.css(O.UNIFORM, h, h, e, None, O.Config(*cfg), "x")
     assert prc == 0
     _compare(res, dec, pres, pdec)
-    assert _jobs(out) > 0, out
+    assert out.split("\n")[1].startswith("guided 1 ") and _jobs(out) > 0, out
