@@ -45,74 +45,75 @@ __device__ __forceinline__ uint32_t flip_threshold(float p) {
   return s >= 4294967295.0f ? 0xFFFFFFFFu : (s <= 0.0f ? 0u : (uint32_t)s);
 }
 
-// One warp per shot.  The flips are packed into the warp's shared-memory word
-// array, then the record entries are written with coalesced int32 stores.
-__global__ void __launch_bounds__(256) sample_kernel(DevCode cd, const float *p,
+// One warp per shot, a block's warps in strides of the grid.  The positions' thresholds are
+// formed once per block, in shared memory, a lane's four of a group side by side.  Flips
+// are rare: a group is asked once whether it has any, and their columns then go straight
+// into the lanes' syndrome (and logical) words, from which the entries are stored
+// coalesced; an error record's entries are the lanes' own comparisons.
+//
+// Bound by instruction issue, the generator's above all: 20 products of 32 x 32 -> 64 bits
+// and as many logic operations per four positions.  65536 shots of the 720-mechanism DEM:
+// 60 us (128 when every word was scanned for flips and the thresholds formed per shot;
+// 650 warp instructions a shot, 1700 then).
+template <bool ERRORS>
+__global__ void __launch_bounds__(256, 8) sample_kernel(DevCode cd, const float *p,
                                                      unsigned long long seed,
                                                      unsigned long long first_shot, int num_shots,
                                                      int *records) {
-  __shared__ uint32_t s_flip[8][kMaxCols / 32];
-  __shared__ uint32_t s_syn[8][kMaxRows / 32];
-  __shared__ uint32_t s_log[8][kMaxLogicals / 32];
+  extern __shared__ uint4 s_thr[];  // per group of 128 positions and lane: those of 32u + lane
   const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  uint32_t *flip = s_flip[wib];
-  uint32_t *syn = s_syn[wib];
-  uint32_t *lg = s_log[wib];
+  const int mpad = (cd.m + 127) & ~127;
+  for (int j = threadIdx.x; j < mpad; j += blockDim.x)  // (zeros past the last position)
+    reinterpret_cast<uint32_t *>(s_thr)[(j & ~127) + 4 * (j & 31) + ((j >> 5) & 3)] =
+        j < cd.m ? flip_threshold(__ldg(p + j)) : 0u;
+  __syncthreads();
   const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
   const int nwarps = gridDim.x * 8;
-  for (int i = blockIdx.x * 8 + wib; i < num_shots; i += nwarps) {
+  const bool dem = cd.family == kDem;
+  const int nw = cd.nw, nlw = dem ? cd.nlw : 0;
+#pragma unroll 1
+  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < num_shots; i += nwarps) {
     const unsigned long long shot = first_shot + (unsigned long long)i;
+    int *rec = records + (size_t)i * cd.rec_len;
+    uint32_t s_lane = 0u, l_lane = 0u;  // syndrome / detector word `lane`, logical word `lane`
     // flips: 128 positions per group, four words of one block per lane
-    for (int g = 0; g * 128 < cd.m; ++g) {
-      uint32_t c[4] = {(uint32_t)(g * 32 + lane), (uint32_t)shot, (uint32_t)(shot >> 32),
+#pragma unroll 1
+    for (int j0 = 0; j0 < mpad; j0 += 128) {
+      uint32_t c[4] = {(uint32_t)(j0 / 4 + lane), (uint32_t)shot, (uint32_t)(shot >> 32),
                        0x47524E44u};
       philox4x32_10(c, k0, k1);
+      const uint4 thr = s_thr[j0 / 4 + lane];
+      const bool f[4] = {c[0] < thr.x, c[1] < thr.y, c[2] < thr.z, c[3] < thr.w};
+      if constexpr (ERRORS) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = g * 128 + u * 32 + lane;
-        const bool f = j < cd.m && c[u] < flip_threshold(__ldg(p + j));
-        const uint32_t bits = __ballot_sync(kFull, f);
-        if (lane == 0 && g * 4 + u < cd.mw) flip[g * 4 + u] = bits;
-      }
-    }
-    __syncwarp();
-    // syndrome / detectors: XOR of the flipped columns (lane w: word w)
-    uint32_t s_lane = 0u;
-    for (int q = 0; q < cd.mw; ++q) {
-      uint32_t word = flip[q];
-      while (word) {
-        const int col = q * 32 + __ffs(word) - 1;
-        word &= word - 1u;
-        if (lane < cd.nw) s_lane ^= __ldg(cd.cols + (size_t)col * cd.nwp + lane);
-      }
-    }
-    if (lane < cd.nw) syn[lane] = s_lane;
-    // DEM: true logical flips, XOR of the flipped mechanisms' rows of L
-    if (cd.family == kDem) {
-      for (int q = lane; q < cd.nlw; q += 32) {
-        uint32_t acc = 0u;
-        for (int qq = 0; qq < cd.mw; ++qq) {
-          uint32_t word = flip[qq];
-          while (word) {
-            const int col = qq * 32 + __ffs(word) - 1;
-            word &= word - 1u;
-            acc ^= __ldg(cd.lcols + (size_t)col * cd.nlw + q);
+        for (int u = 0; u < 4; ++u)
+          if (j0 + 32 * u + lane < cd.m) rec[j0 + 32 * u + lane] = f[u] ? 1 : 0;
+      } else if (__any_sync(kFull, f[0] || f[1] || f[2] || f[3])) {
+#pragma unroll 1
+        for (int u = 0; u < 4; ++u) {
+          const bool mine = u == 0 ? f[0] : (u == 1 ? f[1] : (u == 2 ? f[2] : f[3]));
+#pragma unroll 1
+          for (uint32_t bits = __ballot_sync(kFull, mine); bits; bits &= bits - 1u) {
+            // XOR of the flipped columns, and of their rows of L
+            const int col = j0 + 32 * u + __ffs((int)bits) - 1;
+            if (lane < nw) s_lane ^= __ldg(cd.cols + (size_t)col * cd.nwp + lane);
+            if (lane < nlw) l_lane ^= __ldg(cd.lcols + (size_t)col * cd.nlw + lane);
           }
         }
-        lg[q] = acc;
       }
     }
-    __syncwarp();
-    int *rec = records + (size_t)i * cd.rec_len;
-    if (cd.input_kind == kInErrors) {
-      for (int j = lane; j < cd.m; j += 32) rec[j] = (flip[j >> 5] >> (j & 31)) & 1u;
-    } else {
-      for (int r = lane; r < cd.R; r += 32) rec[r] = (syn[r >> 5] >> (r & 31)) & 1u;
-      if (cd.family == kDem)
-        for (int j = lane; j < cd.n_logicos; j += 32) rec[cd.R + j] = (lg[j >> 5] >> (j & 31)) & 1u;
+    if constexpr (!ERRORS) {
+#pragma unroll 1
+      for (int r = lane; r - lane < cd.R; r += 32) {
+        const uint32_t word = __shfl_sync(kFull, s_lane, r >> 5);
+        if (r < cd.R) rec[r] = (int)((word >> lane) & 1u);
+      }
+#pragma unroll 1
+      for (int j = lane; dem && j - lane < cd.n_logicos; j += 32) {
+        const uint32_t word = __shfl_sync(kFull, l_lane, j >> 5);
+        if (j < cd.n_logicos) rec[cd.R + j] = (int)((word >> lane) & 1u);
+      }
     }
-    __syncwarp();
   }
 }
 
@@ -122,7 +123,11 @@ cudaError_t launch_sample(const DevCode &cd, const float *d_p, unsigned long lon
   if (num_shots <= 0) return cudaSuccess;
   int grid = (num_shots + 7) / 8;
   if (grid > sm_count * 8) grid = sm_count * 8;
-  sample_kernel<<<grid, 256, 0, s>>>(cd, d_p, seed, first_shot, num_shots, d_records);
+  const size_t smem = sizeof(uint32_t) * ((cd.m + 127) & ~127);  // at most 16 KB
+  if (cd.input_kind == kInErrors)
+    sample_kernel<true><<<grid, 256, smem, s>>>(cd, d_p, seed, first_shot, num_shots, d_records);
+  else
+    sample_kernel<false><<<grid, 256, smem, s>>>(cd, d_p, seed, first_shot, num_shots, d_records);
   return cudaGetLastError();
 }
 
