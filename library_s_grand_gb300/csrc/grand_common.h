@@ -118,11 +118,13 @@ enum Counter {
   kCtrSlowDone = 7,       // per-shot-path shots finished (their Jobs published)
   kCtrWarpsDone = 8,      // warps that left the kernel (the last advances the epoch)
   kCtrSettled = 10,       // statistics: shots settled without a search (word 0), by the
-                          // guided search (1), and those of the latter past the light budget (2)
+                          // guided search (1), and those of the latter past the light budget (2);
+                          // words 4 .. 6: the chunk kernel's running sums of the three
   kCtrProfSums = 11,      // profile (DevBatch::profile): warp-ns per kind of work, steps
   kCtrProfEnds = 13,      // profile: latest end per kind of work, ~(first warp start)
   kCtrProfMore = 14,      // profile: the Job publication's steps (kProfPub*)
 };
+constexpr int kStatAcc = 4, kStatShift = 39;  // running sums: blocks counted from bit 39 up
 // Words of the two profile lines: kinds of work in the order of the decode
 // kernel's steps (classification chunks, per-shot path, search tiles, waiting),
 // then the number of steps (sums line) and the complemented start (ends line).

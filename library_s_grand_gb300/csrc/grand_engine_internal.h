@@ -67,6 +67,9 @@ namespace grand {
 // Upload the engine's code descriptors when they changed (caller holds e->mu).
 inline int upload_codes(GrandEngine *e) {
   if (!e->dirty) return 0;
+  // launches captured for the codes before hold their descriptors' address and plan
+  for (auto &g : e->graphs) cudaGraphExecDestroy(g.second);
+  e->graphs.clear();
   cudaError_t r = ensure(&e->d_codes, &e->cap_codes,
                          sizeof(DevCode) * (e->codes.empty() ? 1 : e->codes.size()));
   if (r == cudaSuccess && !e->codes.empty())

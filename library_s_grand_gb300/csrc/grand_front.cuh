@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
   __shared__ ChunkArea areas[kChunkWarps];
   __shared__ HotCode hot[kHotCodes];
   __shared__ uint16_t open[kChunkWarps * kMaxChunk];
-  __shared__ int open_count, open_next;
+  __shared__ int open_count, open_next, stats[3];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int chunk = (int)blockIdx.x * kChunkWarps + wib;
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
           __ldg(reinterpret_cast<const unsigned long long *>(static_cast<const HotCode *>(b.codes + k)) + i -
                 k * kWords);
     }
-    if (threadIdx.x == 0) open_count = open_next = 0;
+    if (threadIdx.x == 0) open_count = open_next = stats[0] = stats[1] = stats[2] = 0;
     __syncthreads();
 #pragma unroll 1
     for (int k = 0; k < n; ++k) {
@@ -110,19 +110,33 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
       }
     }
   }
+  if (lane < 3 && (lane == 0 ? st.settled : lane == 1 ? st.guided : st.heavy))
+    atomicAdd(&stats[lane], lane == 0 ? st.settled : lane == 1 ? st.guided : st.heavy);
   __syncthreads();
 
   if (has) write_chunk(b, hot, chunk, b.chunk, F, tag);
-  if (lane == 0) {
-    add_stats(b, st);
-    if (b.profile) {
-      const unsigned long long t = global_ns();
-      unsigned long long *ends = ctr_ptr(b.counters, kCtrProfEnds);
-      atomicMax(ends + kProfStart, ~t_enter);
-      atomicMax(ends + kProfChunk, t);
-      atomicAdd(ctr_ptr(b.counters, kCtrProfSums) + kProfChunk, t - t_enter);
-      atomicAdd(ctr_ptr(b.counters, kCtrProfSums) + kProfSteps, 1ull);
+  // The statistics: the blocks add theirs to words that count the blocks in their upper bits,
+  // and a word's last block publishes it and clears it for the next launch, so a launch of
+  // this kernel alone needs nothing cleared before it.
+  if (threadIdx.x < 3) {
+    unsigned long long *word = ctr_ptr(b.counters, kCtrSettled) + lane;
+    unsigned long long *acc = word + kStatAcc;
+    const unsigned long long mine_too = (unsigned long long)stats[lane];
+    const unsigned long long old = atomicAdd(acc, (1ull << kStatShift) + mine_too);
+    if ((old >> kStatShift) + 1ull == (unsigned long long)gridDim.x) {
+      const unsigned long long total = (old & ((1ull << kStatShift) - 1ull)) + mine_too;
+      *reinterpret_cast<volatile unsigned long long *>(acc) = 0ull;
+      if (b.guided == kGuidedAll) *reinterpret_cast<volatile unsigned long long *>(word) = total;
+      else atomicAdd(word, total);
     }
+  }
+  if (b.profile && lane == 0) {
+    const unsigned long long t = global_ns();
+    unsigned long long *ends = ctr_ptr(b.counters, kCtrProfEnds);
+    atomicMax(ends + kProfStart, ~t_enter);
+    atomicMax(ends + kProfChunk, t);
+    atomicAdd(ctr_ptr(b.counters, kCtrProfSums) + kProfChunk, t - t_enter);
+    atomicAdd(ctr_ptr(b.counters, kCtrProfSums) + kProfSteps, 1ull);
   }
 }
 

@@ -428,8 +428,11 @@ int decode_blocks_per_sm(int occupancy_bps, const Tuning &tn) {
 
 cudaError_t launch_pipeline(const Context *ctx, const DevBatch &b, const Tuning &tn,
                             cudaStream_t s, cudaEvent_t mid) {
-  cudaError_t e = cudaMemsetAsync(b.counters, 0, kCtlBytes, s);
-  if (e != cudaSuccess) return e;
+  // the chunk kernel alone reads no control word
+  if (b.guided != kGuidedAll || b.profile) {
+    cudaError_t e = cudaMemsetAsync(b.counters, 0, kCtlBytes, s);
+    if (e != cudaSuccess) return e;
+  }
   if (mid) cudaEventRecord(mid, s);
   // persistent: as many blocks as are resident at once (fewer for a small batch,
   // whose shots and tiles would leave most warps idle)
@@ -555,12 +558,17 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
     b.num_shots = todo;
     b.shot_map = rounds == 0 ? nullptr : (const int *)ws->d_map;
     plan_batch(b, req.codes.data(), ncodes, ctx->sm_count, tn);
+    // the chunk kernel alone raises nothing in the course of a batch: its status word can
+    // be the host's own
+    const bool own = b.guided == kGuidedAll;
+    *ws->h_status = 0;
+    if (own) b.status = ws->h_status;
     if (timed) CK(cudaEventRecord(ws->ev[2], s));
     CK(launch_pipeline(ctx, b, tn, s, timed ? ws->ev[3] : nullptr));
     if (timed) CK(cudaEventRecord(ws->ev[4], s));
-    CK(cudaMemcpyAsync(ws->h_status, b.status, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    if (!own) CK(cudaMemcpyAsync(ws->h_status, b.status, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    const unsigned st = *ws->h_status;
+    const unsigned st = *reinterpret_cast<volatile unsigned *>(ws->h_status);
     if (timed) {
       float a = 0, c = 0;
       cudaEventElapsedTime(&a, ws->ev[2], ws->ev[3]);

@@ -57,12 +57,14 @@ static void run_guided_batch(DevBatch &b, int N) {
   b.epoch = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(small) + kCtlBytes);
   if (b.guided) {
     const int chunks = (N - 1) / b.chunk + 1;
-    for (blockIdx.x = 0; (int)blockIdx.x * kChunkWarps < chunks; ++blockIdx.x)
+    gridDim.x = (unsigned)((chunks - 1) / kChunkWarps + 1);
+    for (blockIdx.x = 0; blockIdx.x < gridDim.x; ++blockIdx.x)
       run_block(kChunkWarps * 32, [&] {
         if (b.has_ml) chunk_kernel<true>(b);
         else chunk_kernel<false>(b);
       });
     blockIdx.x = 0;
+    gridDim.x = 1;
   }
   if (b.guided != kGuidedAll)
     run_block(kDecodeWarps * 32, [&] {
