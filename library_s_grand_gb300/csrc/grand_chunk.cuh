@@ -40,7 +40,8 @@ __device__ __forceinline__ void xor_col(const uint32_t *cols, bool wide, unsigne
 constexpr int kFastWords = 8;         // syndrome words of a lane's shot (R <= 256)
 constexpr int kFastLogWords = 4;      // DEM logical words (n_logicos <= 128)
 constexpr int kFastErrWords = 32;     // error-record words (m <= 1024)
-constexpr int kFastLogBallots = kMaxChunk * kFastLogWords;  // ballot words of separate logical entries
+// words of a chunk's separate logical entries (flat_ballots)
+constexpr int kLogBallots = kMaxChunk * kFastLogWords + 8;
 
 // A chunk in its warp's shared memory.  A shot's row holds its syndrome (words 0 .. 7),
 // sketch (8), supplied weight (9) and logical words (10 .. 13) while it is open, and its
@@ -52,11 +53,11 @@ struct alignas(16) FastArea {
   int at[kMaxChunk];                    // where its record starts in bits (-1: elsewhere)
   uint8_t state[kMaxChunk];             // 0: open, 1: settled
   uint32_t bits[kFastBallots + 8];      // the run's records, entry after entry (flat_ballots)
-  uint32_t lbits[kFastLogBallots + 8];  // the same for DEM logicals kept in their own array
 };
 constexpr int kRowSketch = kFastWords, kRowWeight = kFastWords + 1, kRowLog = kFastWords + 2;
 static_assert(kRowLog + kFastLogWords <= 18, "an open shot's words fit its row");
-static_assert(sizeof(FastArea) <= sizeof(WarpArea), "FastArea must fit the decode kernel's area");
+static_assert(sizeof(FastArea) + 4 * kLogBallots <= sizeof(WarpArea),
+              "FastArea must fit the decode kernel's area");
 
 // The nonzero flags of the n entries at p as a bit vector: entry e is bit pad + e, with
 // pad (returned, 0 .. 3) the entries between p and the 16-byte boundary below it; other
@@ -152,7 +153,7 @@ __device__ __forceinline__ void bits_to_bytes(unsigned char *out, int n, uint32_
 }
 
 // Classifies the shots of launch slots size * chunk + [0, size), size <= kMaxChunk, into F.
-// hot: the block's copies of the codes (nullptr: none).  Returns the mask of the lanes whose
+// hot: the block's copies of the codes (nullptr: none); lbits: kLogBallots words of scratch.  Returns the mask of the lanes whose
 // shots the guided search takes: open, with their syndrome, sketch, supplied weight and
 // logical words in their row.
 //
@@ -163,7 +164,8 @@ __device__ __forceinline__ void bits_to_bytes(unsigned char *out, int n, uint32_
 // 0/1 matrices regular or not), a solo column found by the syndrome's sketch.
 template <bool MLK>
 __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotCode *hot, int chunk,
-                                                   int size, FastArea &F, ChunkStats &st) {
+                                                   int size, FastArea &F, uint32_t *lbits,
+                                                   ChunkStats &st) {
   const int lane = threadIdx.x & 31;
   const int slot = chunk * size + lane;
   const bool valid = lane < size && slot < b.num_shots;
@@ -202,7 +204,7 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
     if (__any_sync(kFull, ok && dem && log_ok)) {
       const int first = chunk * size;
       const int cnt = b.num_shots - first < size ? b.num_shots - first : size;
-      lpad = flat_ballots(b.in_log + (long long)first * cd.n_logicos, cnt * cd.n_logicos, F.lbits);
+      lpad = flat_ballots(b.in_log + (long long)first * cd.n_logicos, cnt * cd.n_logicos, lbits);
       __syncwarp();
     }
   }
@@ -263,7 +265,7 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
           uint32_t w = 0u;
           if (k < cd.nlw) {
             if (lw) w = __ldcg(lw + k) & (rem < 32 ? (1u << rem) - 1u : kFull);
-            else if (sep) w = flat_word(F.lbits, lpad + lane * cd.n_logicos, k, cd.n_logicos);
+            else if (sep) w = flat_word(lbits, lpad + lane * cd.n_logicos, k, cd.n_logicos);
             else w = flat_word(F.bits, at + cd.R, k, cd.n_logicos);
           }
           row[kRowLog + k] = w;

@@ -65,8 +65,7 @@ constexpr int kGuidedF = 15;            // filter bits, log2 (4 KB)
 constexpr int kMaxChunk = 32;
 constexpr int kFastBallots = 256;
 constexpr int kGuidedLanes = 8;         // lanes that search a shot (a warp searches 32 / 8 at once)
-constexpr int kGuidedItems = 512;       // partial sets a warp's searches hold (a shot: 1/4 of them, or
-                                        // all when the warp searches it alone)
+constexpr int kGuidedItems = 384;       // partial sets a warp's searches hold together
 constexpr int kHotCodes = 8;            // codes a block of the chunk kernel copies to shared memory
 constexpr int kChunkWarps = 4;          // warps per block of the chunk kernel
 constexpr int kChunkMinBlocks = 4;      // its resident blocks per SM (3 / 4 / 5: mix 93 / 77 / 81 us,

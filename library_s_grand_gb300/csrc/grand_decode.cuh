@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
     a0 = __shfl_sync(kFull, a0, 0);
     if (step == kStepChunk) {
       FastArea &F = *reinterpret_cast<FastArea *>(&A);
-      classify_chunk<MLK>(b, nullptr, (int)a0, chunk, F, st);
+      classify_chunk<MLK>(b, nullptr, (int)a0, chunk, F, reinterpret_cast<uint32_t *>(&F + 1), st);
       write_chunk(b, nullptr, (int)a0, chunk, F, tag);
       cache.stage_lost();
     } else if (step == kStepShot) {

@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
   const unsigned tag = *reinterpret_cast<volatile unsigned *>(b.epoch) + 1u;
   const unsigned long long t_enter = b.profile ? global_ns() : 0ull;
   FastArea &F = areas[wib].fast;
+  GuidedArea &A = areas[wib].guided;
   ChunkStats st{0, 0, 0};
 
   // the codes, and one load per 128-byte line of their tables and of the candidate counts
@@ -77,7 +78,10 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
   }
 
   unsigned mine = 0u;
-  if (has) mine = classify_chunk<MLK>(b, hot, chunk, b.chunk, F, st);
+  if (has) {
+    static_assert(4 * kLogBallots <= sizeof(A.item), "the logicals' ballots fit the items");
+    mine = classify_chunk<MLK>(b, hot, chunk, b.chunk, F, reinterpret_cast<uint32_t *>(A.item), st);
+  }
   if (mine) {
     int base = 0;
     if (lane == 0) base = atomicAdd(&open_count, __popc(mine));
@@ -98,13 +102,13 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
     at = __shfl_sync(kFull, at, 0);
     if (at >= count) break;
     const int cnt = count - at < take ? count - at : take;
-    int r = guided_pass<MLK>(b, hot, areas[wib].guided, &areas[0].fast, sizeof(ChunkArea), open + at, cnt);
+    int r = guided_pass<MLK>(b, hot, A, &areas[0].fast, sizeof(ChunkArea), open + at, cnt);
     st.guided += __popc(r & 255);
     st.heavy += __popc(r >> 8);
     if (!r && cnt > 1) {  // levels that outgrow the items together
 #pragma unroll 1
       for (int k = 0; k < cnt; ++k) {
-        r = guided_pass<MLK>(b, hot, areas[wib].guided, &areas[0].fast, sizeof(ChunkArea), open + at + k, 1);
+        r = guided_pass<MLK>(b, hot, A, &areas[0].fast, sizeof(ChunkArea), open + at + k, 1);
         st.guided += __popc(r & 255);
         st.heavy += __popc(r >> 8);
       }
