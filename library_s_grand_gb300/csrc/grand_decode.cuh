@@ -50,6 +50,9 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
   __shared__ WarpArea areas[kDecodeWarps];
   __shared__ PlanState plans[kDecodeWarps];
   __shared__ TileView views[kDecodeWarps];
+  // After a chunk kernel that left nothing in the queue there is nothing to do, and no entry
+  // or Job carries this launch's tag, so the epoch may stay (3 us in place of 9).
+  if (b.guided && (ld_ctr(b, kCtrChunks) & 0xffffffffull) == 0ull) return;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   WarpArea &A = areas[wib];

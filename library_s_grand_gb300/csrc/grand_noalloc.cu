@@ -15,10 +15,12 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "grand_common.h"
 #include "grand_host.h"
+#include "grand_prep.cuh"
 
 namespace grand {
 namespace {
@@ -35,7 +37,9 @@ constexpr size_t kOffCode = align256(kOffNcr + sizeof(unsigned long long) * (kMa
 constexpr size_t kOffCols = align256(kOffCode + sizeof(DevCode));
 constexpr size_t kOffColw = align256(kOffCols + sizeof(uint32_t) * kNaMaxCols * 8);
 constexpr size_t kOffHcol = align256(kOffColw + sizeof(int) * kNaMaxCols);
-constexpr size_t kOffSmall = align256(kOffHcol + sizeof(uint32_t) * kNaMaxCols);  // control block
+constexpr size_t kOffUpto = align256(kOffHcol + sizeof(uint32_t) * kNaMaxCols);
+constexpr size_t kOffGuided = align256(kOffUpto + 8 * sizeof(unsigned long long) * (kGuidedMaxCols + 1));
+constexpr size_t kOffSmall = align256(kOffGuided + sizeof(uint32_t) * kPrepWords);  // control block
 constexpr size_t kOffDeferred = align256(kOffSmall + kCtlAllocBytes);
 constexpr size_t kOffMap = align256(kOffDeferred + sizeof(int) * kNaChunk);     // re-run list
 constexpr size_t kOffMapCount = align256(kOffMap + sizeof(int) * kNaChunk);     // its length
@@ -53,10 +57,12 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 namespace {
 
-// C(n, k) by the same multiplicative formula as the host table.
-__global__ void noalloc_ncr_kernel(unsigned long long *t) {
+// C(n, k) by the same multiplicative formula as the host table, and their sums over k
+// (DevBatch::upto).
+__global__ void noalloc_ncr_kernel(unsigned long long *t, unsigned long long *upto) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n > kMaxTam) return;
+  unsigned long long sum = 0;
   for (int k = 0; k <= kMaxW; ++k) {
     unsigned long long r = 0;
     if (k <= n) {
@@ -65,53 +71,10 @@ __global__ void noalloc_ncr_kernel(unsigned long long *t) {
         for (int i = 1; i <= k; ++i) r = r * (unsigned long long)(n - i + 1) / (unsigned long long)i;
     }
     t[n * (kMaxW + 1) + k] = r;
+    if (k) sum += r;
+    if (n <= kGuidedMaxCols) upto[8 * n + k] = sum;
   }
-}
-
-// One thread per column: packed bits (LSB-first, nwp words), the column weight
-// and the column sketch.
-__global__ void noalloc_pack_kernel(const int *H, int n, int m, int nwp, uint32_t *cols, int *colw,
-                                    uint32_t *hcol) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m) return;
-  uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-  uint32_t h = 0u;
-  int sum = 0;
-  for (int r = 0; r < n; ++r) {
-    const int v = H[(size_t)r * m + c];
-    sum += v;
-    if (v != 0) {
-      w[r >> 5] |= 1u << (r & 31);
-      h ^= row_hash(r);
-    }
-  }
-  for (int i = 0; i < nwp; ++i) cols[(size_t)c * nwp + i] = w[i];
-  colw[c] = sum;
-  hcol[c] = h;
-}
-
-// One block: maximum column weight and regularity, then the code descriptor.
-__global__ void noalloc_code_kernel(DevCode tmpl, const int *colw, int m, DevCode *out) {
-  __shared__ int s_max, s_irregular;
-  if (threadIdx.x == 0) {
-    s_max = 0;
-    s_irregular = 0;
-  }
-  __syncthreads();
-  int mx = 0, irr = 0;
-  const int c0 = colw[0];
-  for (int c = threadIdx.x; c < m; c += blockDim.x) {
-    mx = max(mx, colw[c]);
-    irr |= colw[c] != c0;
-  }
-  atomicMax(&s_max, mx);
-  if (irr) atomicOr(&s_irregular, 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    tmpl.max_soma = s_max;
-    tmpl.regular = s_irregular ? 0 : 1;
-    *out = tmpl;
-  }
+  if (n <= kGuidedMaxCols) upto[8 * n + 7] = sum;
 }
 
 // One warp: the ascending list of the chunk's shots that the last round deferred
@@ -141,6 +104,7 @@ __global__ void noalloc_clear_kernel(const int *map, int count, GrandDecoderResu
 std::mutex g_mu;
 unsigned char *g_base[64] = {};  // device address of g_noalloc_scratch per device
 int g_sms[64] = {}, g_bps[64] = {};
+unsigned *g_status[64] = {};     // pinned: the status word of a round, raised by the kernels in place
 
 }  // namespace
 }  // namespace grand
@@ -200,12 +164,17 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
       if (e == cudaSuccess) e = decode_occupancy(&bps);
       if (e == cudaSuccess) {
         noalloc_ncr_kernel<<<(kMaxTam + 256) / 256, 256, 0, s>>>(
-            reinterpret_cast<unsigned long long *>((unsigned char *)ptr + kOffNcr));
+            reinterpret_cast<unsigned long long *>((unsigned char *)ptr + kOffNcr),
+            reinterpret_cast<unsigned long long *>((unsigned char *)ptr + kOffUpto));
         e = cudaGetLastError();
       }
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) {
         fprintf(stderr, "grand_decode_cc_noalloc: set-up failed (%s)\n", cudaGetErrorString(e));
+        return GRAND_ERR_CUDA;
+      }
+      if (cudaHostAlloc(reinterpret_cast<void **>(&g_status[dev]), 256, cudaHostAllocDefault) != cudaSuccess) {
+        fprintf(stderr, "grand_decode_cc_noalloc: set-up failed (no pinned status word)\n");
         return GRAND_ERR_CUDA;
       }
       g_sms[dev] = sms;
@@ -242,8 +211,19 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
   t.colw = colw;
   t.hcol = hcol;
 
-  noalloc_pack_kernel<<<(m + 127) / 128, 128, 0, s>>>(d_H, n, m, nwp, cols, colw, hcol);
-  noalloc_code_kernel<<<1, 256, 0, s>>>(t, colw, m, code);
+  {
+    // whether a one-position first iteration is searched, should the code have solo columns
+    DevCode x = t;
+    static const int some = 0;
+    x.solo_cols = &some;
+    x.binary = x.max_soma = 1;
+    t.solo_branch = solo_branch_of(x);
+  }
+  // the code's tables, on every call (nothing is kept), and the control words of the first
+  // round cleared
+  prep_kernel<<<1, 1024, 0, s>>>(t, d_H, cols, colw, hcol, reinterpret_cast<uint32_t *>(base + kOffGuided),
+                                 code, reinterpret_cast<unsigned long long *>(base + kOffSmall),
+                                 kCtlBytes / 8);
   e = cudaGetLastError();
 
   const Tuning &tn = tuning();
@@ -262,10 +242,11 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
     b.in = d_syndromes + (size_t)lo * n;
     b.results = d_results + lo;
     b.ncr = reinterpret_cast<const unsigned long long *>(base + kOffNcr);
+    b.upto = reinterpret_cast<const unsigned long long *>(base + kOffUpto);
     b.jobs = reinterpret_cast<Job *>(base + kOffJobs);
     b.max_jobs = kNaChunk;
     b.counters = reinterpret_cast<unsigned long long *>(base + kOffSmall);
-    b.status = reinterpret_cast<unsigned *>(base + kOffSmall + kStatusByteOffset);
+    b.status = g_status[dev];
     b.scratch = reinterpret_cast<uint32_t *>(base + kOffArena);
     b.scratch_words = kNaArenaWords;
     b.deferred = reinterpret_cast<int *>(base + kOffDeferred);
@@ -282,15 +263,18 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
     for (int round = 0; e == cudaSuccess; ++round) {
       b.num_shots = todo;
       b.shot_map = round == 0 ? nullptr : map;
+      // The chunk kernel first where the code can have a guided search (decided on the
+      // device): what that leaves is in the slow queue.  Its chunks as plan_batch's.
+      b.guided = tn.fast && n <= kGuidedMaxRows ? kGuidedFirst : kGuidedNone;
+      b.chunk = std::min((todo - 1) / (g_sms[dev] * kChunkMinBlocks * kChunkWarps) + 1, (int)kMaxChunk);
       // control words and status restart for every round
-      e = cudaMemsetAsync(base + kOffSmall, 0, kCtlBytes, s);
+      if (lo > 0 || round > 0) e = cudaMemsetAsync(base + kOffSmall, 0, kCtlBytes, s);
+      volatile unsigned *status = g_status[dev];
+      *status = 0u;
       if (e == cudaSuccess) e = launch_decode(b, g_sms[dev] * per_sm, s);
-      unsigned rs = 0;
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&rs, base + kOffSmall + kStatusByteOffset, sizeof(unsigned),
-                            cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) break;
+      const unsigned rs = *status;
       st |= rs & ~(unsigned)(kStatusScratchOverflow | kStatusJobOverflow);
       if (!(rs & (kStatusScratchOverflow | kStatusJobOverflow))) break;
       noalloc_deferred_kernel<<<1, 32, 0, s>>>(b.deferred, cnt, map, map_count);

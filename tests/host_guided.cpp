@@ -3,9 +3,10 @@
 // host_kernels.cpp, whose own codes carry no such tables and so take the general
 // path throughout, with them built as the library builds them.
 //
-// Usage: host_guided DIR   single-code directories of host_kernels.cpp; prints the
+// Usage: host_guided DIR [prep]   single-code directories of host_kernels.cpp; prints the
 // same line, then the kernels that ran (enum GuidedMode) and the number of shots past
-// the light budget that the guided search finished.
+// the light budget that the guided search finished.  prep: instead, checks the tables
+// that prep_kernel builds against the host's (exit code 0: equal).
 #define main host_kernels_main
 #include "host_kernels.cpp"
 #undef main
@@ -23,7 +24,21 @@ static void __syncthreads() {
 }
 static inline int atomicAdd(int *a, int v) { return __atomic_fetch_add(a, v, __ATOMIC_SEQ_CST); }
 
+static inline int atomicMax(int *a, int v) {
+  int cur = __atomic_load_n(a, __ATOMIC_SEQ_CST);
+  while (v > cur && !__atomic_compare_exchange_n(a, &cur, v, false, __ATOMIC_SEQ_CST, __ATOMIC_SEQ_CST)) {
+  }
+  return cur;
+}
+static inline int atomicMin(int *a, int v) {
+  int cur = __atomic_load_n(a, __ATOMIC_SEQ_CST);
+  while (v < cur && !__atomic_compare_exchange_n(a, &cur, v, false, __ATOMIC_SEQ_CST, __ATOMIC_SEQ_CST)) {
+  }
+  return cur;
+}
+
 #include "grand_front.cuh"
+#include "grand_prep.cuh"
 #include "grand_guided_tables.h"
 
 // The kernels of a batch as the library launches them (launch_kernels).
@@ -78,12 +93,58 @@ static void run_guided_batch(DevBatch &b, int N) {
   if (*b.status) exit(4);
 }
 
+// The device-built tables of a code against the host's.
+static int check_prep(const std::string &dir, const Code &k, const GuidedTables &g) {
+  const std::vector<int> H = read_ints(dir + "/H.bin", (size_t)k.n * k.m);
+  alignas(16) static uint32_t guided[kPrepWords], cols[kPrepMaxCols * 8], hcol[kPrepMaxCols];
+  static int colw[kPrepMaxCols];
+  static unsigned long long control[8] = {1, 1, 1, 1, 1, 1, 1, 1};
+  DevCode tmpl = k.d, got;
+  tmpl.g_gs = 0;
+  tmpl.solo_branch = kSoloCpu;
+  run_block(128, [&] { prep_kernel(tmpl, H.data(), cols, colw, hcol, guided, &got, control, 7); });
+  bool same = control[6] == 0 && control[7] == 1;
+  int most = 0, regular = 1;
+  for (int c = 0; c < k.m; ++c) {
+    int sum = 0;
+    for (int r = 0; r < k.n; ++r) sum += H[(size_t)r * k.m + c];
+    same = same && colw[c] == sum && hcol[c] == k.hcol[c];
+    most = std::max(most, sum);
+    regular = regular && colw[c] == colw[0];
+  }
+  same = same && got.max_soma == most && got.regular == regular;
+  same = same && !memcmp(cols, k.cols.data(), sizeof(uint32_t) * k.cols.size());
+  if (g.words.empty()) return same && got.g_gs == 0 && got.solo_branch == kSoloNone ? 0 : 5;
+  const uint32_t *w = g.words.data();
+  const int mw = (k.m + 31) / 32;
+  same = same && got.solo_branch == kSoloCpu && got.g_gs == g.gs && got.g_deg == g.deg &&
+         got.g_max_cw == g.max_cw && got.g_odd == g.odd && got.g_tab_mask == g.tab_mask;
+  same = same && !memcmp(got.g_rows, w + g.o_rows, 4 * (size_t)(k.n + 1) * mw);
+  same = same && !memcmp(got.g_cw, w + g.o_cw, 4 * (size_t)3 * mw);
+  same = same && !memcmp(got.g_adj, w + g.o_adj, 2 * (size_t)k.n * g.deg);
+  same = same && !memcmp(got.g_cols, w + g.o_cols, 4 * (size_t)k.m * g.gs);
+  same = same && !memcmp(got.g_filt, w + g.o_filt, 4u << (kGuidedF - 5));
+  same = same && !memcmp(got.g_hcol, w + g.o_hcol, 4 * (size_t)k.m);
+  for (int c = 0; c < k.m && same; ++c) {  // the table: the same entries, each where a probe finds it
+    uint32_t host = kNoCol, dev = kNoCol;
+    for (uint32_t p = 0, i = k.hcol[c] & g.tab_mask; p <= g.tab_mask; ++p, i = (i + 1) & g.tab_mask) {
+      const uint32_t a = w[g.o_tab + 2 * i + 1], b = got.g_tab[2 * i + 1];
+      if ((a & 0xffffu) == (uint32_t)c) host = a;
+      if (dev == kNoCol && (b & 0xffffu) == (uint32_t)c && got.g_tab[2 * i] == k.hcol[c]) dev = b;
+      if ((b & 0xffffu) == kNoCol && dev == kNoCol) break;
+    }
+    same = host != kNoCol && host == dev;
+  }
+  return same ? 0 : 5;
+}
+
 int main(int argc, char **argv) {
-  if (argc != 2) return 2;
+  if (argc != 2 && argc != 3) return 2;
   const std::string dir = argv[1];
   Code k;
   if (!load_code(dir, k)) return 2;
   const GuidedTables g = build_guided_tables(k.cols, k.d.nwp, k.n, k.m, k.hcol, k.d.binary != 0, k.solo);
+  if (argc == 3) return check_prep(dir, k, g);
   std::vector<uint32_t> aligned(g.words.size() + 4);
   uint32_t *base = aligned.data();
   while (reinterpret_cast<uintptr_t>(base) & 15u) ++base;

@@ -12,7 +12,7 @@ import pytest
 
 import oracle as O
 from library_s_grand_gb300 import synth
-from test_host_kernels import HERE, ROOT, _compare, _cuda_include, _run
+from test_host_kernels import HERE, ROOT, _compare, _cuda_include, _run, _write_code
 
 
 @pytest.fixture(scope="module")
@@ -160,3 +160,26 @@ def test_levels_that_do_not_fit(guided, port, tmp_path):
     assert prc == 0
     _compare(res, dec, pres, pdec)
     assert out.split("\n")[1].startswith("guided 1 ") and _jobs(out) > 0, out
+
+
+@pytest.mark.parametrize("kind", ["bb72", "bb108", "bb288", "odd", "dense", "entries", "limit"])
+def test_tables_built_on_the_device(guided, tmp_path, kind):
+    """The allocation-free entry point's tables (csrc/grand_prep.cuh) equal the library's: 4-
+    and 8-word columns, empty, duplicated and nested columns, codes without a guided
+    search (dense, entries other than 0 and 1) and the entry point's largest matrix."""
+    rng = np.random.default_rng(5)
+    if kind.startswith("bb"):
+        h = synth.BB_CODES[int(kind[2:])]().hz
+    elif kind == "odd":
+        h = _dem("odd", 8).h.copy()
+        h[:, 9] |= h[:, 8]  # a column that holds another
+    elif kind == "dense":
+        h = (rng.random((40, 70)) < 0.4).astype(np.int32)
+    elif kind == "entries":
+        h = synth.BB_CODES[72]().hz.copy()
+        h[3, 5] += 2
+    else:
+        h = synth.random_dem(2, detectors=256, mechanisms=1024).h
+    _write_code(str(tmp_path / "code"), h, 0, 0, (3, 256, 0, 64, 10, -1), [], Ho=h)
+    p = subprocess.run([guided, str(tmp_path / "code"), "prep"], capture_output=True, text=True)
+    assert p.returncode == 0, p.stderr
