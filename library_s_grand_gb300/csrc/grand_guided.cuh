@@ -541,6 +541,13 @@ __device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, G
         const unsigned acts = __ballot_sync(kFull, act);
         const unsigned probes = __ballot_sync(kFull, act && w >= w_first && !(odd && ((w ^ ones) & 1)));
         const unsigned pushes = __ballot_sync(kFull, act && w < w_last);
+        if (d == 0) {
+          // weight 1 ends here unless a root's sketch passes its filter
+          const uint32_t f = hs >> (32 - kGuidedF);
+          const bool pass = gl == 0 && ((probes >> gb) & 1u) &&
+                            ((__ldg(cd.g_filt + (f >> 5)) >> (f & 31u)) & 1u);
+          if (!__any_sync(kFull, pass)) continue;
+        }
         if (gl == 0) S.limit = max_cw * (w_last - d);
         __syncwarp();
         unsigned long long bkey = kNone;  // the group's best of this weight
@@ -580,10 +587,9 @@ __device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, G
                 found_one = c != kNoCol && ((T.am[i][(c >> 5) & 31u] >> (c & 31u)) & 1u);
               }
             }
+            if (p0 + 32 >= pairs) drained = !__any_sync(kFull, zeros);  // (ML, or weights out of order)
           } else {
-            if (zi < 0 && !__any_sync(kFull, zeros)) {  // (zeros: ML, or weights out of order)
-              drained = true;
-            } else if (!__any_sync(kFull, zbits != 0u)) {
+            if (!__any_sync(kFull, zbits != 0u)) {
               zi = zi < 0 ? lo : zi + 1;
               while (zi < hi && !((item[zi].y & 1023u) == kNoRow && ((acts >> (G * (item[zi].y >> 30))) & 1u)))
                 ++zi;
