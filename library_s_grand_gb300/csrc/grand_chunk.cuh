@@ -248,12 +248,21 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
       row[6] = s.b.z;
       row[7] = s.b.w;
     } else {
+#pragma unroll
+      for (int k = 0; k < kFastWords; ++k) row[k] = 0u;
+      // the sketch: four rows at a time from the code's table, where it has one
 #pragma unroll 1
-      for (int k = 0; k < kFastWords; ++k) {
-        uint32_t w = k < nw ? word(k) : 0u;
+      for (int k = 0; k < nw; ++k) {
+        uint32_t w = word(k);
         row[k] = w;
+        if (cd.g_gs) {
+          const uint32_t *nib = cd.g_nib + 128 * k;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) hs ^= __ldg(nib + 16 * u + ((w >> (4 * u)) & 15u));
+        } else {
 #pragma unroll 1
-        for (; w; w &= w - 1u) hs ^= row_hash(k * 32 + __ffs((int)w) - 1);
+          for (; w; w &= w - 1u) hs ^= row_hash(k * 32 + __ffs((int)w) - 1);
+        }
       }
       if (dem) {
         const uint32_t *lw = rw ? (sep ? reinterpret_cast<const uint32_t *>(b.in_log) + (size_t)shot * cd.nlw

@@ -42,6 +42,16 @@ GRAND_HD inline uint32_t row_hash(int r) {
   return x;
 }
 
+// Word i of the sketch table of R rows, four at a time (nib_words of them, for whole words
+// of 32 rows): the sketch of the rows 4 (i / 16) + b with bit b of i % 16 set.
+GRAND_HD inline int nib_words(int R) { return (R + 31) / 32 * 128; }
+GRAND_HD inline uint32_t nib_sketch(int i) {
+  uint32_t h = 0u;
+  for (int b = 0; b < 4; ++b)
+    if ((i >> b) & 1) h ^= row_hash(4 * (i >> 4) + b);
+  return h;
+}
+
 constexpr int kMaxW = GRAND_MAX_W;        // searched weights 1..6
 constexpr int kMaxTam = GRAND_MAX_TAM;    // largest active set searched
 constexpr int kMaxRows = 1024;            // R <= 1024  -> nw <= 32
@@ -178,7 +188,7 @@ struct HotCode {
   uint32_t g_tab_mask;
   int g_words;                 // the tables lie in one block of g_words words from g_rows on
   unsigned long long g_magic;  // ceil(2^32 / g_deg)
-  const uint32_t *g_rows, *g_cw, *g_cols, *g_filt, *g_tab, *g_hcol;
+  const uint32_t *g_rows, *g_cw, *g_cols, *g_filt, *g_tab, *g_hcol, *g_nib;
   const uint16_t *g_adj;
   const uint32_t *lcols;     // m * nlw
   const float *llr;          // m

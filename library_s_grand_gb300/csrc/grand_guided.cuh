@@ -214,12 +214,17 @@ struct GuidedWinner {
   int w_done;               // ML: last weight searched (the bound may stop it early)
 };
 
-// x added to the counters of each bit position.
-__device__ __forceinline__ void add_bits(uint32_t x, uint32_t &c0, uint32_t &c1, uint32_t &c2) {
-  const uint32_t t = c0 & x;
-  c0 ^= x;
-  c2 ^= c1 & t;
-  c1 ^= t;
+// Four rows added to the counters of each bit position (mod 8), by full adders.
+__device__ __forceinline__ uint32_t majority(uint32_t a, uint32_t b, uint32_t c) {
+  return (a & b) | (a & c) | (b & c);
+}
+__device__ __forceinline__ void add_rows(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,
+                                         uint32_t &c0, uint32_t &c1, uint32_t &c2) {
+  const uint32_t s = x0 ^ x1 ^ x2, m = majority(x0, x1, x2);
+  const uint32_t n = majority(c0, s, x3);
+  c0 ^= s ^ x3;
+  c2 ^= majority(c1, m, n);
+  c1 ^= m ^ n;
 }
 
 // Are the bits of delta (word `lane` of the difference of two errors with one syndrome)
@@ -363,10 +368,7 @@ __device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, G
         const uchar4 r = *reinterpret_cast<const uchar4 *>(row_list + i);
         const uint32_t x0 = __ldg(rows + (int)r.x * mw), x1 = __ldg(rows + (int)r.y * mw),
                        x2 = __ldg(rows + (int)r.z * mw), x3 = __ldg(rows + (int)r.w * mw);
-        add_bits(x0, c0, c1, c2);
-        add_bits(x1, c0, c1, c2);
-        add_bits(x2, c0, c1, c2);
-        add_bits(x3, c0, c1, c2);
+        add_rows(x0, x1, x2, x3, c0, c1, c2);
       }
       const uint32_t w0 = __ldg(cd.g_cw + q), w1 = __ldg(cd.g_cw + mw + q), w2 = __ldg(cd.g_cw + 2 * mw + q);
       // missing = weight - count, bit by bit; zero columns are never active

@@ -13,6 +13,8 @@
 //          pairs (column kNoCol = empty slot; kSoloFlag set for a solo column,
 //          grand_solo.h), at most half full
 //   hcol   the column sketches
+//   nib    the sketches of four rows at a time: nib[16 i + v] is that of the rows 4i + b
+//          with bit b of v set
 //
 // A code has them when its matrix is 0/1, with at most 255 rows, 1024 columns, 7
 // ones per column and 64 per row: the search keeps a residual syndrome in 4 or 8
@@ -35,7 +37,7 @@ struct GuidedTables {
   int gs = 0, deg = 0, max_cw = 0, odd = 1;
   uint32_t tab_mask = 0;
   // one block of words; the parts start at these word offsets (16-byte aligned)
-  size_t total = 0, o_rows = 0, o_cw = 0, o_adj = 0, o_cols = 0, o_filt = 0, o_tab = 0, o_hcol = 0;
+  size_t total = 0, o_rows = 0, o_cw = 0, o_adj = 0, o_cols = 0, o_filt = 0, o_tab = 0, o_hcol = 0, o_nib = 0;
   std::vector<uint32_t> words;  // empty: the code has no guided search
 };
 
@@ -78,6 +80,7 @@ inline GuidedTables build_guided_tables(const std::vector<uint32_t> &cols, int n
   g.o_filt = part((size_t)1 << (kGuidedF - 5));
   g.o_tab = part((size_t)2 * slots);
   g.o_hcol = part((size_t)m);
+  g.o_nib = part(nib_words(R));
   g.total = top;
   g.words.assign(top, 0u);
   uint32_t *w = g.words.data();
@@ -103,6 +106,7 @@ inline GuidedTables build_guided_tables(const std::vector<uint32_t> &cols, int n
     w[g.o_tab + 2 * i + 1] = (uint32_t)c;
   }
   memcpy(w + g.o_hcol, hcol.data(), sizeof(uint32_t) * m);
+  for (int i = 0; i < nib_words(R); ++i) w[g.o_nib + i] = nib_sketch(i);
   for (size_t k = 0; k < solo.cols.size(); ++k) {
     if (solo.cols[k] < 0) continue;
     uint32_t i = solo.keys[k] & g.tab_mask;
@@ -128,6 +132,7 @@ inline void set_guided(DevCode &d, const GuidedTables &g, const uint32_t *base) 
   d.g_filt = base + g.o_filt;
   d.g_tab = base + g.o_tab;
   d.g_hcol = base + g.o_hcol;
+  d.g_nib = base + g.o_nib;
   d.g_words = (int)g.total;
 }
 

@@ -19,7 +19,7 @@ constexpr int kPrepMaxRows = 256, kPrepMaxCols = 1024;
 
 // Offsets of the guided tables in their block, for the largest degree (words).
 struct PrepLayout {
-  int rows, cw, adj, cols, filt, tab, hcol, total;
+  int rows, cw, adj, cols, filt, tab, hcol, nib, total;
 };
 GRAND_HD inline PrepLayout prep_layout(int n, int m, int deg, int slots) {
   PrepLayout L;
@@ -31,12 +31,13 @@ GRAND_HD inline PrepLayout prep_layout(int n, int m, int deg, int slots) {
   L.filt = L.cols + m * gs;
   L.tab = L.filt + (1 << (kGuidedF - 5));
   L.hcol = L.tab + 2 * slots;
-  L.total = L.hcol + ((m + 3) & ~3);
+  L.nib = L.hcol + ((m + 3) & ~3);
+  L.total = L.nib + nib_words(n);
   return L;
 }
 // Words the guided tables can take at the entry point's limits.
 constexpr size_t kPrepWords = (kPrepMaxRows + 1) * 32 + 96 + kPrepMaxRows * kGuidedMaxDegree / 2 +
-                              kPrepMaxCols * 8 + (1 << (kGuidedF - 5)) + 4 * kPrepMaxCols + kPrepMaxCols + 64;
+                              kPrepMaxCols * 8 + (1 << (kGuidedF - 5)) + 4 * kPrepMaxCols + kPrepMaxCols + 1024 + 64;
 
 struct PrepShared {
   uint32_t bits[(kPrepMaxRows + 1) * 32];  // the rows, then the sketch table
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(1024, 1) prep_kernel(const DevCode tmpl, const
       for (int k = base + lane; k < deg; k += 32) adj[r * deg + k] = (uint16_t)kNoCol;
     }
     for (int i = t; i < (n + 1) * mw; i += T) guided[L.rows + i] = S.bits[i];
+    for (int i = t; i < nib_words(n); i += T) guided[L.nib + i] = nib_sketch(i);
     for (int i = t; i < 96; i += T)
       if ((i & 31) < mw) guided[L.cw + (i >> 5) * mw + (i & 31)] = S.cw[i >> 5][i & 31];
     for (int i = t; i < (1 << (kGuidedF - 5)); i += T) guided[L.filt + i] = S.filt[i];
@@ -256,6 +258,7 @@ __global__ void __launch_bounds__(1024, 1) prep_kernel(const DevCode tmpl, const
       d.g_filt = guided + L.filt;
       d.g_tab = guided + L.tab;
       d.g_hcol = guided + L.hcol;
+      d.g_nib = guided + L.nib;
       d.g_adj = reinterpret_cast<const uint16_t *>(guided + L.adj);
     } else {
       d.solo_branch = kSoloNone;

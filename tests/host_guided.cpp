@@ -125,6 +125,7 @@ static int check_prep(const std::string &dir, const Code &k, const GuidedTables 
   same = same && !memcmp(got.g_cols, w + g.o_cols, 4 * (size_t)k.m * g.gs);
   same = same && !memcmp(got.g_filt, w + g.o_filt, 4u << (kGuidedF - 5));
   same = same && !memcmp(got.g_hcol, w + g.o_hcol, 4 * (size_t)k.m);
+  same = same && !memcmp(got.g_nib, w + g.o_nib, 4 * (size_t)nib_words(k.n));
   for (int c = 0; c < k.m && same; ++c) {  // the table: the same entries, each where a probe finds it
     uint32_t host = kNoCol, dev = kNoCol;
     for (uint32_t p = 0, i = k.hcol[c] & g.tab_mask; p <= g.tab_mask; ++p, i = (i + 1) & g.tab_mask) {
