@@ -13,6 +13,7 @@ fails loudly when it has not been built.
 from __future__ import annotations
 
 import ctypes
+import mmap
 import os
 
 import numpy as np
@@ -125,17 +126,63 @@ def _flat(a):
     return np.ascontiguousarray(np.asarray(a).ravel(), dtype=np.int32)
 
 
+_INT1 = ctypes.c_int * 1
+_NULL = IP()
+
+
 def _p(a):
-    return a.ctypes.data_as(IP)
+    """A (POINTER(c_int)) argument for a's memory; the buffer protocol is four times as fast
+    as a.ctypes.data_as, which remains for what it does not take (read-only, empty)."""
+    try:
+        return _INT1.from_buffer(a)
+    except (TypeError, ValueError):
+        return a.ctypes.data_as(IP)
+
+
+# Output buffers the library fills are not zeroed first: that costs the time of the fill,
+# and again the GPU's, whose writes then find every line in the CPU's caches (16384
+# results: 8 + 13 us).  Their pages are touched, one byte each, so that the GPU does not
+# fault on them, and a call that did not decode leaves them zero as before.
+
+def _uninit(nbytes):
+    a = np.empty(nbytes, dtype=np.uint8)
+    a[::mmap.PAGESIZE] = 0
+    return a
+
+
+def _new_results(shots):
+    if shots < 64:
+        return (GrandDecoderResult * shots)()
+    return (GrandDecoderResult * shots).from_buffer(_uninit(72 * shots))
+
+
+_ERR_LIMIT = -3  # matrix beyond the size limits (not decoded), or an active set (decoded)
+
+
+def _undecoded(rc, n, m, nl=0):
+    return rc != 0 and (rc != _ERR_LIMIT or n > 1024 or m > 4096 or nl > 1024)
+
+
+def _finish(rc, results, n, m, nl=0, arrays=()):
+    if _undecoded(rc, n, m, nl):
+        ctypes.memset(results, 0, ctypes.sizeof(results))
+        for a in arrays:
+            a.fill(0)
+    return rc
+
+
+def _bytes_of(a, ctype):
+    """a's memory for a pointer field of GrandDecodeOutputs."""
+    return (ctype * 1).from_buffer(a) if a.size else None
 
 
 def _outputs(shots, m, nl, ml):
-    dec = np.zeros((shots, m), dtype=np.uint8)
-    dlog = np.zeros((shots, max(nl, 1)), dtype=np.uint8)
+    dec = _uninit(shots * m).reshape(shots, m)
+    dlog = _uninit(shots * nl).reshape(shots, nl) if nl else np.zeros((shots, 1), dtype=np.uint8)
     cost = np.zeros(shots, dtype=np.float32)
-    o = GrandDecodeOutputs(dec.ctypes.data_as(ctypes.POINTER(ctypes.c_ubyte)),
-                           dlog.ctypes.data_as(ctypes.POINTER(ctypes.c_ubyte)) if nl else None,
-                           cost.ctypes.data_as(ctypes.POINTER(ctypes.c_float)) if ml else None)
+    o = GrandDecodeOutputs(_bytes_of(dec, ctypes.c_ubyte),
+                           _bytes_of(dlog, ctypes.c_ubyte) if nl else None,
+                           _bytes_of(cost, ctypes.c_float) if ml else None)
     return o, dec, dlog[:, :nl], cost
 
 
@@ -147,31 +194,37 @@ def results_array(results) -> np.ndarray:
     return buf.copy()
 
 
+def _as_array(results) -> np.ndarray:
+    """A call's own ctypes results as a structured array, without a copy."""
+    return np.frombuffer(results, dtype=RESULT_DTYPE) if len(results) else results_array(results)
+
+
 def _css_args(Hx, Hz, errors, syndromes):
     n_rows, n_cols = np.asarray(Hx).shape
     hx, hz = _flat(Hx), _flat(Hz)
-    null = IP()
     if errors is not None:
         shots = np.asarray(errors).shape[0]
         e = _flat(errors)
-        return (hx, hz, e), [_p(hx), _p(hz), n_rows, n_cols, _p(e), null, shots], shots, n_cols
+        return (hx, hz, e), [_p(hx), _p(hz), n_rows, n_cols, _p(e), _NULL, shots], shots, n_cols
     shots = np.asarray(syndromes).shape[0]
     s = _flat(syndromes)
-    return (hx, hz, s), [_p(hx), _p(hz), n_rows, n_cols, null, _p(s), shots], shots, n_cols
+    return (hx, hz, s), [_p(hx), _p(hz), n_rows, n_cols, _NULL, _p(s), shots], shots, n_cols
 
 
 def run_grand_shots_cc(lib, Hx, Hz, errors, syndromes, cfg, error_type):
     keep, args, shots, _ = _css_args(Hx, Hz, errors, syndromes)
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     rc = lib.grand_decode_cc(*args, ctypes.byref(cfg), results, ctypes.c_char(error_type))
+    _finish(rc, results, args[2], args[3])
     return rc, results
 
 
 def run_grand_prob_shots_cc(lib, Hx, Hz, errors, syndromes, cfg, prob_file_path, error_type):
     keep, args, shots, _ = _css_args(Hx, Hz, errors, syndromes)
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     rc = lib.grand_decode_prob_cc(*args, ctypes.byref(cfg), results, ctypes.c_char(error_type),
                                   prob_file_path.encode("utf-8"))
+    _finish(rc, results, args[2], args[3])
     return rc, results
 
 
@@ -185,24 +238,27 @@ def _dem_args(H_dem, L_dem, detectors, logicals, n_logicos):
 
 def run_grand_shots_cln(lib, H_dem, L_dem, detectors, logicals, n_logicos, cfg):
     keep, args, shots, _ = _dem_args(H_dem, L_dem, detectors, logicals, n_logicos)
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     rc = lib.grand_decode_cln(*args, ctypes.byref(cfg), results)
+    _finish(rc, results, args[2], args[3], n_logicos)
     return rc, results
 
 
 def run_grand_prob_shots_cln(lib, H_dem, L_dem, detectors, logicals, n_logicos, cfg,
                              prob_file_path):
     keep, args, shots, _ = _dem_args(H_dem, L_dem, detectors, logicals, n_logicos)
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     rc = lib.grand_decode_prob_cln(*args, ctypes.byref(cfg), results,
                                    prob_file_path.encode("utf-8"))
+    _finish(rc, results, args[2], args[3], n_logicos)
     return rc, results
 
 
 def run_grand_ML_shots_cln(lib, H_dem, L_dem, detectors, logicals, n_logicos, cfg, llr_file_path):
     keep, args, shots, _ = _dem_args(H_dem, L_dem, detectors, logicals, n_logicos)
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     rc = lib.grand_decode_ML_cln(*args, ctypes.byref(cfg), results, llr_file_path.encode("utf-8"))
+    _finish(rc, results, args[2], args[3], n_logicos)
     return rc, results
 
 
@@ -211,7 +267,7 @@ def run_grand_ML_shots_cln(lib, H_dem, L_dem, detectors, logicals, n_logicos, cf
 def decode_css_ex(lib, variant, Hx, Hz, errors, syndromes, cfg, error_type, prob_file=None):
     """variant: "uniform" or "prob".  Returns (rc, results ndarray, decoded errors)."""
     keep, args, shots, m = _css_args(Hx, Hz, errors, syndromes)
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     out, dec, _, _ = _outputs(shots, m, 0, False)
     et = ctypes.c_char(error_type if isinstance(error_type, bytes) else error_type.encode())
     if variant == "prob":
@@ -219,7 +275,8 @@ def decode_css_ex(lib, variant, Hx, Hz, errors, syndromes, cfg, error_type, prob
                                          os.fsencode(prob_file), ctypes.byref(out))
     else:
         rc = lib.grand_decode_cc_ex(*args, ctypes.byref(cfg), results, et, ctypes.byref(out))
-    return rc, results_array(results), dec
+    _finish(rc, results, args[2], m, 0, (dec,))
+    return rc, _as_array(results), dec
 
 
 def decode_dem_ex(lib, variant, H_dem, L_dem, detectors, logicals, cfg, file=None):
@@ -227,7 +284,7 @@ def decode_dem_ex(lib, variant, H_dem, L_dem, detectors, logicals, cfg, file=Non
     decoded errors, decoded logical flips, ML costs)."""
     nl = int(np.asarray(L_dem).shape[1])
     keep, args, shots, m = _dem_args(H_dem, L_dem, detectors, logicals, nl)
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     out, dec, dlog, cost = _outputs(shots, m, nl, variant == "ml")
     if variant == "prob":
         rc = lib.grand_decode_prob_cln_ex(*args, ctypes.byref(cfg), results, os.fsencode(file),
@@ -237,7 +294,8 @@ def decode_dem_ex(lib, variant, H_dem, L_dem, detectors, logicals, cfg, file=Non
                                         ctypes.byref(out))
     else:
         rc = lib.grand_decode_cln_ex(*args, ctypes.byref(cfg), results, ctypes.byref(out))
-    return rc, results_array(results), dec, dlog, cost
+    _finish(rc, results, args[2], m, nl, (dec, dlog))
+    return rc, _as_array(results), dec, dlog, cost
 
 
 PACKED_SYNDROMES, PACKED_ERRORS = 0, 1
@@ -266,10 +324,11 @@ def run_grand_shots_cc_packed(lib, Hx, Hz, words, kind, cfg, error_type, prob_fi
     hx, hz = _flat(Hx), _flat(Hz)
     w = np.ascontiguousarray(words, dtype=np.uint32)
     shots = w.shape[0]
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     rc = lib.grand_decode_cc_packed(_p(hx), _p(hz), n_rows, n_cols, w.ctypes.data, kind, shots,
                                     ctypes.byref(cfg), results, ctypes.c_char(_type_byte(error_type)),
                                     os.fsencode(prob_file) if prob_file else None)
+    _finish(rc, results, n_rows, n_cols)
     return rc, results
 
 
@@ -281,11 +340,12 @@ def decode_css_packed(lib, Hx, Hz, words, kind, cfg, error_type, prob_file=None)
     hx, hz = _flat(Hx), _flat(Hz)
     w = np.ascontiguousarray(words, dtype=np.uint32)
     shots = w.shape[0]
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     rc = lib.grand_decode_cc_packed(_p(hx), _p(hz), n_rows, n_cols, w.ctypes.data, kind, shots,
                                     ctypes.byref(cfg), results, ctypes.c_char(_type_byte(error_type)),
                                     os.fsencode(prob_file) if prob_file else None)
-    return rc, results_array(results)
+    _finish(rc, results, n_rows, n_cols)
+    return rc, _as_array(results)
 
 
 def decode_dem_packed(lib, variant, H_dem, L_dem, det_words, log_words, cfg, file=None):
@@ -297,9 +357,10 @@ def decode_dem_packed(lib, variant, H_dem, L_dem, det_words, log_words, cfg, fil
     d = np.ascontiguousarray(det_words, dtype=np.uint32)
     g = np.ascontiguousarray(log_words, dtype=np.uint32)
     shots = d.shape[0]
-    results = (GrandDecoderResult * shots)()
+    results = _new_results(shots)
     v = {"uniform": 0, "prob": 1, "ml": 2}[variant]
     rc = lib.grand_decode_cln_packed(_p(h), _p(l), n_rows, n_cols, nl, d.ctypes.data, g.ctypes.data,
                                      shots, ctypes.byref(cfg), results, v,
                                      os.fsencode(file) if file else None)
-    return rc, results_array(results)
+    _finish(rc, results, n_rows, n_cols, nl)
+    return rc, _as_array(results)
