@@ -8,6 +8,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <vector>
 #include <mutex>
 #include <string>
@@ -296,6 +297,7 @@ int decode_dem(int variant, const int *H, const int *L, int n, int m, int nl, co
       return GRAND_ERR_CUDA;
     }
     p.d_llr = (const float *)g.w->d_llr;
+    p.llr_min = *std::min_element(llr.begin(), llr.end());
   }
   p.input_kind = kInDetectors;
   p.W = W;

@@ -192,6 +192,8 @@ struct HotCode {
   const uint16_t *g_adj;
   const uint32_t *lcols;     // m * nlw
   const float *llr;          // m
+  float llr_min;             // the least of them
+  int pad_;                  // (whole 8-byte words)
 };
 
 // Immutable per-code tables plus the per-call search parameters.

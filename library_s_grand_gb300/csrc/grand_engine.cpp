@@ -5,6 +5,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -110,6 +111,7 @@ int grand_engine_add_dem(GrandEngine *e, const int *H, const int *L, int n, int 
       return GRAND_ERR_CUDA;
     }
     p.d_llr = d_llr;
+    p.llr_min = *std::min_element(llr.begin(), llr.end());
   }
   p.input_kind = kInDetectors;
   p.rec_len = n + nl;  // detectors followed by the true logical flips

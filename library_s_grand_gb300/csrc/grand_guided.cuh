@@ -499,9 +499,21 @@ __device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, G
       float psum = 0.0f;                // ML: sum of the pw smallest LLRs of the active set,
       unsigned long long plast = 0ull;  //   {LLR key, column} of the last of them, plus one
       int pw = 0;
+      float floor = 0.0f;  // ML: w times the code's least LLR, added up as the prefix sums are
 #pragma unroll 1
       for (int w = 1; __any_sync(kFull, go && w <= w_last); ++w) {
         bool act = go && w <= w_last;
+        // The bound: the search stops where the sum of the w smallest LLRs reaches the best
+        // cost.  That sum is no less than floor (FP32 addition is monotonic), which mostly
+        // settles it; only otherwise is it formed (65536 shots of the 720-mechanism DEM,
+        // drawing them included: 134 us, 139 with the sum formed for every weight).
+        if (MLK && ml) {
+          floor = __fadd_rn(floor, cd.llr_min);
+          if (act && wn.w && floor >= key_cost(wn.cost)) {
+            wn.w_done = w - 1;
+            go = act = false;
+          }
+        }
         if (MLK && __any_sync(kFull, act && ml && wn.w)) {
           // upstream's prefix sums: the w smallest LLRs, added in ascending order
 #pragma unroll 1

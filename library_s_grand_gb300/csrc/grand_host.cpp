@@ -385,6 +385,7 @@ DevCode make_devcode(const CodeTables &t, const CallParams &p) {
   d.pivrow = t.pivrow;
   d.lcols = t.lcols;
   d.llr = p.d_llr;
+  d.llr_min = p.llr_min;
   d.hcol = t.hcol;
   d.binary = t.binary;
   d.solo_keys = t.solo_keys;

@@ -56,6 +56,7 @@ struct CallParams {
   int mask_tam_upper[kMaxMasks] = {};
   int mask_order[kMaxMasks][3] = {};
   const float *d_llr = nullptr;   // device LLRs (ML)
+  float llr_min = 0.0f;            // and the least of them
   int rec_len = 0;                 // int32 entries per record (0: R, or m for errors)
   int packed = 0;                  // records are bit-packed words (rec_len then counts words)
 };

@@ -152,6 +152,7 @@ int main(int argc, char **argv) {
   std::copy(g.words.begin(), g.words.end(), base);
   set_guided(k.d, g, g.words.empty() ? nullptr : base);
   k.d.solo_branch = solo_branch_of(k.d);
+  k.d.llr_min = *std::min_element(k.llr.begin(), k.llr.end());
   const int N = k.N, m = k.m, nl = k.nl;
   const bool dem = k.family == kDem;
   const std::vector<int> rec = read_ints(dir + "/rec.bin", (size_t)N * k.rec_len);
