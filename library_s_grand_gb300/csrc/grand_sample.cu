@@ -51,10 +51,10 @@ __device__ __forceinline__ uint32_t flip_threshold(float p) {
 // into the lanes' syndrome (and logical) words, from which the entries are stored
 // coalesced; an error record's entries are the lanes' own comparisons.
 //
-// Bound by instruction issue, the generator's above all: 20 products of 32 x 32 -> 64 bits
-// and as many logic operations per four positions.  65536 shots of the 720-mechanism DEM:
-// 60 us (128 when every word was scanned for flips and the thresholds formed per shot;
-// 650 warp instructions a shot, 1700 then).
+// Bound by the generator's products, 20 of 32 x 32 -> 64 bits per four positions (with a
+// quarter of the other instructions taken out -- keys held in registers -- the time stayed
+// the same).  65536 shots of the 720-mechanism DEM: 60 us, 128 when every word was scanned for
+// flips and the thresholds formed per shot.
 template <bool ERRORS>
 __global__ void __launch_bounds__(256, 8) sample_kernel(DevCode cd, const float *p,
                                                      unsigned long long seed,
