@@ -22,20 +22,56 @@
 
 namespace grand {
 
-__host__ __device__ inline void philox4x32_10(uint32_t (&c)[4], uint32_t k0, uint32_t k1) {
+constexpr uint32_t kPhiloxM0 = 0xD2511F53u, kPhiloxM1 = 0xCD9E8D57u;
+constexpr uint32_t kPhiloxW0 = 0x9E3779B9u, kPhiloxW1 = 0xBB67AE85u;
+constexpr uint32_t kPhiloxTag = 0x47524E44u;
+
+__device__ __forceinline__ void mul_wide(uint32_t a, uint32_t b, uint32_t &hi, uint32_t &lo) {
+  const unsigned long long p = (unsigned long long)a * b;
+  hi = (uint32_t)(p >> 32);
+  lo = (uint32_t)p;
+}
+
+// The first two rounds multiply words that depend on the block alone (its number, then that
+// product's words) or on the shot alone, never on both: each half is formed once.
+struct PhiloxBlock {
+  uint32_t x0, x1, x2;  // after two rounds: word 0 and word 2 less the shot's part, word 1
+};
+struct PhiloxShot {
+  uint32_t x0, x2, x3;  // the shot's part of words 0 and 2, word 3
+};
+__device__ __forceinline__ PhiloxBlock philox_block(uint32_t block, uint32_t k1) {
+  PhiloxBlock r;
+  uint32_t hi;
+  mul_wide(kPhiloxM0, block, hi, r.x2);
+  mul_wide(kPhiloxM1, hi ^ kPhiloxTag ^ k1, r.x0, r.x1);
+  return r;
+}
+__device__ __forceinline__ PhiloxShot philox_shot(unsigned long long shot, uint32_t k0, uint32_t k1) {
+  PhiloxShot r;
+  uint32_t hi, lo;
+  mul_wide(kPhiloxM1, (uint32_t)(shot >> 32), hi, lo);
+  r.x0 = lo ^ (k0 + kPhiloxW0);
+  mul_wide(kPhiloxM0, hi ^ (uint32_t)shot ^ k0, hi, r.x3);
+  r.x2 = hi ^ (k1 + kPhiloxW1);
+  return r;
+}
+// The other eight rounds.
+__device__ __forceinline__ void philox_finish(const PhiloxBlock &b, const PhiloxShot &s,
+                                              const uint32_t (&keys)[16], uint32_t (&c)[4]) {
+  c[0] = b.x0 ^ s.x0;
+  c[1] = b.x1;
+  c[2] = b.x2 ^ s.x2;
+  c[3] = s.x3;
 #pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const unsigned long long p0 = 0xD2511F53ull * c[0];
-    const unsigned long long p1 = 0xCD9E8D57ull * c[2];
-    const uint32_t hi0 = (uint32_t)(p0 >> 32), lo0 = (uint32_t)p0;
-    const uint32_t hi1 = (uint32_t)(p1 >> 32), lo1 = (uint32_t)p1;
-    const uint32_t n0 = hi1 ^ c[1] ^ k0, n2 = hi0 ^ c[3] ^ k1;
-    c[0] = n0;
+  for (int r = 2; r < 10; ++r) {
+    uint32_t hi0, lo0, hi1, lo1;
+    mul_wide(kPhiloxM0, c[0], hi0, lo0);
+    mul_wide(kPhiloxM1, c[2], hi1, lo1);
+    c[0] = hi1 ^ c[1] ^ keys[2 * r - 4];
     c[1] = lo1;
-    c[2] = n2;
+    c[2] = hi0 ^ c[3] ^ keys[2 * r - 3];
     c[3] = lo0;
-    k0 += 0x9E3779B9u;
-    k1 += 0xBB67AE85u;
   }
 }
 
@@ -45,44 +81,71 @@ __device__ __forceinline__ uint32_t flip_threshold(float p) {
   return s >= 4294967295.0f ? 0xFFFFFFFFu : (s <= 0.0f ? 0u : (uint32_t)s);
 }
 
-// One warp per shot, a block's warps in strides of the grid.  The positions' thresholds are
-// formed once per block, in shared memory, a lane's four of a group side by side.  Flips
-// are rare: a group is asked once whether it has any, and their columns then go straight
-// into the lanes' syndrome (and logical) words, from which the entries are stored
+// One block per SM, its warps drawing the block's shots one at a time (a shared counter: in
+// fixed strides the warps that the scheduler prefers ended early, and the rest ran at 42 of
+// 64 warps).  The positions' thresholds and the blocks' halves of the first two rounds are
+// formed once per block, in shared memory, the thresholds of a lane's four positions side by
+// side.  Flips are rare: a group is asked once whether it has any, and their columns then
+// go straight into the lanes' syndrome (and logical) words, from which the entries are stored
 // coalesced; an error record's entries are the lanes' own comparisons.
 //
-// Bound by the generator's products, 20 of 32 x 32 -> 64 bits per four positions (with a
-// quarter of the other instructions taken out -- keys held in registers -- the time stayed
-// the same).  65536 shots of the 720-mechanism DEM: 60 us, 128 when every word was scanned for
-// flips and the thresholds formed per shot.
+// Bound by issue: the products (16 of 32 x 32 -> 64 bits per four positions) keep their pipe
+// 51 % busy, logic and comparisons theirs 59 %.  65536 shots of the 720-mechanism DEM: 50 us
+// (60 with all 20 products, 64 warps per SM in strides and keys formed in every group;
+// 2 x 1024, 3 x 512 or 2 x 768 threads per SM are 4 to 16 us slower, 1 x 512 as well).
+constexpr int kSampleThreads = 1024;
+
 template <bool ERRORS>
-__global__ void __launch_bounds__(256, 8) sample_kernel(DevCode cd, const float *p,
-                                                     unsigned long long seed,
-                                                     unsigned long long first_shot, int num_shots,
-                                                     int *records) {
+__global__ void __launch_bounds__(kSampleThreads, 1) sample_kernel(DevCode cd, const float *p,
+                                                                   unsigned long long seed,
+                                                                   unsigned long long first_shot, int num_shots,
+                                                                   int *records) {
+  __shared__ int s_next;
   extern __shared__ uint4 s_thr[];  // per group of 128 positions and lane: those of 32u + lane
   const int lane = threadIdx.x & 31;
   const int mpad = (cd.m + 127) & ~127;
   for (int j = threadIdx.x; j < mpad; j += blockDim.x)  // (zeros past the last position)
     reinterpret_cast<uint32_t *>(s_thr)[(j & ~127) + 4 * (j & 31) + ((j >> 5) & 3)] =
         j < cd.m ? flip_threshold(__ldg(p + j)) : 0u;
-  __syncthreads();
   const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-  const int nwarps = gridDim.x * 8;
+  uint32_t *s_blk = reinterpret_cast<uint32_t *>(s_thr + mpad / 4);  // the blocks' halves, by word
+  const int nblk = mpad / 4;
+  for (int j = threadIdx.x; j < nblk; j += blockDim.x) {
+    const PhiloxBlock h = philox_block((uint32_t)j, k1);
+    s_blk[j] = h.x0;
+    s_blk[nblk + j] = h.x1;
+    s_blk[2 * nblk + j] = h.x2;
+  }
+  uint32_t keys[16];  // of rounds 3 .. 10 (held: formed anew they were a fifth of the instructions)
+#pragma unroll
+  for (int r = 2; r < 10; ++r) {
+    keys[2 * r - 4] = k0 + (uint32_t)r * kPhiloxW0;
+    keys[2 * r - 3] = k1 + (uint32_t)r * kPhiloxW1;
+    asm volatile("" : "+r"(keys[2 * r - 4]), "+r"(keys[2 * r - 3]));
+  }
+  // the block's shots, drawn by its warps
+  const int last = (int)((long long)num_shots * (blockIdx.x + 1) / gridDim.x);
+  if (threadIdx.x == 0) s_next = (int)((long long)num_shots * blockIdx.x / gridDim.x);
+  __syncthreads();
   const bool dem = cd.family == kDem;
   const int nw = cd.nw, nlw = dem ? cd.nlw : 0;
 #pragma unroll 1
-  for (int i = blockIdx.x * 8 + (threadIdx.x >> 5); i < num_shots; i += nwarps) {
+  for (;;) {
+    int i = 0;
+    if (lane == 0) i = atomicAdd(&s_next, 1);
+    i = __shfl_sync(kFull, i, 0);
+    if (i >= last) break;
     const unsigned long long shot = first_shot + (unsigned long long)i;
     int *rec = records + (size_t)i * cd.rec_len;
+    const PhiloxShot half = philox_shot(shot, k0, k1);
     uint32_t s_lane = 0u, l_lane = 0u;  // syndrome / detector word `lane`, logical word `lane`
     // flips: 128 positions per group, four words of one block per lane
 #pragma unroll 1
     for (int j0 = 0; j0 < mpad; j0 += 128) {
-      uint32_t c[4] = {(uint32_t)(j0 / 4 + lane), (uint32_t)shot, (uint32_t)(shot >> 32),
-                       0x47524E44u};
-      philox4x32_10(c, k0, k1);
-      const uint4 thr = s_thr[j0 / 4 + lane];
+      const int blk = j0 / 4 + lane;
+      uint32_t c[4];
+      philox_finish(PhiloxBlock{s_blk[blk], s_blk[nblk + blk], s_blk[2 * nblk + blk]}, half, keys, c);
+      const uint4 thr = s_thr[blk];
       const bool f[4] = {c[0] < thr.x, c[1] < thr.y, c[2] < thr.z, c[3] < thr.w};
       if constexpr (ERRORS) {
 #pragma unroll
@@ -121,13 +184,14 @@ cudaError_t launch_sample(const DevCode &cd, const float *d_p, unsigned long lon
                           unsigned long long first_shot, int num_shots, int *d_records,
                           int sm_count, cudaStream_t s) {
   if (num_shots <= 0) return cudaSuccess;
-  int grid = (num_shots + 7) / 8;
-  if (grid > sm_count * 8) grid = sm_count * 8;
-  const size_t smem = sizeof(uint32_t) * ((cd.m + 127) & ~127);  // at most 16 KB
+  int grid = num_shots;
+  if (grid > sm_count) grid = sm_count;
+  const int mpad = (cd.m + 127) & ~127;
+  const size_t smem = sizeof(uint32_t) * (mpad + 3 * (mpad / 4));  // at most 28 KB
   if (cd.input_kind == kInErrors)
-    sample_kernel<true><<<grid, 256, smem, s>>>(cd, d_p, seed, first_shot, num_shots, d_records);
+    sample_kernel<true><<<grid, kSampleThreads, smem, s>>>(cd, d_p, seed, first_shot, num_shots, d_records);
   else
-    sample_kernel<false><<<grid, 256, smem, s>>>(cd, d_p, seed, first_shot, num_shots, d_records);
+    sample_kernel<false><<<grid, kSampleThreads, smem, s>>>(cd, d_p, seed, first_shot, num_shots, d_records);
   return cudaGetLastError();
 }
 
