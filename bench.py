@@ -9,18 +9,19 @@ synthetic data (numpy PCG64); no dataset exists for this workload.
 
 Reported (one JSON line, rank 0):
   value      shots/s of the persistent batched decoder, records resident in HBM,
-             graph-replayed decode launches (one persistent kernel per batch), L2
+             graph-replayed decode launches (one kernel per batch: chunk_kernel), L2
              flushed between steps;
   e2e        shots/s through the upstream-compatible C ABI (grand_decode_prob_cc)
              from host buffers, the records' trip to the GPU and the results' trip
              back included (read and written in place over NVLink-C2C where the
              GPU can access pageable memory, else copied);
-  roofline   the decode kernel on the stress input the integer roofline is
-             defined on (random syndromes, W = 4, exhaustive enumeration):
-             candidates at 1.5 integer ops each against the measured lop3 issue
-             rate, and beside it the prefix probes the lookup search executes
-             against the shared-memory bound of two words per probe;
-  roofline_dem  the same conventions on the capped DEM stress (random detectors
+  roofline   the kernel on random syndromes (W = 4; nothing matches, so upstream
+             enumerates every candidate): warp instructions issued against the
+             SMs' issue rate, and beside it the candidates excluded per second
+             in the conventions of an enumerating search (1.5 integer ops a
+             candidate against the measured lop3 rate), above 1 where the guided
+             search excludes candidates without forming them;
+  roofline_dem  the same figures on the capped DEM stress (random detectors
              of the 120 x 720 DEM, W = 3, cap 64), at the default and at a tuned
              light budget;
   cpu_baseline  the upstream CPU search algorithm (its C restatement in oracle/,
@@ -445,9 +446,9 @@ def run_ours(args):
     return out
 
 
-# DRAM bytes (read + write) of one decode_kernel launch on the headline batch, from an ncu
-# --set full capture (profiles/decode_kernel_prob_cc_bb144_16384.md).
-HEADLINE_TRAFFIC = 9.694976e6 + 768.0
+# DRAM bytes (read + write) of one chunk_kernel launch on the headline batch, from an ncu
+# --set full capture (profiles/chunk_kernel.md).
+HEADLINE_TRAFFIC = 9.527808e6
 
 
 def hbm_peak():
@@ -461,12 +462,12 @@ def hbm_peak():
 
 
 def hbm_streaming(code, dec_ms):
-    """Record streaming of the decode kernel on the headline batch: int32 error records in
+    """Record streaming of the chunk kernel on the headline batch: int32 error records in
     (4m bytes per shot) and 72-byte results out, per launch, over the kernel's event time."""
     peak, src = hbm_peak()
     per_shot = 4 * code.m + 72
     gbs = SHOTS * per_shot / (dec_ms * 1e-3) / 1e9
-    return {"kernel": "decode_kernel", "achieved": gbs, "peak": peak, "unit": "GB/s",
+    return {"kernel": "chunk_kernel", "achieved": gbs, "peak": peak, "unit": "GB/s",
             "frac": gbs / peak, "peak_source": src + " copy bandwidth (MEASURED_PEAKS.json)",
             "algorithmic_bytes_per_launch": SHOTS * per_shot, "traffic": HEADLINE_TRAFFIC,
             "traffic_unit": "bytes per launch (ncu)", "decode_ms": dec_ms,
@@ -474,15 +475,20 @@ def hbm_streaming(code, dec_ms):
 
 
 STRESS_SHOTS = 192
-SKETCH_OPS_PER_CANDIDATE = 1.5
-# DRAM bytes (read + write) of one decode_kernel launch on the 192 stress shots, from an
-# ncu --set full capture (profiles/decode_kernel_stress_bb144_w4.md), per shot.
-STRESS_TRAFFIC_PER_SHOT = (317184.0 + 6656.0) / 192
-# The lookup search's bound per prefix probe: two shared-memory words (the last
-# element's sketch and one filter word) at 32 words per SM per clock.
-PROBE_WORDS = 2
-SMEM_WORDS_PER_SM_CLOCK = 32
+SKETCH_OPS_PER_CANDIDATE = 1.5  # an enumerating search by column sketches: XOR + half a 3-way min
+# One chunk_kernel launch on the 192 stress shots and on the 8192 DEM stress shots, from ncu
+# --set full captures (profiles/chunk_kernel.md): DRAM bytes and warp instructions.
+STRESS_TRAFFIC = 142080.0
+STRESS_INSTRUCTIONS = 556033
+DEM_STRESS_INSTRUCTIONS = 10054839
+ISSUE_PER_SM_CLOCK = 4  # one warp instruction per scheduler
 SM_CLOCK_HZ = 2.07e9  # the GB300's maximum SM clock (the runs' median clock, bench `clocks`)
+
+
+def issue_peak(torch, dev):
+    """Warp instructions per second the SMs can issue."""
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    return sms * ISSUE_PER_SM_CLOCK * SM_CLOCK_HZ
 
 
 def stress_case(torch, lib, dev, n=STRESS_SHOTS):
@@ -499,22 +505,19 @@ def stress_case(torch, lib, dev, n=STRESS_SHOTS):
 
 
 def stress_roofline(torch, lib, dev, sp):
-    """Decode kernel on exhaustive random-syndrome shots of [[144,12,12]], W=4.
+    """Chunk kernel on random-syndrome shots of [[144,12,12]], W=4: nothing matches, so
+    upstream enumerates every candidate of three threshold iterations.
 
-    Candidate convention (comparable across versions of the search): a candidate
-    tested by a sketch scan costs one XOR (its last column's sketch against the
-    prefix sketch) and half a 3-way minimum, 1.5 integer ops whatever R, against
-    the lop3 issue rate measured on this GPU; the word-compare count ceil(R/32)+1
-    and the fixed count (w+1)*ceil(R/32) are reported beside it.  The lookup
-    search tests a prefix's candidates with one probe, so it also gets a probe
-    convention: prefix probes per second against the shared-memory bound of two
-    words per probe (the fraction of the machine the search itself uses)."""
+    `frac` is the share of the SMs' issue slots used (48 blocks of four warps on 152 SMs:
+    the launch is one shot's chain of dependent instructions long).  The guided search
+    excludes most candidates without forming them, so candidates per second in the
+    conventions of an enumerating search (1.5, ceil(R/32)+1 or (w+1)*ceil(R/32) integer
+    ops per candidate against the measured lop3 rate) exceed that machine's peak; they
+    compare the work upstream would do, not how busy the ALUs are."""
     from library_s_grand_gb300 import capi
     n = STRESS_SHOTS
     code, syn, eng, d_rec, d_res = stress_case(torch, lib, dev, n)
-    cands, ops_fixed, prefixes = stress_ops(code.hz, syn, 4)
-    sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    probe_peak = sms * SMEM_WORDS_PER_SM_CLOCK / PROBE_WORDS * SM_CLOCK_HZ
+    cands, ops_fixed, _ = stress_ops(code.hz, syn, 4)
     words = math.ceil(code.n / 32)
     times = []
     for rep in range(4):
@@ -528,25 +531,26 @@ def stress_roofline(torch, lib, dev, sp):
     search_ms = float(np.median(times[1:]))
     peak = eng.int_peak()
     rate = cands / (search_ms * 1e-3)
-    achieved = rate * SKETCH_OPS_PER_CANDIDATE
-    return {"bound": "int_alu", "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "Gop/s",
-            "frac": achieved / peak, "traffic": STRESS_TRAFFIC_PER_SHOT * n,
+    achieved = STRESS_INSTRUCTIONS / (search_ms * 1e-3)
+    issue = issue_peak(torch, dev)
+    return {"bound": "issue", "achieved": achieved / 1e9, "peak": issue / 1e9,
+            "unit": "G warp instructions/s", "frac": achieved / issue, "traffic": STRESS_TRAFFIC,
             "traffic_unit": "bytes per launch (ncu capture of the same 192 shots)",
-            "kernel": "decode_kernel",
+            "kernel": "chunk_kernel",
             "workload": f"{n} random-syndrome shots of BB[[144,12,12]], W=4, exhaustive "
                         f"({cands} candidates, 3 threshold iterations)",
-            "ops_per_candidate": "1.5 (sketch XOR + half a 3-way min)",
+            "instructions": STRESS_INSTRUCTIONS,
+            "instructions_source": "smsp__inst_executed.sum (ncu capture of the same shots)",
             "search_ms": search_ms, "candidates_per_s": rate,
+            "frac_sketch_convention": rate * SKETCH_OPS_PER_CANDIDATE / peak,
+            "sketch_convention": "1.5 ops per candidate (sketch XOR + half a 3-way min); above 1: "
+                                 "candidates excluded without being formed",
             "frac_word_convention": rate * (words + 1) / peak,
             "word_convention": f"ceil(R/32)+1 = {words + 1} ops per candidate (XOR-OR words + min)",
             "frac_fixed_convention": ops_fixed / (search_ms * 1e-3) / peak,
             "fixed_convention": "(w+1)*ceil(R/32) ops per candidate",
-            "peak_source": "lop3.b32 issue rate measured on this GPU (grand_measure_int_peak)",
-            "prefix_probes": prefixes, "probes_per_s": prefixes / (search_ms * 1e-3),
-            "probe_peak_per_s": probe_peak,
-            "frac_probe_convention": prefixes / (search_ms * 1e-3) / probe_peak,
-            "probe_convention": "one prefix probe = 2 shared-memory words (sketch, filter word); "
-                                "peak = SMs x 32 words/clock / 2 x 2.07 GHz"}
+            "peak_source": "issue: SMs x 4 schedulers x 2.07 GHz; conventions: lop3.b32 issue rate "
+                           "measured on this GPU (grand_measure_int_peak)"}
 
 
 STRESS_DEM_SHOTS = 8192
@@ -566,14 +570,11 @@ def dem_stress_case(torch, lib, dev, n=STRESS_DEM_SHOTS):
 
 
 def dem_stress_roofline(torch, lib, dev, sp):
-    """Decode kernel on the capped DEM stress, in the conventions of stress_roofline.  Each
-    shot's search is small (at most 43,744 candidates per iteration), so the figure covers
-    the whole per-shot pipeline (record, counts, planning, Job publication) as much as
-    the scan."""
+    """Chunk kernel on the capped DEM stress, with the figures of stress_roofline."""
     from library_s_grand_gb300 import autotune, capi
     n = STRESS_DEM_SHOTS
     wl, eng, d_rec, d_res = dem_stress_case(torch, lib, dev, n)
-    cands, ops_fixed, prefixes = dem_stress_ops(wl.dem.h, wl.detectors, wl.W, wl.cap)
+    cands, ops_fixed, _ = dem_stress_ops(wl.dem.h, wl.detectors, wl.W, wl.cap)
 
     def timed():
         times = []
@@ -588,8 +589,8 @@ def dem_stress_roofline(torch, lib, dev, sp):
         return float(np.median(times[1:])), eng.launch_stats(sp)
 
     search_ms, stats = timed()
-    # the same shots with the light budget tuned for them (larger budgets keep these
-    # small searches in the warp that triages the shot instead of publishing Jobs)
+    # the same shots with the light budget tuned for them (the guided search only counts
+    # the shots past it)
     best, table = autotune.tune(eng, "dem-stress", n, d_rec.data_ptr(), d_res.data_ptr(), sp,
                                 use_cache=False, grid=[(l, 4, 0) for l in (10, 12, 14, 16)])
     tuned_ms, tuned_stats = timed()
@@ -597,22 +598,25 @@ def dem_stress_roofline(torch, lib, dev, sp):
     peak = eng.int_peak()
     rate = cands / (search_ms * 1e-3)
     words = math.ceil(wl.dem.n / 32)
-    return {"bound": "int_alu", "achieved": rate * SKETCH_OPS_PER_CANDIDATE / 1e9,
-            "peak": peak / 1e9, "unit": "Gop/s", "frac": rate * SKETCH_OPS_PER_CANDIDATE / peak,
-            "kernel": "decode_kernel",
+    issue = issue_peak(torch, dev)
+    achieved = DEM_STRESS_INSTRUCTIONS / (search_ms * 1e-3)
+    return {"bound": "issue", "achieved": achieved / 1e9, "peak": issue / 1e9,
+            "unit": "G warp instructions/s", "frac": achieved / issue, "kernel": "chunk_kernel",
+            "instructions": DEM_STRESS_INSTRUCTIONS,
+            "instructions_source": "smsp__inst_executed.sum (ncu capture of the same shots)",
             "workload": f"{n} random-detector shots (Bernoulli 0.36) of the 120 x 720 DEM, "
                         f"grand_decode_cln, W=3, cap 64, exhaustive ({cands} candidates)",
-            "ops_per_candidate": "1.5 (sketch XOR + half a 3-way min)",
             "search_ms": search_ms, "candidates_per_s": rate, "shots_per_s": n / (search_ms * 1e-3),
-            "jobs": int(stats[2]), "lookup_tiles": int(stats[3]),
+            "past_light_budget": int(stats[2]), "lookup_tiles": int(stats[3]),
+            "frac_sketch_convention": rate * SKETCH_OPS_PER_CANDIDATE / peak,
             "frac_word_convention": rate * (words + 1) / peak,
             "frac_fixed_convention": ops_fixed / (search_ms * 1e-3) / peak,
-            "prefix_probes": prefixes, "probes_per_s": prefixes / (search_ms * 1e-3),
-            "peak_source": "lop3.b32 issue rate measured on this GPU (grand_measure_int_peak)",
+            "peak_source": "issue: SMs x 4 schedulers x 2.07 GHz; conventions: lop3.b32 issue rate "
+                           "measured on this GPU (grand_measure_int_peak)",
             "tuned": {"light_log2": best[0], "search_ms": tuned_ms,
                       "candidates_per_s": cands / (tuned_ms * 1e-3),
-                      "frac": cands / (tuned_ms * 1e-3) * SKETCH_OPS_PER_CANDIDATE / peak,
-                      "jobs": int(tuned_stats[2]), "table_ms": table}}
+                      "frac": DEM_STRESS_INSTRUCTIONS / (tuned_ms * 1e-3) / issue,
+                      "past_light_budget": int(tuned_stats[2]), "table_ms": table}}
 
 
 def _time_device(torch, eng, n, d_rec, d_res, sp, flush, steps, warmup, d_sc=0, d_off=0):
@@ -880,7 +884,7 @@ def run_case(args):
         if eng.sync_status(sp) != 0:
             raise RuntimeError("status error")
         rst, dec = eng.kernel_times(sp)
-        print(f"case {args.case}: decode kernel {dec:.4f} ms (control reset {rst:.4f} ms)", flush=True)
+        print(f"case {args.case}: kernels {dec:.4f} ms (control reset {rst:.4f} ms)", flush=True)
 
 
 def run_reference(args):

@@ -4,10 +4,11 @@
  * No upstream counterpart: upstream decodes one code per call with a serial
  * host loop over shots (grand_decoder.cu:885, 1199, 1466, 1762, 2073).  An
  * engine keeps any number of registered codes resident on the GPU and decodes
- * batches whose shots may use different codes in one persistent launch (its
- * warps classify shots, triage the hard ones and search the heaviest, work
- * stealing from each other), optionally replayed from a captured CUDA graph.  Results are identical to the five grand_decode_* calls on the
- * same shots.
+ * batches whose shots may use different codes in one launch (a kernel whose
+ * warps classify shots 32 at a time and search the open ones; codes that it does
+ * not take go to a persistent kernel after it), optionally replayed from a
+ * captured CUDA graph.  Results are identical to the five grand_decode_* calls on
+ * the same shots.
  *
  * Shot records are int32 0/1 rows: the syndrome (n entries) or the error (m
  * entries) for CSS codes, as chosen at registration; the detectors followed by
@@ -95,13 +96,15 @@ int grand_engine_decode_plain(GrandEngine *engine, int num_shots, const int *sho
  * light_log2: largest per-shot search (2^x candidates) finished by the warp
  * that triages the shot (larger ones become Jobs that every warp searches);
  * tile_k: prefixes per lane per search tile; search_ctas_per_sm: resident CTAs
- * per SM of the persistent decode kernel (0 = occupancy maximum). */
+ * per SM of the persistent decode kernel (0 = occupancy maximum).  They shape
+ * that kernel only, which batches whose codes all have a guided search do not
+ * need; there light_log2 only sets which shots grand_engine_launch_stats counts. */
 int grand_engine_set_tuning(GrandEngine *engine, int light_log2, int tile_k,
                             int search_ctas_per_sm);
 
 /* Device times of the last non-graph device decode on `stream` (valid after
  * grand_engine_sync_status): *reset_ms the control-word reset before the
- * launch, *decode_ms the decode kernel. */
+ * launch (where the batch needs one), *decode_ms the decoding kernel or kernels. */
 int grand_engine_kernel_times(GrandEngine *engine, void *stream, float *reset_ms,
                               float *decode_ms);
 
@@ -112,7 +115,8 @@ int grand_engine_kernel_times(GrandEngine *engine, void *stream, float *reset_ms
  * unless the guided search finished it), out[3] search tiles of the Jobs,
  * out[4] scratch words staged for them.  With GRAND_PROFILE=1 in the
  * environment when the engine was created, out[5..8] are the warp-nanoseconds
- * the decode kernel's warps spent classifying, on the per-shot path, on search
+ * the kernels' warps spent classifying (the chunk kernel's whole time counts as
+ * that), on the per-shot path, on search
  * tiles and waiting for work, out[9..12] when the last of each ended (ns after
  * the first warp started; -1: none), out[13] the number of work steps and
  * out[14..23] a finer split of the warp-nanoseconds: classification (records
@@ -127,7 +131,7 @@ int grand_engine_kernel_times(GrandEngine *engine, void *stream, float *reset_ms
 int grand_engine_launch_stats(GrandEngine *engine, void *stream, long long *out);
 
 /* Times of the last host-buffer decode (grand_engine_decode / _decode_plain):
- * copies in, the control-word reset(s), the decode kernel(s) and copies out,
+ * copies in, the control-word reset(s), the decoding kernel(s) and copies out,
  * from CUDA events on the call's stream.  With zero-copy (records read and results
  * written in place over NVLink-C2C) the copy times are ~0 and the kernels'
  * times include reading host memory.  Any pointer may be NULL. */

@@ -8,8 +8,10 @@ Three knobs shape a launch and none of them changes a result:
                       and every weight when R > 256);
   search_ctas_per_sm  resident CTAs per SM of the persistent decode kernel (0:
                       the occupancy maximum).
+They act on the persistent decode kernel; a batch whose codes all have a guided search runs
+without it, and every setting takes the same time there.
 The tuner times a workload's device decode (CUDA events around the control
-reset and the decode kernel) over a small grid, keeps the fastest setting on the engine and
+reset and the kernels) over a small grid, keeps the fastest setting on the engine and
 caches it in a JSON file keyed by the workload's name and the GPU.
 """
 from __future__ import annotations

@@ -1,5 +1,5 @@
-// grand_decode.cuh -- the persistent decode kernel (sm_103a): one launch per batch, for the
-// codes and shots the guided search does not take (grand_chunk.cuh).
+// grand_decode.cuh -- the persistent decode kernel (sm_103a), for the codes and shots the
+// guided search does not take (grand_front.cuh): one launch per batch that has any.
 //
 // Every warp of the grid loops over whatever work the batch has left, in this
 // order of preference:

@@ -1,4 +1,4 @@
-// grand_decode_ml.cu -- the decode kernel built with the ML (cost-ordered)
+// grand_decode_ml.cu -- the chunk and decode kernels built with the ML (cost-ordered)
 // search paths, for batches with an ML code.
 #include "grand_decode.cuh"
 #include "grand_front.cuh"

@@ -1,4 +1,4 @@
-// grand_decode_plain.cu -- the decode kernel built without the ML paths (smaller
+// grand_decode_plain.cu -- the chunk and decode kernels built without the ML paths (smaller
 // code, fewer registers), for batches without an ML code; and the launcher that
 // picks the build.
 #include "grand_decode.cuh"

@@ -163,7 +163,7 @@ struct Tuning {
   int fast = 1;              // settle shots 32 at a time before the per-shot path (GRAND_FAST)
   int zero_copy = 1;         // read records / write results in the caller's host memory
                              // when the device can access pageable memory (GRAND_ZERO_COPY)
-  int profile = 0;           // the decode kernel records per-phase times (GRAND_PROFILE)
+  int profile = 0;           // the kernels record per-phase times (GRAND_PROFILE)
 };
 Tuning &tuning();  // process defaults (GRAND_LIGHT_LOG2, GRAND_TILE_K, GRAND_SEARCH_GRID_MULT)
 
@@ -175,7 +175,7 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
 // codes, b.num_shots and b.shot_map.
 void plan_batch(DevBatch &b, const DevCode *codes, int ncodes, int sm_count, const Tuning &tn);
 
-// Enqueue one decoding launch (control-word reset, decode kernel) on s.
+// Enqueue one batch on s: the control-word reset and the kernels it needs.
 cudaError_t launch_pipeline(const Context *ctx, const DevBatch &b, const Tuning &tn,
                             cudaStream_t s, cudaEvent_t mid = nullptr);
 

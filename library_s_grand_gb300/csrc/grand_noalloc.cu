@@ -8,9 +8,12 @@
 // cudaMalloc on first use (and grow them); this one keeps everything it needs
 // beyond the caller's inputs and outputs in one fixed, file-scope device array.
 //
-// The batch runs through the same decode kernel as the other entry points.  Only the place their scratch lives differs: the binomial table, the
-// packed columns, the code descriptor, the counters, the job table and the
-// scratch arena are carved out of g_noalloc_scratch.
+// One kernel builds the code's tables on every call (grand_prep.cuh), and the batch then runs
+// through the same kernels as the other entry points': the chunk kernel, then the decode
+// kernel, which leaves at once when no shot is left to it.  Only the place their scratch
+// lives differs: the binomial table, the packed columns and the guided search's tables, the
+// code descriptor, the counters, the job table and the scratch arena are carved out of
+// g_noalloc_scratch.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>

@@ -9,10 +9,11 @@
 //     (max_shots_per_batch, and the search scratch expected from the recent
 //     batches' scratch per shot within 3/4 of the slot's arena), packs their
 //     offsets (records are read in place where the GPU can reach pageable
-//     memory, copied through pinned staging otherwise), and enqueues copy-in, counter
-//     reset, the decode kernel and copy-out on the slot's stream; each slot's
-//     persistent kernel gets 1/slots of the resident blocks, so all slots'
-//     kernels are on the GPU at once.
+//     memory, copied through pinned staging otherwise), and enqueues the batch on the
+//     slot's stream: one launch that reads and writes the slot's pinned memory where the
+//     chunk kernel decodes the batch alone, otherwise copy-in, counter reset, the kernels
+//     and copy-out; there each slot's persistent kernel gets 1/slots of the resident
+//     blocks, so all slots' kernels are on the GPU at once.
 // Requests arriving while slots run simply wait for the next free slot, so the
 // GPU always has up to `slots` micro-batches in flight.
 #include "grand_server.h"
@@ -192,7 +193,7 @@ cudaError_t start_slot(GrandServer *S, SrvSlot *sl) {
   b.fast = e->tn.fast;
   b.light_max_log2 = e->tn.light_max_log2;
   b.tile_k = e->tn.tile_k;
-  // each slot's persistent grid takes its share of the resident blocks, so the
+  // each slot's decode kernel takes its share of the resident blocks, so the
   // slots' kernels are resident together and their batches overlap on the GPU
   Tuning tn = e->tn;
   const int share = std::max(1, e->ctx->decode_bps / std::max(1, (int)S->slots.size()));
