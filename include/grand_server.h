@@ -35,8 +35,9 @@ typedef struct GrandServer GrandServer;
 /* slots: micro-batches in flight at once; max_shots_per_batch: shots a slot
  * holds; hbm_budget_bytes: device memory the slots may use (0 = 1/4 of the free
  * memory).  Fewer slots than asked are created when the budget is smaller; the
- * call fails when not even one fits.  The engine's codes must be registered
- * before the server is created and the engine must outlive the server. */
+ * call fails when not even one fits.  At least one code must be registered before the
+ * server is created (codes registered later may be used from then on), and the
+ * engine must outlive the server. */
 int grand_server_create(GrandEngine *engine, int slots, int max_shots_per_batch,
                         size_t hbm_budget_bytes, GrandServer **server);
 void grand_server_destroy(GrandServer *server);

@@ -119,6 +119,11 @@ void CUDART_CB slot_done(void *p) {
 // Called without the server lock; the slot is owned by the dispatcher.
 cudaError_t start_slot(GrandServer *S, SrvSlot *sl) {
   GrandEngine *e = S->eng;
+  // The launch reads the descriptors of every registered code, whatever its shots use: those
+  // registered since the last upload go to the device first, and none is added (nor the
+  // device copy moved) until the batch is in the stream.
+  std::lock_guard<std::mutex> elk(e->mu);
+  if (upload_codes(e)) return cudaErrorUnknown;
   // Where the GPU can read pageable host memory (NVLink-C2C on GB300) the kernel
   // reads every request's records in place: offsets are taken from the lowest
   // record address of the batch, and no record is copied on the host or to the
@@ -220,11 +225,14 @@ void finish_slot(GrandServer *S, SrvSlot *sl, int rc) {
     Workspace *ws = S->eng->ctx->acquire();
     BatchRequest req;
     req.num_shots = sl->nshots;
-    req.codes = S->eng->codes;
     req.h_in = sl->in_base ? sl->in_base : sl->h_rec;
     long long extent = 0;
-    for (int i = 0; i < sl->nshots; ++i)
-      extent = std::max(extent, sl->h_off[i] + (long long)S->eng->rec_len[sl->h_code[i]]);
+    {
+      std::lock_guard<std::mutex> elk(S->eng->mu);
+      req.codes = S->eng->codes;
+      for (int i = 0; i < sl->nshots; ++i)
+        extent = std::max(extent, sl->h_off[i] + (long long)S->eng->rec_len[sl->h_code[i]]);
+    }
     req.in_ints = (size_t)extent;
     req.h_off = sl->h_off;
     req.h_shot_code = sl->h_code;
@@ -426,10 +434,16 @@ int grand_server_info(GrandServer *S, int *slots, size_t *device_bytes) {
 int grand_server_submit(GrandServer *S, int n, const int *shot_code, const int *records,
                         GrandDecoderResult *results, unsigned long long *request_id) {
   if (!S || n <= 0 || n > S->max_shots || !records || !results) return GRAND_ERR_INVALID;
-  const int ncodes = (int)S->eng->rec_len.size();
-  if (shot_code)
-    for (int i = 0; i < n; ++i)
-      if (shot_code[i] < 0 || shot_code[i] >= ncodes) return GRAND_ERR_INVALID;
+  {
+    std::lock_guard<std::mutex> elk(S->eng->mu);
+    const std::vector<int> &len = S->eng->rec_len;
+    // a slot's staging holds records of the codes registered when the server was created
+    const bool staged = !(S->eng->tn.zero_copy && S->eng->ctx->pageable_access);
+    for (int i = 0; shot_code && i < n; ++i)
+      if (shot_code[i] < 0 || shot_code[i] >= (int)len.size() ||
+          (staged && len[shot_code[i]] > S->max_rec))
+        return GRAND_ERR_INVALID;
+  }
   auto r = std::make_shared<SrvRequest>();
   r->n = n;
   r->shot_code = shot_code;
@@ -468,14 +482,19 @@ int grand_server_replay(GrandServer *S, int nreq, const double *arrival_s, const
   if (!S || nreq < 0 || (nreq > 0 && (!arrival_s || !num_shots || !records || !results)))
     return GRAND_ERR_INVALID;
   std::vector<long long> shot0(nreq + 1, 0), rec0(nreq + 1, 0);
+  std::vector<int> rec_len;
+  {
+    std::lock_guard<std::mutex> elk(S->eng->mu);
+    rec_len = S->eng->rec_len;
+  }
   for (int i = 0; i < nreq; ++i) {
     if (num_shots[i] <= 0 || num_shots[i] > S->max_shots) return GRAND_ERR_INVALID;
     shot0[i + 1] = shot0[i] + num_shots[i];
     long long ints = 0;
     for (int j = 0; j < num_shots[i]; ++j) {
       const int c = shot_code ? shot_code[shot0[i] + j] : 0;
-      if (c < 0 || c >= (int)S->eng->rec_len.size()) return GRAND_ERR_INVALID;
-      ints += S->eng->rec_len[c];
+      if (c < 0 || c >= (int)rec_len.size()) return GRAND_ERR_INVALID;
+      ints += rec_len[c];
     }
     rec0[i + 1] = rec0[i] + ints;
   }
