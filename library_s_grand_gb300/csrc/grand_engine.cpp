@@ -161,8 +161,7 @@ int grand_engine_set_tuning(GrandEngine *e, int light_log2, int tile_k, int sear
   e->tn.light_max_log2 = light_log2;
   e->tn.tile_k = tile_k;
   e->tn.search_grid_mult = search_ctas_per_sm;
-  for (auto &g : e->graphs) cudaGraphExecDestroy(g.second);
-  e->graphs.clear();
+  drop_graphs(e, nullptr);
   return 0;
 }
 
@@ -240,11 +239,16 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   }
   const int max_jobs = num_shots;
   const size_t scratch_words = 64ull << 20;
+  const void *const held[] = {slot->d_jobs, slot->d_scratch, slot->d_small, slot->d_deferred};
   cudaError_t r = ensure_zeroed(&slot->d_jobs, &slot->cap_jobs, sizeof(Job) * (size_t)max_jobs);
   if (r == cudaSuccess) r = ensure(&slot->d_scratch, &slot->cap_scratch, scratch_words * 4);
   if (r == cudaSuccess) r = ensure_zeroed(&slot->d_small, &slot->cap_small, kCtlAllocBytes);
   if (r == cudaSuccess)
     r = ensure_zeroed(&slot->d_deferred, &slot->cap_deferred, shot_buffer_bytes(num_shots));
+  // launches captured on buffers that have moved would write where they were
+  if (held[0] != slot->d_jobs || held[1] != slot->d_scratch || held[2] != slot->d_small ||
+      held[3] != slot->d_deferred)
+    drop_graphs(e, slot);
   if (r != cudaSuccess) {
     set_error("grand: device workspace allocation failed (%s)", cudaGetErrorString(r));
     return GRAND_ERR_CUDA;
@@ -284,12 +288,10 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
     slot->timed = true;
   } else {
     slot->timed = false;
-    GraphKey key{num_shots, d_shot_code, d_offsets, d_records, d_results};
+    GraphKey key{slot, num_shots, d_shot_code, d_offsets, d_records, d_results};
     auto it = e->graphs.find(key);
     cudaGraphExec_t exec = nullptr;
-    if (it != e->graphs.end() && it->first.a == key.a) {
-      exec = it->second;
-    }
+    if (it != e->graphs.end()) exec = it->second;
     if (!exec) {
       cudaStream_t cs;
       r = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);

@@ -30,11 +30,14 @@ struct EngineSlot {
   }
 };
 
+// A captured launch: it holds the addresses of its stream's workspace and of the caller's
+// buffers.
 struct GraphKey {
+  const EngineSlot *slot;
   int n;
   const void *a, *b, *c, *d;
   bool operator<(const GraphKey &o) const {
-    return std::tie(n, a, b, c, d) < std::tie(o.n, o.a, o.b, o.c, o.d);
+    return std::tie(slot, n, a, b, c, d) < std::tie(o.slot, o.n, o.a, o.b, o.c, o.d);
   }
 };
 
@@ -64,12 +67,23 @@ struct GrandEngine {
 
 namespace grand {
 
+// Drop the launches captured on a workspace (nullptr: on all; caller holds e->mu).
+inline void drop_graphs(GrandEngine *e, const EngineSlot *slot) {
+  for (auto it = e->graphs.begin(); it != e->graphs.end();) {
+    if (slot && it->first.slot != slot) {
+      ++it;
+      continue;
+    }
+    cudaGraphExecDestroy(it->second);
+    it = e->graphs.erase(it);
+  }
+}
+
 // Upload the engine's code descriptors when they changed (caller holds e->mu).
 inline int upload_codes(GrandEngine *e) {
   if (!e->dirty) return 0;
   // launches captured for the codes before hold their descriptors' address and plan
-  for (auto &g : e->graphs) cudaGraphExecDestroy(g.second);
-  e->graphs.clear();
+  drop_graphs(e, nullptr);
   cudaError_t r = ensure(&e->d_codes, &e->cap_codes,
                          sizeof(DevCode) * (e->codes.empty() ? 1 : e->codes.size()));
   if (r == cudaSuccess && !e->codes.empty())
