@@ -239,15 +239,15 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   }
   const int max_jobs = num_shots;
   const size_t scratch_words = 64ull << 20;
-  const void *const held[] = {slot->d_jobs, slot->d_scratch, slot->d_small, slot->d_deferred};
+  const size_t held[] = {slot->cap_jobs, slot->cap_scratch, slot->cap_small, slot->cap_deferred};
   cudaError_t r = ensure_zeroed(&slot->d_jobs, &slot->cap_jobs, sizeof(Job) * (size_t)max_jobs);
   if (r == cudaSuccess) r = ensure(&slot->d_scratch, &slot->cap_scratch, scratch_words * 4);
   if (r == cudaSuccess) r = ensure_zeroed(&slot->d_small, &slot->cap_small, kCtlAllocBytes);
   if (r == cudaSuccess)
     r = ensure_zeroed(&slot->d_deferred, &slot->cap_deferred, shot_buffer_bytes(num_shots));
-  // launches captured on buffers that have moved would write where they were
-  if (held[0] != slot->d_jobs || held[1] != slot->d_scratch || held[2] != slot->d_small ||
-      held[3] != slot->d_deferred)
+  // launches captured before a buffer was replaced would write where it was
+  if (held[0] != slot->cap_jobs || held[1] != slot->cap_scratch || held[2] != slot->cap_small ||
+      held[3] != slot->cap_deferred)
     drop_graphs(e, slot);
   if (r != cudaSuccess) {
     set_error("grand: device workspace allocation failed (%s)", cudaGetErrorString(r));
@@ -271,7 +271,7 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   b.scratch = (uint32_t *)slot->d_scratch;
   b.scratch_words = scratch_words;
   b.deferred = (int *)slot->d_deferred;
-  b.queue = shot_queue(slot->d_deferred, num_shots);
+  b.queue = shot_queue(slot->d_deferred, slot->cap_deferred);
   // records in device memory: the per-shot path reads them again from L2 (the
   // record cache pays off only for records read in place from host memory)
   b.rec_cache = nullptr;

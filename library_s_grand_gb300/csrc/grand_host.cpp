@@ -61,9 +61,11 @@ cudaError_t ensure(void **p, size_t *cap, size_t bytes) {
 }
 
 cudaError_t ensure_zeroed(void **p, size_t *cap, size_t bytes) {
-  void *before = *p;
+  const bool enough = *p && *cap >= bytes;
   cudaError_t e = ensure(p, cap, bytes);
-  if (e == cudaSuccess && *p != before) e = cudaMemset(*p, 0, *cap);
+  // (a new allocation may have the old address; done before any other stream's launch)
+  if (e == cudaSuccess && !enough) e = cudaMemset(*p, 0, *cap);
+  if (e == cudaSuccess && !enough) e = cudaStreamSynchronize(nullptr);
   return e;
 }
 
@@ -540,10 +542,10 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
   b.scratch = (uint32_t *)ws->d_scratch;
   b.scratch_words = scratch_words;
   b.deferred = (int *)ws->d_deferred;
-  b.queue = shot_queue(ws->d_deferred, N);
+  b.queue = shot_queue(ws->d_deferred, ws->cap_deferred);
   // records read in place from host memory: the per-shot path takes the bits the
   // chunk step kept instead of a second read over NVLink-C2C
-  b.rec_cache = zc ? shot_rec_cache(ws->d_deferred, N) : nullptr;
+  b.rec_cache = zc ? shot_rec_cache(ws->d_deferred, ws->cap_deferred) : nullptr;
   b.epoch = (unsigned *)((char *)ws->d_small + kCtlBytes);
   b.fast = tn.fast;
   b.profile = tn.profile;

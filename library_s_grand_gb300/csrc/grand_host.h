@@ -93,9 +93,10 @@ cudaError_t ensure(void **p, size_t *cap, size_t bytes);
 // launch tag: zero is no launch's tag).
 cudaError_t ensure_zeroed(void **p, size_t *cap, size_t bytes);
 
-// Bytes of the per-shot buffer: num_shots re-run flags (int), then, 8-byte
-// aligned, num_shots slow-queue entries (u64), then, 16-byte aligned, num_shots
-// record-cache rows (kRecCacheWords words each).
+// The per-shot buffer: re-run flags (int), then, 8-byte aligned, slow-queue entries (u64),
+// then, 16-byte aligned, record-cache rows (kRecCacheWords words each), as many of each
+// as the whole buffer holds, however small the batch: a queue entry is told from an older
+// launch's by its tag, so flags and records must never lie where a later batch's entries do.
 inline size_t shot_queue_offset(size_t num_shots) { return (4 * num_shots + 7) & ~(size_t)7; }
 inline size_t shot_cache_offset(size_t num_shots) {
   return (shot_queue_offset(num_shots) + 8 * num_shots + 15) & ~(size_t)15;
@@ -103,12 +104,19 @@ inline size_t shot_cache_offset(size_t num_shots) {
 inline size_t shot_buffer_bytes(size_t num_shots) {
   return shot_cache_offset(num_shots) + sizeof(uint32_t) * kRecCacheWords * num_shots;
 }
-inline unsigned long long *shot_queue(void *shot_buffer, size_t num_shots) {
-  return reinterpret_cast<unsigned long long *>(static_cast<char *>(shot_buffer) +
-                                                shot_queue_offset(num_shots));
+// Shots that a buffer of this size was made for (the largest batch so far).
+inline size_t shot_capacity(size_t buffer_bytes) {
+  size_t n = buffer_bytes / (4 + 8 + sizeof(uint32_t) * kRecCacheWords);
+  while (n > 0 && shot_buffer_bytes(n) > buffer_bytes) --n;
+  return n;
 }
-inline uint32_t *shot_rec_cache(void *shot_buffer, size_t num_shots) {
-  return reinterpret_cast<uint32_t *>(static_cast<char *>(shot_buffer) + shot_cache_offset(num_shots));
+inline unsigned long long *shot_queue(void *shot_buffer, size_t buffer_bytes) {
+  return reinterpret_cast<unsigned long long *>(static_cast<char *>(shot_buffer) +
+                                                shot_queue_offset(shot_capacity(buffer_bytes)));
+}
+inline uint32_t *shot_rec_cache(void *shot_buffer, size_t buffer_bytes) {
+  return reinterpret_cast<uint32_t *>(static_cast<char *>(shot_buffer) +
+                                      shot_cache_offset(shot_capacity(buffer_bytes)));
 }
 
 class Context {

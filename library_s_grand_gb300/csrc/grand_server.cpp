@@ -192,8 +192,8 @@ cudaError_t start_slot(GrandServer *S, SrvSlot *sl) {
   b.scratch = sl->d_scratch;
   b.scratch_words = kSrvArenaWords;
   b.deferred = direct ? nullptr : sl->d_deferred;
-  b.queue = shot_queue(sl->d_deferred, S->max_shots);
-  b.rec_cache = in_place ? shot_rec_cache(sl->d_deferred, S->max_shots) : nullptr;
+  b.queue = shot_queue(sl->d_deferred, shot_buffer_bytes(S->max_shots));
+  b.rec_cache = in_place ? shot_rec_cache(sl->d_deferred, shot_buffer_bytes(S->max_shots)) : nullptr;
   b.epoch = (unsigned *)((char *)sl->d_small + kCtlBytes);
   b.fast = e->tn.fast;
   b.light_max_log2 = e->tn.light_max_log2;
