@@ -1,5 +1,6 @@
 // grand_host.cpp -- device context, code tables, workspaces and the batch driver.
 #include "grand_host.h"
+#include "grand_plan.h"
 #include "grand_solo.h"
 
 #include <stdarg.h>
@@ -552,7 +553,7 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
   b.light_max_log2 = tn.light_max_log2;
   b.tile_k = tn.tile_k;
 
-  std::vector<int> map;
+  std::vector<int> map, unsearched;
   int todo = N;
   float tri_ms = 0, sea_ms = 0;
   int rounds = 0;
@@ -585,14 +586,12 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
     // Re-run the shots that did not fit the job table or scratch.
     std::vector<int> def(N);
     CK(cudaMemcpy(def.data(), ws->d_deferred, sizeof(int) * N, cudaMemcpyDeviceToHost));
-    std::vector<int> prev = map;
-    map.clear();
-    if (rounds == 1) {
-      for (int i = 0; i < N; ++i) if (def[i]) map.push_back(i);
-    } else {
-      for (int i : prev) if (def[i]) map.push_back(i);
+    const bool fewer = next_round(map, def, rounds == 1);
+    if (map.empty()) break;
+    if (!fewer) {
+      unsearched.swap(map);
+      break;
     }
-    if (map.empty() || rounds > 64) break;
     todo = (int)map.size();
     CK(ensure(&ws->d_map, &ws->cap_map, sizeof(int) * map.size()));
     CK(cudaMemcpyAsync(ws->d_map, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice, s));
@@ -621,6 +620,17 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
     timing->decode_ms = sea_ms;
     timing->d2h_ms = d2h;
     timing->rounds = rounds;
+  }
+  for (int i : unsearched) {  // nothing wrote these
+    memset(req.h_results + i, 0, sizeof(GrandDecoderResult));
+    if (req.h_dec_err) memset(req.h_dec_err + (size_t)i * req.dec_m, 0, req.dec_m);
+    if (req.h_dec_log) memset(req.h_dec_log + (size_t)i * req.dec_nl, 0, req.dec_nl);
+    if (req.h_cost) req.h_cost[i] = 0.0f;
+  }
+  if (!unsearched.empty()) {
+    set_error("grand: %zu shot(s) need more than the search arena on their own; their results "
+              "are zero (found = 0)", unsearched.size());
+    return GRAND_ERR_LIMIT;
   }
   if (status_all & kStatusTamLimit) {
     set_error("grand: an active-position set exceeded GRAND_MAX_TAM=%d; those shots are "

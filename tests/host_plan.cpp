@@ -1,12 +1,13 @@
 // Host-side checks of what the library decides before a launch, for
 // tests/test_plan_host.py.
 //
-// Usage: host_plan layout
+// Usage: host_plan layout | rounds
 #include <cstdio>
 #include <cstring>
 #include <vector>
 
 #include "grand_host.h"
+#include "grand_plan.h"
 
 using namespace grand;
 
@@ -30,7 +31,44 @@ static int layout() {
   return 0;
 }
 
+// Rounds of a batch against an arena that `fit` shots fill: each shot is searched once, in
+// however many rounds that takes, and shots that alone outgrow it are told from the rest.
+static int rounds() {
+  for (int shots : {1, 63, 1000}) {
+    for (int fit : {1, 7, 2000}) {
+      for (int huge : {0, 1, 5}) {
+        std::vector<int> flags(shots, 0), searched(shots, 0), map;
+        int round = 0;
+        for (;; ++round) {
+          if (round > shots + 1) return 1;
+          int room = fit, any = 0;
+          const int todo = round ? (int)map.size() : shots;
+          for (int k = 0; k < todo; ++k) {
+            const int i = round ? map[k] : k;
+            const bool full = i % 97 < huge || room == 0;
+            flags[i] = full;
+            any |= full;
+            if (!full) --room, ++searched[i];
+          }
+          if (!any) {
+            map.clear();
+            break;
+          }
+          const bool fewer = next_round(map, flags, round == 0);
+          if (map.empty() || !fewer) break;
+        }
+        std::vector<int> left(shots, 0);
+        for (int i : map) left[i] = 1;
+        for (int i = 0; i < shots; ++i)
+          if (searched[i] != (i % 97 < huge ? 0 : 1) || left[i] != (i % 97 < huge ? 1 : 0)) return 2;
+      }
+    }
+  }
+  return 0;
+}
+
 int main(int argc, char **argv) {
   if (argc == 2 && !strcmp(argv[1], "layout")) return layout();
+  if (argc == 2 && !strcmp(argv[1], "rounds")) return rounds();
   return 9;
 }

@@ -29,3 +29,7 @@ def _run(exe, *args):
 
 def test_per_shot_buffer_layout(plan):
     _run(plan, "layout")
+
+
+def test_rounds_go_on_while_shots_get_fewer(plan):
+    _run(plan, "rounds")
