@@ -150,21 +150,24 @@ def _uninit(nbytes):
     return a
 
 
+_UNWRITTEN = -1  # `found` of the first result until the library has written it
+
+
 def _new_results(shots):
     if shots < 64:
-        return (GrandDecoderResult * shots)()
-    return (GrandDecoderResult * shots).from_buffer(_uninit(72 * shots))
+        results = (GrandDecoderResult * shots)()
+    else:
+        results = (GrandDecoderResult * shots).from_buffer(_uninit(72 * shots))
+    if shots:
+        results[0].found = _UNWRITTEN
+    return results
 
 
-_ERR_LIMIT = -3  # matrix beyond the size limits (not decoded), or an active set (decoded)
+_ERR_LIMIT = -3  # a size beyond the limits (nothing written), or a search's (all written)
 
 
-def _undecoded(rc, n, m, nl=0):
-    return rc != 0 and (rc != _ERR_LIMIT or n > 1024 or m > 4096 or nl > 1024)
-
-
-def _finish(rc, results, n, m, nl=0, arrays=()):
-    if _undecoded(rc, n, m, nl):
+def _finish(rc, results, arrays=()):
+    if rc != 0 and not (rc == _ERR_LIMIT and len(results) and results[0].found != _UNWRITTEN):
         ctypes.memset(results, 0, ctypes.sizeof(results))
         for a in arrays:
             a.fill(0)
@@ -215,7 +218,7 @@ def run_grand_shots_cc(lib, Hx, Hz, errors, syndromes, cfg, error_type):
     keep, args, shots, _ = _css_args(Hx, Hz, errors, syndromes)
     results = _new_results(shots)
     rc = lib.grand_decode_cc(*args, ctypes.byref(cfg), results, ctypes.c_char(error_type))
-    _finish(rc, results, args[2], args[3])
+    _finish(rc, results)
     return rc, results
 
 
@@ -224,7 +227,7 @@ def run_grand_prob_shots_cc(lib, Hx, Hz, errors, syndromes, cfg, prob_file_path,
     results = _new_results(shots)
     rc = lib.grand_decode_prob_cc(*args, ctypes.byref(cfg), results, ctypes.c_char(error_type),
                                   prob_file_path.encode("utf-8"))
-    _finish(rc, results, args[2], args[3])
+    _finish(rc, results)
     return rc, results
 
 
@@ -240,7 +243,7 @@ def run_grand_shots_cln(lib, H_dem, L_dem, detectors, logicals, n_logicos, cfg):
     keep, args, shots, _ = _dem_args(H_dem, L_dem, detectors, logicals, n_logicos)
     results = _new_results(shots)
     rc = lib.grand_decode_cln(*args, ctypes.byref(cfg), results)
-    _finish(rc, results, args[2], args[3], n_logicos)
+    _finish(rc, results)
     return rc, results
 
 
@@ -250,7 +253,7 @@ def run_grand_prob_shots_cln(lib, H_dem, L_dem, detectors, logicals, n_logicos, 
     results = _new_results(shots)
     rc = lib.grand_decode_prob_cln(*args, ctypes.byref(cfg), results,
                                    prob_file_path.encode("utf-8"))
-    _finish(rc, results, args[2], args[3], n_logicos)
+    _finish(rc, results)
     return rc, results
 
 
@@ -258,7 +261,7 @@ def run_grand_ML_shots_cln(lib, H_dem, L_dem, detectors, logicals, n_logicos, cf
     keep, args, shots, _ = _dem_args(H_dem, L_dem, detectors, logicals, n_logicos)
     results = _new_results(shots)
     rc = lib.grand_decode_ML_cln(*args, ctypes.byref(cfg), results, llr_file_path.encode("utf-8"))
-    _finish(rc, results, args[2], args[3], n_logicos)
+    _finish(rc, results)
     return rc, results
 
 
@@ -275,7 +278,7 @@ def decode_css_ex(lib, variant, Hx, Hz, errors, syndromes, cfg, error_type, prob
                                          os.fsencode(prob_file), ctypes.byref(out))
     else:
         rc = lib.grand_decode_cc_ex(*args, ctypes.byref(cfg), results, et, ctypes.byref(out))
-    _finish(rc, results, args[2], m, 0, (dec,))
+    _finish(rc, results, (dec,))
     return rc, _as_array(results), dec
 
 
@@ -294,7 +297,7 @@ def decode_dem_ex(lib, variant, H_dem, L_dem, detectors, logicals, cfg, file=Non
                                         ctypes.byref(out))
     else:
         rc = lib.grand_decode_cln_ex(*args, ctypes.byref(cfg), results, ctypes.byref(out))
-    _finish(rc, results, args[2], m, nl, (dec, dlog))
+    _finish(rc, results, (dec, dlog))
     return rc, _as_array(results), dec, dlog, cost
 
 
@@ -328,7 +331,7 @@ def run_grand_shots_cc_packed(lib, Hx, Hz, words, kind, cfg, error_type, prob_fi
     rc = lib.grand_decode_cc_packed(_p(hx), _p(hz), n_rows, n_cols, w.ctypes.data, kind, shots,
                                     ctypes.byref(cfg), results, ctypes.c_char(_type_byte(error_type)),
                                     os.fsencode(prob_file) if prob_file else None)
-    _finish(rc, results, n_rows, n_cols)
+    _finish(rc, results)
     return rc, results
 
 
@@ -344,7 +347,7 @@ def decode_css_packed(lib, Hx, Hz, words, kind, cfg, error_type, prob_file=None)
     rc = lib.grand_decode_cc_packed(_p(hx), _p(hz), n_rows, n_cols, w.ctypes.data, kind, shots,
                                     ctypes.byref(cfg), results, ctypes.c_char(_type_byte(error_type)),
                                     os.fsencode(prob_file) if prob_file else None)
-    _finish(rc, results, n_rows, n_cols)
+    _finish(rc, results)
     return rc, _as_array(results)
 
 
@@ -362,5 +365,5 @@ def decode_dem_packed(lib, variant, H_dem, L_dem, det_words, log_words, cfg, fil
     rc = lib.grand_decode_cln_packed(_p(h), _p(l), n_rows, n_cols, nl, d.ctypes.data, g.ctypes.data,
                                      shots, ctypes.byref(cfg), results, v,
                                      os.fsencode(file) if file else None)
-    _finish(rc, results, n_rows, n_cols, nl)
+    _finish(rc, results)
     return rc, _as_array(results)
