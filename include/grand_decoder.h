@@ -163,7 +163,7 @@ int grand_decode_ML_cln_ex(int *H_dem, const int *L_dem, int n, int m, int n_log
  * syndromes, ...) field for field, and the timing fields are per-shot GPU timer
  * values as with the other entry points.  Everything else lives in one fixed
  * file-scope device array of about 25 MiB, held by every GPU that loads it until
- * the process exits.  Limits: n <= 256, m <= 1024 (larger sizes return
+ * the process exits, and one word a GPU of the library's own host memory.  Limits: n <= 256, m <= 1024 (larger sizes return
  * GRAND_ERR_LIMIT with a message).  Shots run in chunks of 2048; hard shots of a
  * chunk share a 16 MiB search arena, and shots that find it full are re-run in
  * further rounds of the chunk with the arena emptied; a shot whose search data

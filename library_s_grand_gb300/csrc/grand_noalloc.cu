@@ -107,7 +107,13 @@ __global__ void noalloc_clear_kernel(const int *map, int count, GrandDecoderResu
 std::mutex g_mu;
 unsigned char *g_base[64] = {};  // device address of g_noalloc_scratch per device
 int g_sms[64] = {}, g_bps[64] = {};
-unsigned *g_status[64] = {};     // pinned: the status word of a round, raised by the kernels in place
+// The status word of a round.  Where the device reaches the host's own memory (NVLink-C2C) the
+// kernels raise it here, in place; otherwise in the control block, from where it is copied.
+struct alignas(128) StatusWord {
+  unsigned bits;
+};
+StatusWord g_status[64] = {};
+bool g_status_here[64] = {};
 
 }  // namespace
 }  // namespace grand
@@ -176,10 +182,10 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
         fprintf(stderr, "grand_decode_cc_noalloc: set-up failed (%s)\n", cudaGetErrorString(e));
         return GRAND_ERR_CUDA;
       }
-      if (cudaHostAlloc(reinterpret_cast<void **>(&g_status[dev]), 256, cudaHostAllocDefault) != cudaSuccess) {
-        fprintf(stderr, "grand_decode_cc_noalloc: set-up failed (no pinned status word)\n");
-        return GRAND_ERR_CUDA;
-      }
+      int reach = 0, atomics = 0;
+      cudaDeviceGetAttribute(&reach, cudaDevAttrPageableMemoryAccess, dev);
+      cudaDeviceGetAttribute(&atomics, cudaDevAttrHostNativeAtomicSupported, dev);
+      g_status_here[dev] = reach && atomics;
       g_sms[dev] = sms;
       g_bps[dev] = bps > 0 ? bps : 1;
       g_base[dev] = (unsigned char *)ptr;
@@ -249,7 +255,8 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
     b.jobs = reinterpret_cast<Job *>(base + kOffJobs);
     b.max_jobs = kNaChunk;
     b.counters = reinterpret_cast<unsigned long long *>(base + kOffSmall);
-    b.status = g_status[dev];
+    b.status = g_status_here[dev] ? &g_status[dev].bits
+                                  : reinterpret_cast<unsigned *>(base + kOffSmall + kStatusByteOffset);
     b.scratch = reinterpret_cast<uint32_t *>(base + kOffArena);
     b.scratch_words = kNaArenaWords;
     b.deferred = reinterpret_cast<int *>(base + kOffDeferred);
@@ -272,12 +279,15 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
       b.chunk = std::min((todo - 1) / (g_sms[dev] * kChunkMinBlocks * kChunkWarps) + 1, (int)kMaxChunk);
       // control words and status restart for every round
       if (lo > 0 || round > 0) e = cudaMemsetAsync(base + kOffSmall, 0, kCtlBytes, s);
-      volatile unsigned *status = g_status[dev];
+      volatile unsigned *status = &g_status[dev].bits;
+      unsigned rs = 0u;
       *status = 0u;
       if (e == cudaSuccess) e = launch_decode(b, g_sms[dev] * per_sm, s);
+      if (e == cudaSuccess && !g_status_here[dev])
+        e = cudaMemcpyAsync(&rs, b.status, sizeof(rs), cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
       if (e != cudaSuccess) break;
-      const unsigned rs = *status;
+      rs |= *status;
       st |= rs & ~(unsigned)(kStatusScratchOverflow | kStatusJobOverflow);
       if (!(rs & (kStatusScratchOverflow | kStatusJobOverflow))) break;
       noalloc_deferred_kernel<<<1, 32, 0, s>>>(b.deferred, cnt, map, map_count);
