@@ -13,6 +13,7 @@
 
 #include "grand_engine_internal.h"
 #include "grand_host.h"
+#include "grand_plan.h"
 
 namespace grand {
 double measure_lop3_peak(int sm_count);
@@ -333,16 +334,15 @@ int grand_engine_sync_status(GrandEngine *e, void *stream) {
                    cudaMemcpyDeviceToHost);
   }
   if (r != cudaSuccess) return GRAND_ERR_CUDA;
+  const int rc = status_code(st);
+  if (rc == GRAND_ERR_CUDA) return rc;
   if (st & (kStatusJobOverflow | kStatusScratchOverflow)) {
     set_error("grand: device decode ran out of job table or scratch space; use grand_engine_decode");
     return GRAND_ERR_LIMIT;
   }
-  if (st & kStatusTamLimit) {
+  if (rc == GRAND_ERR_LIMIT)
     set_error("grand: an active-position set exceeded GRAND_MAX_TAM=%d", kMaxTam);
-    return GRAND_ERR_LIMIT;
-  }
-  if (st & (kStatusCasLimit | kStatusWaitLimit)) return GRAND_ERR_CUDA;
-  return 0;
+  return rc;
 }
 
 int grand_engine_launch_stats(GrandEngine *e, void *stream, long long *out) {

@@ -627,25 +627,19 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
     if (req.h_dec_log) memset(req.h_dec_log + (size_t)i * req.dec_nl, 0, req.dec_nl);
     if (req.h_cost) req.h_cost[i] = 0.0f;
   }
-  if (!unsearched.empty()) {
+  const int rc = status_code(status_all);
+  if (rc == GRAND_ERR_CUDA) {
+    set_error("grand: internal %s limit reached",
+              status_all & kStatusCasLimit ? "ML reduction retry" : "wait");
+  } else if (!unsearched.empty()) {
     set_error("grand: %zu shot(s) need more than the search arena on their own; their results "
               "are zero (found = 0)", unsearched.size());
     return GRAND_ERR_LIMIT;
-  }
-  if (status_all & kStatusTamLimit) {
+  } else if (rc == GRAND_ERR_LIMIT) {
     set_error("grand: an active-position set exceeded GRAND_MAX_TAM=%d; those shots are "
               "reported unsearched", kMaxTam);
-    return GRAND_ERR_LIMIT;
   }
-  if (status_all & kStatusCasLimit) {
-    set_error("grand: internal ML reduction retry limit reached");
-    return GRAND_ERR_CUDA;
-  }
-  if (status_all & kStatusWaitLimit) {
-    set_error("grand: internal wait limit reached");
-    return GRAND_ERR_CUDA;
-  }
-  return 0;
+  return rc;
 }
 
 }  // namespace grand

@@ -23,6 +23,7 @@
 
 #include "grand_common.h"
 #include "grand_host.h"
+#include "grand_plan.h"
 #include "grand_prep.cuh"
 
 namespace grand {
@@ -311,6 +312,12 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
     fprintf(stderr, "grand_decode_cc_noalloc: CUDA error %s\n", cudaGetErrorString(e));
     return GRAND_ERR_CUDA;
   }
+  const int rc = status_code(st);
+  if (rc == GRAND_ERR_CUDA) {
+    fprintf(stderr, "grand_decode_cc_noalloc: internal %s limit reached\n",
+            st & kStatusCasLimit ? "ML reduction retry" : "wait");
+    return rc;
+  }
   if (unsearched) {
     fprintf(stderr,
             "grand_decode_cc_noalloc: %lld shot(s) need more than the fixed %llu-word search "
@@ -318,10 +325,7 @@ extern "C" int grand_decode_cc_noalloc(const int *d_H, int n, int m, const int *
             unsearched, kNaArenaWords);
     return GRAND_ERR_LIMIT;
   }
-  if (st & kStatusTamLimit) {
+  if (rc == GRAND_ERR_LIMIT)
     fprintf(stderr, "grand_decode_cc_noalloc: an active-position set exceeded %d\n", kMaxTam);
-    return GRAND_ERR_LIMIT;
-  }
-  if (st & kStatusCasLimit) return GRAND_ERR_CUDA;
-  return 0;
+  return rc;
 }

@@ -3,7 +3,17 @@
 
 #include <vector>
 
+#include "grand_common.h"
+
 namespace grand {
+
+// The return code for the status bits of a finished batch (those of a full job table or arena
+// apart): a warp that gave up waiting left shots undecoded, which comes before a set that
+// was too large, reported in its result.
+inline int status_code(unsigned status) {
+  if (status & (kStatusCasLimit | kStatusWaitLimit)) return GRAND_ERR_CUDA;
+  return status & kStatusTamLimit ? GRAND_ERR_LIMIT : 0;
+}
 
 // The shots of the next round after one in which some found the job table or the arena full:
 // those of map (in the first round: of all shots) whose re-run flag is set.  False when there

@@ -34,6 +34,7 @@
 
 #include "grand_engine_internal.h"
 #include "grand_host.h"
+#include "grand_plan.h"
 
 using namespace grand;
 using Clock = std::chrono::steady_clock;
@@ -239,10 +240,8 @@ void finish_slot(GrandServer *S, SrvSlot *sl, int rc) {
     req.h_results = sl->h_res;
     rc = ws ? run_batch(S->eng->ctx, ws, req, nullptr, &S->eng->tn) : GRAND_ERR_CUDA;
     if (ws) S->eng->ctx->release(ws);
-  } else if (rc == 0 && (*sl->h_status & kStatusTamLimit)) {
-    rc = GRAND_ERR_LIMIT;
-  } else if (rc == 0 && (*sl->h_status & (kStatusCasLimit | kStatusWaitLimit))) {
-    rc = GRAND_ERR_CUDA;
+  } else if (rc == 0) {
+    rc = status_code(*sl->h_status);
   }
   if (rc == 0 && sl->nshots > 0) {
     // an overflowing batch staged at least the whole arena

@@ -1,7 +1,7 @@
 // Host-side checks of what the library decides before a launch, for
 // tests/test_plan_host.py.
 //
-// Usage: host_plan layout | rounds
+// Usage: host_plan layout | rounds | status
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -67,8 +67,20 @@ static int rounds() {
   return 0;
 }
 
+// Every combination of status bits: a wait or retry that gave up is an error whatever else
+// was raised.
+static int status() {
+  for (unsigned st = 0; st < 64; ++st) {
+    const bool gave_up = st & (kStatusCasLimit | kStatusWaitLimit);
+    const int want = gave_up ? GRAND_ERR_CUDA : (st & kStatusTamLimit ? GRAND_ERR_LIMIT : 0);
+    if (status_code(st) != want) return 1;
+  }
+  return 0;
+}
+
 int main(int argc, char **argv) {
   if (argc == 2 && !strcmp(argv[1], "layout")) return layout();
   if (argc == 2 && !strcmp(argv[1], "rounds")) return rounds();
+  if (argc == 2 && !strcmp(argv[1], "status")) return status();
   return 9;
 }

@@ -33,3 +33,15 @@ def test_per_shot_buffer_layout(plan):
 
 def test_rounds_go_on_while_shots_get_fewer(plan):
     _run(plan, "rounds")
+
+
+def test_status_bits(plan):
+    _run(plan, "status")
+
+
+def test_every_entry_point_uses_the_same_rule():
+    """No entry point tests the bits by itself: one that left the wait limit out returned 0."""
+    for name in ("grand_host.cpp", "grand_engine.cpp", "grand_server.cpp", "grand_noalloc.cu"):
+        with open(os.path.join(ROOT, "library_s_grand_gb300", "csrc", name), encoding="utf-8") as f:
+            code = f.read()
+        assert "status_code(" in code and "kStatusWaitLimit" not in code and "kStatusTamLimit" not in code, name
