@@ -75,6 +75,7 @@ int grand_engine_add_css(GrandEngine *e, const int *Hx, const int *Hz, int n, in
   e->codes.push_back(make_devcode(*tab, p));
   e->tabs.push_back(tab);
   e->llr.push_back(nullptr);
+  std::lock_guard<std::mutex> llk(e->len_mu);
   e->rec_len.push_back(records_are_errors ? m : n);
   e->dirty = true;
   if (code_id) *code_id = (int)e->codes.size() - 1;
@@ -124,6 +125,7 @@ int grand_engine_add_dem(GrandEngine *e, const int *H, const int *L, int n, int 
   e->codes.push_back(make_devcode(*tab, p));
   e->tabs.push_back(tab);
   e->llr.push_back(d_llr);
+  std::lock_guard<std::mutex> llk(e->len_mu);
   e->rec_len.push_back(n + nl);
   e->dirty = true;
   if (code_id) *code_id = (int)e->codes.size() - 1;

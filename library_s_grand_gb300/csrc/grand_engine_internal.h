@@ -50,6 +50,7 @@ struct GrandEngine {
   std::vector<std::shared_ptr<grand::CodeTables>> tabs;
   std::vector<float *> llr;
   std::vector<int> rec_len;
+  std::mutex len_mu;  // with mu, around changes of rec_len; alone, to read it without waiting for launches
   void *d_codes = nullptr;
   size_t cap_codes = 0;
   bool dirty = true;

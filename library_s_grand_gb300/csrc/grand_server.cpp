@@ -434,7 +434,7 @@ int grand_server_submit(GrandServer *S, int n, const int *shot_code, const int *
                         GrandDecoderResult *results, unsigned long long *request_id) {
   if (!S || n <= 0 || n > S->max_shots || !records || !results) return GRAND_ERR_INVALID;
   {
-    std::lock_guard<std::mutex> elk(S->eng->mu);
+    std::lock_guard<std::mutex> elk(S->eng->len_mu);
     const std::vector<int> &len = S->eng->rec_len;
     // a slot's staging holds records of the codes registered when the server was created
     const bool staged = !(S->eng->tn.zero_copy && S->eng->ctx->pageable_access);
@@ -483,7 +483,7 @@ int grand_server_replay(GrandServer *S, int nreq, const double *arrival_s, const
   std::vector<long long> shot0(nreq + 1, 0), rec0(nreq + 1, 0);
   std::vector<int> rec_len;
   {
-    std::lock_guard<std::mutex> elk(S->eng->mu);
+    std::lock_guard<std::mutex> elk(S->eng->len_mu);
     rec_len = S->eng->rec_len;
   }
   for (int i = 0; i < nreq; ++i) {
