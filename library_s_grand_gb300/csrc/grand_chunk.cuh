@@ -37,9 +37,6 @@ __device__ __forceinline__ void xor_col(const uint32_t *cols, bool wide, unsigne
 // ---------------------------------------------------------------------------
 // Chunks of up to kMaxChunk launch slots, one lane per shot.
 // ---------------------------------------------------------------------------
-constexpr int kFastWords = 8;         // syndrome words of a lane's shot (R <= 256)
-constexpr int kFastLogWords = 4;      // DEM logical words (n_logicos <= 128)
-constexpr int kFastErrWords = 32;     // error-record words (m <= 1024)
 // words of a chunk's separate logical entries (flat_ballots)
 constexpr int kLogBallots = kMaxChunk * kFastLogWords + 8;
 
@@ -181,8 +178,7 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
   const int nw = cd.nw;
   const int nbits = errs ? cd.m : cd.R;       // entries of the record's leading bit vector
   const int nwords = (nbits + 31) >> 5;
-  bool ok = valid && nw <= kFastWords && (!errs || nwords <= kFastErrWords) &&
-            (!dem || cd.nlw <= kFastLogWords);
+  bool ok = valid && chunk_takes(cd);
   const long long rbase = valid ? (b.in_off ? b.in_off[shot] : (long long)shot * cd.rec_len) : 0;
   uint32_t *row = F.row[valid ? lane : 0];
   if (valid) {
@@ -287,9 +283,10 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
   ok = ok && (packed || !dem || log_ok || !sep);
   // Runs of consecutive lanes whose int32 records lie back to back (one run for a
   // batch packed in slot order; a few where requests' records sit in separate
-  // buffers): each run's entries through one pass of ballots.
+  // buffers): each run's entries through one pass of ballots.  Records the chunk does not
+  // take are left out: with them a run could outgrow the ballot area.
   const int rlen = dem && !sep ? cd.R + cd.n_logicos : nbits;
-  const bool mine = valid && !packed;
+  const bool mine = ok && !packed;
   const long long pend = __shfl_up_sync(kFull, rbase + rlen, 1);
   const bool pint = __shfl_up_sync(kFull, mine ? 1 : 0, 1) != 0;
   const unsigned members_all = __ballot_sync(kFull, mine);

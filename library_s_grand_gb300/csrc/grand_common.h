@@ -74,6 +74,9 @@ constexpr int kGuidedF = 15;            // filter bits, log2 (4 KB)
 // stays L1 for the code tables.
 constexpr int kMaxChunk = 32;
 constexpr int kFastBallots = 256;
+constexpr int kFastWords = 8;           // syndrome words of a chunk's shot (R <= 256)
+constexpr int kFastLogWords = 4;        // its DEM logical words (n_logicos <= 128)
+constexpr int kFastErrWords = 32;       // its error-record words (m <= 1024)
 constexpr int kGuidedLanes = 8;         // lanes that search a shot (a warp searches 32 / 8 at once)
 constexpr int kGuidedItems = 384;       // partial sets a warp's searches hold together
 constexpr int kHotCodes = 8;            // codes a block of the chunk kernel copies to shared memory
@@ -195,6 +198,12 @@ struct HotCode {
   float llr_min;             // the least of them
   int pad_;                  // (whole 8-byte words)
 };
+
+// Do the chunk step's rows hold this code's shots?
+GRAND_HD inline bool chunk_takes(const HotCode &cd) {
+  return cd.nw <= kFastWords && (cd.input_kind != kInErrors || cd.mw <= kFastErrWords) &&
+         (cd.family != kDem || cd.nlw <= kFastLogWords);
+}
 
 // Immutable per-code tables plus the per-call search parameters.
 struct DevCode : HotCode {

@@ -283,7 +283,7 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   b.profile = e->tn.profile;
   b.light_max_log2 = e->tn.light_max_log2;
   b.tile_k = e->tn.tile_k;
-  plan_batch(b, e->codes.data(), (int)e->codes.size(), e->ctx->sm_count, e->tn);
+  plan_batch(b, e->codes.data(), (int)e->codes.size(), e->ctx->sm_count, e->tn.fast != 0);
   if (!use_graph) {
     cudaEventRecord(slot->ev[0], s);
     r = launch_pipeline(e->ctx, b, e->tn, s, slot->ev[1]);

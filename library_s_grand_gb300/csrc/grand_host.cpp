@@ -399,32 +399,6 @@ DevCode make_devcode(const CodeTables &t, const CallParams &p) {
   return d;
 }
 
-void plan_batch(DevBatch &b, const DevCode *codes, int ncodes, int sm_count, const Tuning &tn) {
-  bool any = false, all = true;
-  long long entries = 1;  // int32 entries of the longest record
-  b.has_ml = 0;
-  for (int i = 0; i < ncodes; ++i) {
-    b.has_ml |= codes[i].variant == kMl;
-    any = any || codes[i].g_gs;
-    all = all && guided_closed(codes[i]);
-    if (!codes[i].packed) entries = std::max<long long>(entries, codes[i].rec_len);
-  }
-  all = all && entries <= 32 * kFastBallots && !b.shot_map;
-  b.guided = !tn.fast || !any ? kGuidedNone : (all ? kGuidedAll : kGuidedFirst);
-  b.chunk = kMaxChunk;
-  if (b.guided) {
-    // full waves of the resident warps, in chunks as large as they may be: a chunk costs
-    // its records' round trips whatever its size, a part wave costs a whole one (twice
-    // the chunks in half the size: headline 30.8 -> 40.3 us, noisy [[288]] 52 -> 62)
-    const int warps = sm_count * kChunkMinBlocks * kChunkWarps;
-    const int most = (int)std::min<long long>(kMaxChunk, 32 * kFastBallots / entries);
-    const int waves = (b.num_shots - 1) / (warps * std::max(most, 1)) + 1;
-    const int c = std::min((b.num_shots - 1) / (warps * waves) + 1, most);
-    b.chunk = std::max(c, 1);
-  }
-  if (b.guided == kGuidedAll) b.deferred = nullptr;  // nothing is ever deferred
-}
-
 int decode_blocks_per_sm(int occupancy_bps, const Tuning &tn) {
   const int occ = std::max(occupancy_bps, 1);
   return tn.search_grid_mult ? std::min(tn.search_grid_mult, occ) : occ;
@@ -561,7 +535,7 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
   for (;;) {
     b.num_shots = todo;
     b.shot_map = rounds == 0 ? nullptr : (const int *)ws->d_map;
-    plan_batch(b, req.codes.data(), ncodes, ctx->sm_count, tn);
+    plan_batch(b, req.codes.data(), ncodes, ctx->sm_count, tn.fast != 0);
     // the chunk kernel alone raises nothing in the course of a batch: its status word can
     // be the host's own
     const bool own = b.guided == kGuidedAll;

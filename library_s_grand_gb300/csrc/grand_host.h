@@ -179,10 +179,6 @@ Tuning &tuning();  // process defaults (GRAND_LIGHT_LOG2, GRAND_TILE_K, GRAND_SE
 int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming *timing,
               const Tuning *tn = nullptr);
 
-// Which kernels decode the batch, and its chunks: b.has_ml, b.guided, b.chunk, from its
-// codes, b.num_shots and b.shot_map.
-void plan_batch(DevBatch &b, const DevCode *codes, int ncodes, int sm_count, const Tuning &tn);
-
 // Enqueue one batch on s: the control-word reset and the kernels it needs.
 cudaError_t launch_pipeline(const Context *ctx, const DevBatch &b, const Tuning &tn,
                             cudaStream_t s, cudaEvent_t mid = nullptr);

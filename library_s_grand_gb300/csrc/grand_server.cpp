@@ -167,7 +167,7 @@ cudaError_t start_slot(GrandServer *S, SrvSlot *sl) {
   memset(&b, 0, sizeof(b));
   b.num_shots = shot;
   b.num_codes = (int)e->codes.size();
-  plan_batch(b, e->codes.data(), b.num_codes, e->ctx->sm_count, e->tn);
+  plan_batch(b, e->codes.data(), b.num_codes, e->ctx->sm_count, e->tn.fast != 0);
   // The chunk kernel alone, with the records read in place, also reads the offsets and
   // codes and writes the results and the status word in the slot's pinned memory: the
   // batch is one launch (seven copies and resets before: a burst of 64 requests 341 ->

@@ -1,0 +1,124 @@
+"""CPU parity of whole batches planned as the library plans them (tests/host_route.cpp): which
+kernel takes which shots, in chunks of what size, for codes with and without guided tables."""
+import os
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+import oracle as O
+from library_s_grand_gb300 import capi, synth
+from test_host_kernels import HERE, ROOT, _cuda_include, _write_code
+
+
+@pytest.fixture(scope="module")
+def route(tmp_path_factory):
+    cxx, inc = shutil.which("g++"), _cuda_include()
+    if cxx is None or inc is None:
+        pytest.skip("needs g++ and the CUDA headers")
+    exe = str(tmp_path_factory.mktemp("hr") / "host_route")
+    subprocess.run([cxx, "-std=c++20", "-O2", "-pthread",
+                    "-I", os.path.join(ROOT, "library_s_grand_gb300", "csrc"),
+                    "-I", os.path.join(ROOT, "include"), "-I", inc, "-I", HERE,
+                    os.path.join(HERE, "host_route.cpp"), "-o", exe],
+                   check=True, capture_output=True, text=True)
+    return exe
+
+
+def sparse(rows, cols, weight, seed):
+    rng = np.random.default_rng(seed)
+    h = np.zeros((rows, cols), np.int32)
+    for c in range(cols):
+        h[rng.choice(rows, weight, replace=False), c] = 1
+    return h
+
+
+def decode(exe, d, codes, records, shot_code, starts=None, light=10, tables=True):
+    """codes: argument tuples of _write_code after the directory, with its keywords; starts: where
+    each record begins in the flat records (None: back to back).  Returns the results and the
+    numbers of the program's two lines by name."""
+    for k, (args, kw) in enumerate(codes):
+        _write_code(str(d / f"code{k}"), *args, **kw)
+    n = len(records)
+    lens = np.array([len(r) for r in records])
+    if starts is None:
+        starts = np.concatenate([[0], np.cumsum(lens)[:-1]])
+    flat = np.zeros(int((starts + lens).max()), np.int32)
+    for s, r in zip(starts, records):
+        flat[s:s + len(r)] = r
+    with open(d / "mixed.txt", "w") as f:
+        f.write(f"{len(codes)} {n} {light} 4\n")
+    flat.tofile(d / "rec.bin")
+    np.asarray(starts, np.int64).tofile(d / "off.bin")
+    np.asarray(shot_code, np.int32).tofile(d / "code.bin")
+    p = subprocess.run([exe, str(d)] + ([] if tables else ["tables=0"]), capture_output=True, text=True,
+                       timeout=600)
+    assert p.returncode == 0, (p.returncode, p.stdout, p.stderr)
+    first, second = p.stdout.split("\n")[:2]
+    w = first.replace(",", "").split()
+    info = {"jobs": int(w[3]), "slow": int(w[5])}
+    w = second.split()
+    info.update({w[i]: int(w[i + 1]) for i in range(0, len(w), 2)})
+    return np.fromfile(d / "res.bin", dtype=capi.RESULT_DTYPE), info
+
+
+@pytest.mark.parametrize("cols,errors", [(200, True), (256, True), (257, True), (300, True), (512, True),
+                                         (1000, True), (300, False)])
+def test_chunks_of_codes_without_tables(route, port, tmp_path, cols, errors):
+    """Nine ones a column: no guided tables.  Empty records and single columns are settled in
+    chunks, whatever the records' length; only the others take the per-shot path."""
+    h = sparse(60, cols, 9, cols)
+    rng = np.random.default_rng(2)
+    e = np.zeros((70, cols), np.int32)
+    for i in range(70):
+        e[i, rng.choice(cols, (0, 1, 0, 1, 2)[i % 5], replace=False)] = 1
+    syn = (e @ h.T & 1).astype(np.int32)
+    cfg = (2, 256, 0, 64, 10, -1)
+    rec = e if errors else syn
+    res, info = decode(route, tmp_path, [((h, 0, 1 if errors else 0, cfg, []), {"Ho": h})], list(rec),
+                       [0] * 70)
+    prc, want, _ = port.css(O.UNIFORM, h, h, e if errors else None, None if errors else syn,
+                            O.Config(*cfg), "x")
+    assert prc == 0 and len(O.fields_equal(res, want)) == 0
+    assert info["guided"] == 0 and info["settled"] == 56 and info["slow"] == 14, info
+
+
+def test_long_records_of_other_codes_leave_the_chunks_alone(route, port, tmp_path):
+    """Records that the chunk step does not take (more than 256 rows, or errors of more than 1024
+    columns) lie between others': those are settled as without them."""
+    small, long, wide = sparse(60, 100, 9, 1), sparse(300, 400, 3, 2), sparse(40, 3000, 9, 3)
+    cfg = (1, 256, 0, 64, 10, -1)
+    rng = np.random.default_rng(4)
+    recs, codes, errs = [], [], []
+    for i in range(60):
+        k = (0, 0, 0, 1, 0, 2)[i % 6]
+        h = (small, long, wide)[k]
+        e = np.zeros(h.shape[1], np.int32)
+        e[rng.integers(h.shape[1])] = 1
+        errs.append(e)
+        recs.append((h @ e & 1).astype(np.int32) if k == 1 else e)
+        codes.append(k)
+    res, info = decode(route, tmp_path, [((small, 0, 1, cfg, []), {"Ho": small}),
+                                         ((long, 0, 0, cfg, []), {"Ho": long}),
+                                         ((wide, 0, 1, cfg, []), {"Ho": wide})], recs, codes, tables=False)
+    for k, h in enumerate((small, long, wide)):
+        idx = [i for i in range(60) if codes[i] == k]
+        rows = np.stack([recs[i] for i in idx])
+        prc, want, _ = port.css(O.UNIFORM, h, h, None if k == 1 else rows, rows if k == 1 else None,
+                                O.Config(*cfg), "x")
+        assert prc == 0 and len(O.fields_equal(res[idx], want)) == 0
+    assert info["settled"] == 40 and info["slow"] == 20, info
+
+
+@pytest.mark.parametrize("shots", [1, 63, 200])
+def test_plan_of_closed_codes(route, port, tmp_path, shots):
+    """Error records of 300 entries, a closed code: the plan's chunks hold them, so the chunk
+    kernel decodes every shot alone."""
+    h = sparse(60, 300, 3, 5)
+    e = (np.random.default_rng(6).random((shots, 300)) < 0.005).astype(np.int32)
+    cfg = (2, 256, 0, 64, 10, -1)
+    res, info = decode(route, tmp_path, [((h, 0, 1, cfg, []), {"Ho": h})], list(e), [0] * shots)
+    prc, want, _ = port.css(O.UNIFORM, h, h, e, None, O.Config(*cfg), "x")
+    assert prc == 0 and len(O.fields_equal(res, want)) == 0
+    assert info["guided"] == 2 and info["settled"] + info["searched"] == shots, info
