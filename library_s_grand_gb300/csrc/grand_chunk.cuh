@@ -47,10 +47,12 @@ struct alignas(16) FastArea {
   uint32_t row[kMaxChunk][18];
   unsigned long long key[kMaxChunk];    // settled shots: the decoded columns (set_col), row[1] of them
   int shot[kMaxChunk], code[kMaxChunk];
-  int at[kMaxChunk];                    // where its record starts in bits (-1: elsewhere)
+  int at[kMaxChunk];                    // where its record starts in bits (-1: elsewhere, kKept:
+                                        // in the record cache)
   uint8_t state[kMaxChunk];             // 0: open, 1: settled
   uint32_t bits[kFastBallots + 8];      // the run's records, entry after entry (flat_ballots)
 };
+constexpr int kKept = -2;
 constexpr int kRowSketch = kFastWords, kRowWeight = kFastWords + 1, kRowLog = kFastWords + 2;
 static_assert(kRowLog + kFastLogWords <= 18, "an open shot's words fit its row");
 static_assert(sizeof(FastArea) + 4 * kLogBallots <= sizeof(WarpArea),
@@ -147,6 +149,22 @@ __device__ __forceinline__ void bits_to_bytes(unsigned char *out, int n, uint32_
     const uint32_t w = __shfl_sync(kFull, word, c0 >> 5);
     if (c0 + lane < n) out[c0 + lane] = (unsigned char)((w >> lane) & 1u);
   }
+}
+
+// The record of a lane's shot (its bits from entry `at` of F.bits, its logical words from its row)
+// into the record cache, for the per-shot path in place of a second read of the caller's.
+// False: longer than a cache row.
+static __device__ __noinline__ bool keep_record(const DevBatch &b, const HotCode &cd, const FastArea &F,
+                                                int lane, int at, int slot) {
+  const int nbits = cd.input_kind == kInErrors ? cd.m : cd.R, nwords = (nbits + 31) >> 5;
+  const int nlw = cd.family == kDem ? cd.nlw : 0;
+  if (nwords + nlw > kRecCacheWords) return false;
+  uint32_t *cp = b.rec_cache + (size_t)slot * kRecCacheWords;
+#pragma unroll 1
+  for (int q = 0; q < nwords; ++q) cp[q] = flat_word(F.bits, at, q, nbits);
+#pragma unroll 1
+  for (int k = 0; k < nlw; ++k) cp[nwords + k] = F.row[lane][kRowLog + k];
+  return true;
 }
 
 // Classifies the shots of launch slots size * chunk + [0, size), size <= kMaxChunk, into F.
@@ -293,6 +311,7 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
   const unsigned all_starts = __ballot_sync(kFull, mine && (lane == 0 || !pint || pend != rbase));
   const bool one_run = (all_starts & (all_starts - 1u)) == 0u;
   int at = 0;  // where this lane's record starts in the ballots
+  bool kept = false;
   unsigned starts = all_starts;
   bool words = __any_sync(kFull, ok && packed);  // packed records still to be taken
 #pragma unroll 1
@@ -319,7 +338,12 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
       words = false;
       rw = reinterpret_cast<const uint32_t *>(b.in) + rbase;
     }
-    if (in_run && ok) take(at, rw);
+    if (in_run && ok) {
+      take(at, rw);
+      // (the next run's bits take the place of these; a guided search seldom leaves a shot)
+      if (!one_run && !rw && !cd.g_gs && b.rec_cache)
+        kept = keep_record(b, cd, F, lane, at, slot);
+    }
     __syncwarp();  // every lane has read the run's bits before the next run's
   }
   tp = prof_lap(b, kProfChunkRead, tp);
@@ -409,7 +433,7 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
     F.state[lane] = done ? 1 : 0;
     F.key[lane] = found ? (unsigned long long)pos : 0ull;
     // (one run: its bits stay; a later run takes an earlier one's place)
-    F.at[lane] = ok && !packed && one_run ? at : -1;
+    F.at[lane] = ok && !packed && one_run ? at : (kept ? kKept : -1);
   }
   __syncwarp();
   prof_lap(b, kProfChunkWrite, tp);
@@ -472,19 +496,9 @@ __device__ __forceinline__ void write_chunk(const DevBatch &b, const HotCode *ho
   if (slow) {
     base = __shfl_sync(kFull, base, 0) & 0xffffffffull;
     if (open) {
-      // its record's bits for the per-shot path, in place of a second read of the caller's
-      const int ci = F.code[lane];
+      const int ci = F.code[lane], at = F.at[lane];
       const HotCode &cd = hot && ci < kHotCodes ? hot[ci] : static_cast<const HotCode &>(b.codes[ci]);
-      const int nbits = cd.input_kind == kInErrors ? cd.m : cd.R, nwords = (nbits + 31) >> 5;
-      const int nlw = cd.family == kDem ? cd.nlw : 0, at = F.at[lane];
-      const bool cache = b.rec_cache && at >= 0 && nwords + nlw <= kRecCacheWords;
-      if (cache) {
-        uint32_t *cp = b.rec_cache + (size_t)slot * kRecCacheWords;
-#pragma unroll 1
-        for (int q = 0; q < nwords; ++q) cp[q] = flat_word(F.bits, at, q, nbits);
-#pragma unroll 1
-        for (int k = 0; k < nlw; ++k) cp[nwords + k] = F.row[lane][kRowLog + k];
-      }
+      const bool cache = at == kKept || (b.rec_cache && at >= 0 && keep_record(b, cd, F, lane, at, slot));
       // the entry carries this launch's tag: a ticket holder that reads it knows it
       // is not a leftover of an earlier launch
       *reinterpret_cast<volatile unsigned long long *>(b.queue + base + __popc(slow & ((1u << lane) - 1u))) =

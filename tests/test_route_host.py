@@ -122,3 +122,32 @@ def test_plan_of_closed_codes(route, port, tmp_path, shots):
     prc, want, _ = port.css(O.UNIFORM, h, h, e, None, O.Config(*cfg), "x")
     assert prc == 0 and len(O.fields_equal(res, want)) == 0
     assert info["guided"] == 2 and info["settled"] + info["searched"] == shots, info
+
+
+@pytest.mark.parametrize("gap", [0, 1, 3])
+def test_records_of_several_runs_are_kept(route, port, tmp_path, gap):
+    """Requests' records in separate buffers (gap entries between groups of five): the per-shot
+    path finds every record of a chunk in the cache, not those of one run only."""
+    h = sparse(60, 200, 9, 7)
+    dem = synth.random_dem(3, detectors=48, mechanisms=200, logicals=40, col_weights=(8, 9),
+                           p_range=(4e-3, 2e-2))
+    rng = np.random.default_rng(8)
+    e = np.zeros((60, 200), np.int32)
+    for i in range(60):
+        e[i, rng.choice(200, 2, replace=False)] = 1
+    det, log, _ = synth.dem_shots(dem, 60, seed=9)
+    cfg = (2, 256, 0, 64, 10, -1)
+    recs = [r for i in range(60) for r in (e[i], np.concatenate([det[i], log[i]]))]
+    starts, at = [], 0
+    for i, r in enumerate(recs):
+        at += gap if i % 5 == 0 else 0
+        starts.append(at)
+        at += len(r)
+    res, info = decode(route, tmp_path, [((h, 0, 1, cfg, []), {"Ho": h}),
+                                         ((dem.h, 0, 2, cfg, []), {"L": dem.l})],
+                       recs, [0, 1] * 60, np.array(starts))
+    prc, want, _ = port.css(O.UNIFORM, h, h, e, None, O.Config(*cfg), "x")
+    assert prc == 0 and len(O.fields_equal(res[::2], want)) == 0
+    prc, want, *_ = port.dem(O.UNIFORM, dem.h, dem.l, det, log, O.Config(*cfg))
+    assert prc == 0 and len(O.fields_equal(res[1::2], want)) == 0
+    assert info["guided"] == 0 and info["slow"] > 60 and info["cached"] == info["slow"], info
