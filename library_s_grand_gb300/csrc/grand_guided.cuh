@@ -310,7 +310,8 @@ __device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, G
   const bool prob = cd.variant == kProb;
   const int mw = cd.mw, max_cw = cd.g_max_cw;
   const float *llr = ml ? cd.llr : nullptr;
-  const uint32_t hs = row[kRowSketch];
+  // (a group without a shot reads nothing of entry 0's, which its warp may be writing)
+  const uint32_t hs = live ? row[kRowSketch] : 0u;
   if (gl == 0) {
     S.cols = cd.g_cols;
     S.hcol = cd.g_hcol;
@@ -803,7 +804,7 @@ __device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, G
       }
     }
   }
-  const int ow = (int)row[kRowWeight];
+  const int ow = live ? (int)row[kRowWeight] : 0;
   __syncwarp();  // every lane has read the open shot's words
   if (live && gl == 0) {
     const unsigned long long now = global_ns();

@@ -151,3 +151,24 @@ def test_records_of_several_runs_are_kept(route, port, tmp_path, gap):
     prc, want, *_ = port.dem(O.UNIFORM, dem.h, dem.l, det, log, O.Config(*cfg))
     assert prc == 0 and len(O.fields_equal(res[1::2], want)) == 0
     assert info["guided"] == 0 and info["slow"] > 60 and info["cached"] == info["slow"], info
+
+
+def test_no_data_race_between_warps(route, port, tmp_path):
+    """The chunk kernel under the thread sanitizer: blocks whose open shots leave groups of lanes
+    without one (these must not read another warp's shot), chunks that end in every phase."""
+    exe = tmp_path / "host_route_tsan"
+    built = subprocess.run([shutil.which("g++"), "-std=c++20", "-O1", "-g", "-pthread", "-fsanitize=thread",
+                            "-I", os.path.join(ROOT, "library_s_grand_gb300", "csrc"),
+                            "-I", os.path.join(ROOT, "include"), "-I", _cuda_include(), "-I", HERE,
+                            os.path.join(HERE, "host_route.cpp"), "-o", str(exe)],
+                           capture_output=True, text=True)
+    if built.returncode != 0 and "tsan" in built.stderr:
+        pytest.skip("no thread sanitizer library")
+    assert built.returncode == 0, built.stderr
+    code = synth.BB_CODES[72]()
+    cfg = (3, 256, 0, 64, 10, -1)
+    e = synth.css_shots(code.hz, 23, 0.03, seed=3)[0]
+    res, info = decode(str(exe), tmp_path, [((code.hz, 0, 1, cfg, []), {"Ho": code.hx})], list(e), [0] * 23)
+    prc, want, _ = port.css(O.UNIFORM, code.hx, code.hz, e, None, O.Config(*cfg), "x")
+    assert prc == 0 and len(O.fields_equal(res, want)) == 0
+    assert info["guided"] == 2 and info["searched"] > 8, info
