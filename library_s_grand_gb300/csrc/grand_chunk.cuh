@@ -182,8 +182,9 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
                                                    int size, FastArea &F, uint32_t *lbits,
                                                    ChunkStats &st) {
   const int lane = threadIdx.x & 31;
-  const int slot = chunk * size + lane;
-  const bool valid = lane < size && slot < b.num_shots;
+  const int first_slot = chunk * size;  // < num_shots (the sum with a lane need not be an int)
+  const bool valid = lane < size && lane < b.num_shots - first_slot;
+  const int slot = valid ? first_slot + lane : first_slot;
   const unsigned long long t_start = global_ns();
   unsigned long long tp = b.profile ? t_start : 0ull;
   const int shot = valid ? (b.shot_map ? b.shot_map[slot] : slot) : 0;
@@ -216,9 +217,8 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
     // call: every lane has the same code)
     log_ok = !b.shot_map && !packed && b.num_codes == 1;
     if (__any_sync(kFull, ok && dem && log_ok)) {
-      const int first = chunk * size;
-      const int cnt = b.num_shots - first < size ? b.num_shots - first : size;
-      lpad = flat_ballots(b.in_log + (long long)first * cd.n_logicos, cnt * cd.n_logicos, lbits);
+      const int cnt = b.num_shots - first_slot < size ? b.num_shots - first_slot : size;
+      lpad = flat_ballots(b.in_log + (long long)first_slot * cd.n_logicos, cnt * cd.n_logicos, lbits);
       __syncwarp();
     }
   }
@@ -449,8 +449,9 @@ __device__ __forceinline__ unsigned classify_chunk(const DevBatch &b, const HotC
 __device__ __forceinline__ void write_chunk(const DevBatch &b, const HotCode *hot, int chunk, int size,
                                             const FastArea &F, unsigned tag) {
   const int lane = threadIdx.x & 31;
-  const int slot = chunk * size + lane;
-  const bool valid = lane < size && slot < b.num_shots;
+  const int first_slot = chunk * size;
+  const bool valid = lane < size && lane < b.num_shots - first_slot;
+  const int slot = valid ? first_slot + lane : first_slot;
   const bool open = valid && F.state[valid ? lane : 0] == 0;
   const unsigned settled = __ballot_sync(kFull, valid && !open);
   const unsigned slow = __ballot_sync(kFull, open);

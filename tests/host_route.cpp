@@ -6,6 +6,8 @@
 // codes; DEM records are detectors and then logical flips); writes res.bin and prints that
 // program's line, then the plan and what became of the shots.  tables=0: codes without guided
 // tables, so the decode kernel alone.
+#include <sys/mman.h>
+
 #define main host_kernels_main
 #include "host_kernels.cpp"
 #undef main
@@ -25,6 +27,33 @@ static inline int atomicAdd(int *a, int v) { return __atomic_fetch_add(a, v, __A
 
 #include "grand_front.cuh"
 #include "grand_plan.h"
+
+// The last block of a batch of the most shots that an int counts, in address space that only
+// its records and results occupy.
+static int run_edge(const std::string &dir, DevBatch &b, const DevCode &cd, const std::vector<int> &rec) {
+  const size_t all = 0x7fffffff, count = rec.size() / cd.rec_len;
+  auto space = [](size_t bytes) {
+    return (char *)mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+  };
+  char *in = space(all * cd.rec_len * 4), *out = space(all * sizeof(GrandDecoderResult));
+  if (in == MAP_FAILED || out == MAP_FAILED) return 7;
+  memcpy(in + (all - count) * cd.rec_len * 4, rec.data(), 4 * rec.size());
+  b.in = (const int *)in;
+  b.results = (GrandDecoderResult *)out;
+  b.in_off = nullptr;
+  b.shot_code = nullptr;
+  b.num_codes = 1;
+  b.num_shots = (int)all;
+  plan_batch(b, &cd, 1, 152, true);
+  if (b.guided != kGuidedAll) return 8;
+  b.chunk = 27;  // (one that does not divide the batch)
+  gridDim.x = (unsigned)(((all - 1) / b.chunk) / kChunkWarps + 1);
+  blockIdx.x = gridDim.x - 1;
+  run_block(kChunkWarps * 32, [&] { chunk_kernel<false>(b); });
+  if (*b.status) return 4;
+  write_bytes(dir + "/res.bin", out + (all - count) * sizeof(GrandDecoderResult), sizeof(GrandDecoderResult) * count);
+  return 0;
+}
 
 int main(int argc, char **argv) {
   if (argc < 2) return 2;
@@ -103,6 +132,7 @@ int main(int argc, char **argv) {
   b.fast = 1;
   b.light_max_log2 = light;
   b.tile_k = tile_k;
+  if (argc > 2 && !strcmp(argv[2], "edge")) return run_edge(dir, b, dcs[0], rec);
   plan_batch(b, dcs.data(), K, 1, true);
   if (b.guided) {
     gridDim.x = (unsigned)(((N - 1) / b.chunk) / kChunkWarps + 1);

@@ -34,7 +34,7 @@ def sparse(rows, cols, weight, seed):
     return h
 
 
-def decode(exe, d, codes, records, shot_code, starts=None, light=10, tables=True):
+def decode(exe, d, codes, records, shot_code, starts=None, light=10, mode=None):
     """codes: argument tuples of _write_code after the directory, with its keywords; starts: where
     each record begins in the flat records (None: back to back).  Returns the results and the
     numbers of the program's two lines by name."""
@@ -52,9 +52,11 @@ def decode(exe, d, codes, records, shot_code, starts=None, light=10, tables=True
     flat.tofile(d / "rec.bin")
     np.asarray(starts, np.int64).tofile(d / "off.bin")
     np.asarray(shot_code, np.int32).tofile(d / "code.bin")
-    p = subprocess.run([exe, str(d)] + ([] if tables else ["tables=0"]), capture_output=True, text=True,
+    p = subprocess.run([exe, str(d)] + ([mode] if mode else []), capture_output=True, text=True,
                        timeout=600)
     assert p.returncode == 0, (p.returncode, p.stdout, p.stderr)
+    if mode == "edge":
+        return np.fromfile(d / "res.bin", dtype=capi.RESULT_DTYPE)
     first, second = p.stdout.split("\n")[:2]
     w = first.replace(",", "").split()
     info = {"jobs": int(w[3]), "slow": int(w[5])}
@@ -101,7 +103,7 @@ def test_long_records_of_other_codes_leave_the_chunks_alone(route, port, tmp_pat
         codes.append(k)
     res, info = decode(route, tmp_path, [((small, 0, 1, cfg, []), {"Ho": small}),
                                          ((long, 0, 0, cfg, []), {"Ho": long}),
-                                         ((wide, 0, 1, cfg, []), {"Ho": wide})], recs, codes, tables=False)
+                                         ((wide, 0, 1, cfg, []), {"Ho": wide})], recs, codes, mode="tables=0")
     for k, h in enumerate((small, long, wide)):
         idx = [i for i in range(60) if codes[i] == k]
         rows = np.stack([recs[i] for i in idx])
@@ -172,3 +174,15 @@ def test_no_data_race_between_warps(route, port, tmp_path):
     prc, want, _ = port.css(O.UNIFORM, code.hx, code.hz, e, None, O.Config(*cfg), "x")
     assert prc == 0 and len(O.fields_equal(res, want)) == 0
     assert info["guided"] == 2 and info["searched"] > 8, info
+
+
+def test_last_chunk_of_the_largest_batch(route, port, tmp_path):
+    """The last of INT_MAX shots, in a chunk that ends past them: its lanes' slots are not counted
+    beyond the largest int, where they would be taken for shots."""
+    h = sparse(3, 6, 2, 1)
+    # 2^31 - 1 = 27 * 79536431 + 10 shots: the last chunk has 10, its block 10 more chunks' at most
+    syn = (np.random.default_rng(2).random((10, 3)) < 0.5).astype(np.int32)
+    cfg = (2, 256, 0, 64, 10, -1)
+    res = decode(route, tmp_path, [((h, 0, 0, cfg, []), {"Ho": h})], list(syn), [0] * 10, mode="edge")
+    prc, want, _ = port.css(O.UNIFORM, h, h, None, syn, O.Config(*cfg), "x")
+    assert prc == 0 and len(O.fields_equal(res, want)) == 0
