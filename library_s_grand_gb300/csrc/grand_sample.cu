@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kSampleThreads, 1) sample_kernel(DevCode cd, c
                                                                    unsigned long long seed,
                                                                    unsigned long long first_shot, int num_shots,
                                                                    int *records) {
-  __shared__ int s_next;
+  __shared__ unsigned s_next;  // (goes on past the last shot, which can be the largest int)
   extern __shared__ uint4 s_thr[];  // per group of 128 positions and lane: those of 32u + lane
   const int lane = threadIdx.x & 31;
   const int mpad = (cd.m + 127) & ~127;
@@ -124,18 +124,18 @@ __global__ void __launch_bounds__(kSampleThreads, 1) sample_kernel(DevCode cd, c
     asm volatile("" : "+r"(keys[2 * r - 4]), "+r"(keys[2 * r - 3]));
   }
   // the block's shots, drawn by its warps
-  const int last = (int)((long long)num_shots * (blockIdx.x + 1) / gridDim.x);
-  if (threadIdx.x == 0) s_next = (int)((long long)num_shots * blockIdx.x / gridDim.x);
+  const unsigned last = (unsigned)((long long)num_shots * (blockIdx.x + 1) / gridDim.x);
+  if (threadIdx.x == 0) s_next = (unsigned)((long long)num_shots * blockIdx.x / gridDim.x);
   __syncthreads();
   const bool dem = cd.family == kDem;
   const int nw = cd.nw, nlw = dem ? cd.nlw : 0;
 #pragma unroll 1
   for (;;) {
-    int i = 0;
-    if (lane == 0) i = atomicAdd(&s_next, 1);
+    unsigned i = 0;
+    if (lane == 0) i = atomicAdd(&s_next, 1u);
     i = __shfl_sync(kFull, i, 0);
     if (i >= last) break;
-    const unsigned long long shot = first_shot + (unsigned long long)i;
+    const unsigned long long shot = first_shot + i;
     int *rec = records + (size_t)i * cd.rec_len;
     const PhiloxShot half = philox_shot(shot, k0, k1);
     uint32_t s_lane = 0u, l_lane = 0u;  // syndrome / detector word `lane`, logical word `lane`
