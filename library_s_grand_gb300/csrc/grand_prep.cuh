@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(1024, 1) prep_kernel(const DevCode tmpl, const
     S.cw[0][t] = S.cw[1][t] = S.cw[2][t] = 0u;
   }
   if (t == 0) {
-    S.deg = S.max_w = S.max_cw = S.even = S.nonbinary = 0;
+    S.deg = S.max_cw = S.even = S.nonbinary = 0;
+    S.max_w = -0x7fffffff - 1;
     S.min_w = 0x7fffffff;
   }
   __syncthreads();
@@ -151,14 +152,14 @@ __global__ void __launch_bounds__(1024, 1) prep_kernel(const DevCode tmpl, const
       atomicOr(&S.filt[(h >> (32 - kGuidedF)) >> 5], 1u << ((h >> (32 - kGuidedF)) & 31u));
     }
     {  // the block's extremes, one shared atomic per warp (weights biased to stay in order)
-      const unsigned bias = 0x40000000u;
-      const unsigned wu = (unsigned)w + bias;
+      const unsigned bias = 0x80000000u;
+      const unsigned wu = (unsigned)w ^ bias;
       const unsigned hi = __reduce_max_sync(kFull, c < m ? wu : 0u);
       const unsigned lo = __reduce_min_sync(kFull, c < m ? wu : kFull);
       const unsigned oh = __reduce_max_sync(kFull, c < m ? (unsigned)ones : 0u);
-      if (lane == 0 && hi) {
-        atomicMax(&S.max_w, (int)(hi - bias));
-        atomicMin(&S.min_w, (int)(lo - bias));
+      if (lane == 0 && c < m) {
+        atomicMax(&S.max_w, (int)(hi ^ bias));
+        atomicMin(&S.min_w, (int)(lo ^ bias));
         atomicMax(&S.max_cw, (int)oh);
       }
     }
@@ -242,7 +243,7 @@ __global__ void __launch_bounds__(1024, 1) prep_kernel(const DevCode tmpl, const
   }
   if (t == 0) {
     DevCode &d = *out;  // (the template's words were copied at the start)
-    d.max_soma = S.max_w;
+    d.max_soma = S.max_w > 0 ? S.max_w : 0;
     d.regular = S.min_w == S.max_w ? 1 : 0;
     if (ok) {
       d.g_gs = gs;
