@@ -79,6 +79,11 @@ constexpr int kFastLogWords = 4;        // its DEM logical words (n_logicos <= 1
 constexpr int kFastErrWords = 32;       // its error-record words (m <= 1024)
 constexpr int kGuidedLanes = 8;         // lanes that search a shot (a warp searches 32 / 8 at once)
 constexpr int kGuidedItems = 384;       // partial sets a warp's searches hold together
+// (item, neighbour) pairs of a level past which a shot is left to the decode kernel.  Without /
+// with the rule, weight 6 on a 120 x 1000 DEM with rows of up to 58 columns (8192 shots, two
+// of them so long): 384 / 215 us; weight 4 on a 24 x 230 code (256 shots) 414 / 197.  At 4096
+// weight 4 on DEMs gets slower (8192 shots of a 60 x 720 one 119 -> 151 us).
+constexpr int kLevelPairs = 6144;
 constexpr int kHotCodes = 8;            // codes a block of the chunk kernel copies to shared memory
 constexpr int kChunkWarps = 4;          // warps per block of the chunk kernel
 constexpr int kChunkMinBlocks = 4;      // its resident blocks per SM (3 / 4 / 5: mix 93 / 77 / 81 us,

@@ -104,13 +104,15 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
     const int cnt = count - at < take ? count - at : take;
     int r = guided_pass<MLK>(b, hot, A, &areas[0].fast, sizeof(ChunkArea), open + at, cnt);
     st.guided += __popc(r & 255);
-    st.heavy += __popc(r >> 8);
-    if (!r && cnt > 1) {  // levels that outgrow the items together
+    st.heavy += __popc((r >> 8) & 255);
+    if (!(r & 255) && cnt > 1) {  // levels that outgrow the items together
+      const int left = r >> 16;
 #pragma unroll 1
       for (int k = 0; k < cnt; ++k) {
+        if ((left >> k) & 1) continue;
         r = guided_pass<MLK>(b, hot, A, &areas[0].fast, sizeof(ChunkArea), open + at + k, 1);
         st.guided += __popc(r & 255);
-        st.heavy += __popc(r >> 8);
+        st.heavy += __popc((r >> 8) & 255);
       }
     }
   }

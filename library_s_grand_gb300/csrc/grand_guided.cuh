@@ -26,7 +26,9 @@
 // steps whatever the shape of the trees; each new set probes the sketch filter for its
 // last column (weight d + 1) and, while larger weights remain, is kept for the next
 // level.  Shots whose levels together outgrow the items are searched again one by one;
-// one that outgrows them alone takes the general path.
+// one that outgrows them alone takes the general path, and so does one with a level of more
+// than kLevelPairs (item, neighbour) pairs, where a decode kernel follows: its warps share
+// such a search, which this one would walk while the rest of the GPU waits for it.
 //
 // The flagged-check counts (upstream grand_decoder.cu:67-81, 406-416) are formed
 // from the rows: a lane holds a mask word of the columns, the rows of H selected by
@@ -276,11 +278,27 @@ static __device__ __noinline__ uint32_t error_word(const DevBatch &b, const HotC
   return mine;
 }
 
+// The groups whose items among lo .. hi - 1 make more than kLevelPairs pairs, as a mask (rare).
+static __device__ __noinline__ int long_groups(const GuidedArea &A, int lo, int hi, int deg) {
+  const int lane = threadIdx.x & 31;
+  unsigned long long n = 0ull;  // items per group, 16 bits each
+#pragma unroll 1
+  for (int i = lo + lane; i < hi; i += 32) n += 1ull << (16 * (A.item[i].y >> 30));
+#pragma unroll 1
+  for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(kFull, n, o);
+  int mask = 0;
+#pragma unroll 1
+  for (int k = 0; k < 32 / kGuidedLanes; ++k)
+    if ((int)((n >> (16 * k)) & 0xffffu) * deg > kLevelPairs) mask |= 1 << k;
+  return mask;
+}
+
 // cnt (1 .. 4) open shots of the block: the threshold iterations in upstream's order
 // (grand_decoder.cu:1284-1343) until one has a match, and the shot's result into its row.
 // An entry is (warp of the block << 8) | lane of its chunk.  Returns the mask of the shots
-// finished (bit k: entry k; none of them when the levels do not fit), and in bits 8 .. those
-// past the light budget.
+// finished (bit k: entry k; none of them when the levels do not fit), in bits 8 .. those past
+// the light budget, and in bits 16 .. those that a level's length leaves to the decode kernel
+// (then none is finished).
 //
 // Eight lanes (a group) count, plan and report for one shot; the sets are extended by
 // all lanes for all of them.  The groups run in step: every loop goes on while some group
@@ -571,6 +589,10 @@ __device__ __noinline__ int guided_pass(const DevBatch &b, const HotCode *hot, G
         uint32_t bcost = 0xffffffffu;
         const Path none{0xffffffffu, 0xffffffffu};
         const int pairs = d == 0 ? hi : (hi - lo) * deg;
+        if (pairs > kLevelPairs && b.guided != kGuidedAll) {
+          const int left = long_groups(A, lo, hi, deg);
+          if (left) return left << 16;
+        }
         int top = hi, queued = 0;
         bool zeros = false, drained = false;
         int zi = -1;  // an item of residual zero being extended by every active column

@@ -186,3 +186,21 @@ def test_last_chunk_of_the_largest_batch(route, port, tmp_path):
     res = decode(route, tmp_path, [((h, 0, 0, cfg, []), {"Ho": h})], list(syn), [0] * 10, mode="edge")
     prc, want, _ = port.css(O.UNIFORM, h, h, None, syn, O.Config(*cfg), "x")
     assert prc == 0 and len(O.fields_equal(res, want)) == 0
+
+
+@pytest.mark.parametrize("shots", [1, 70])
+def test_long_levels_go_to_the_decode_kernel(route, port, tmp_path, shots):
+    """Columns of weight 5 on 24 rows: sets of three columns make levels of some 18000 pairs.
+    Such a shot is left to the decode kernel's warps; those beside it in the warp are not."""
+    h = sparse(24, 230, 5, 7)
+    rng = np.random.default_rng(3)
+    e = np.zeros((shots, 230), np.int32)
+    for i in range(shots):
+        e[i, rng.choice(230, 4 if i % 23 == 0 else 1 + i % 2, replace=False)] = 1
+    cfg = (4, 256, 0, 230, 10, -1)
+    res, info = decode(route, tmp_path, [((h, 0, 1, cfg, []), {"Ho": h})], list(e), [0] * shots)
+    prc, want, _ = port.css(O.UNIFORM, h, h, e, None, O.Config(*cfg), "x")
+    assert prc == 0 and len(O.fields_equal(res, want)) == 0
+    long = -(-shots // 23)
+    assert info["guided"] == 1 and info["slow"] == long == info["jobs"], info
+    assert info["settled"] + info["searched"] == shots - long, info
