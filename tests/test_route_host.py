@@ -204,3 +204,24 @@ def test_long_levels_go_to_the_decode_kernel(route, port, tmp_path, shots):
     long = -(-shots // 23)
     assert info["guided"] == 1 and info["slow"] == long == info["jobs"], info
     assert info["settled"] + info["searched"] == shots - long, info
+
+
+def test_more_codes_than_a_block_copies(route, port, tmp_path):
+    """Ten codes: the descriptors past the eighth are read from memory, guided and general alike."""
+    bb = synth.BB_CODES[72]()
+    hs = [bb.hz if i % 3 else sparse(60, 100, 9, i) for i in range(10)]
+    cfgs = [(1 + i % 4, 256, 0, 64, 10, (-1, 0, 1)[i % 3]) for i in range(10)]
+    rng = np.random.default_rng(12)
+    which = rng.permutation(np.repeat(np.arange(10), 12))
+    recs = []
+    for k in which:
+        e = np.zeros(hs[k].shape[1], np.int32)
+        e[rng.choice(len(e), int(rng.integers(0, 4)), replace=False)] = 1
+        recs.append(e)
+    res, info = decode(route, tmp_path, [((h, 0, 1, c, []), {"Ho": h}) for h, c in zip(hs, cfgs)], recs, which)
+    for k in range(10):
+        idx = np.nonzero(which == k)[0]
+        prc, want, _ = port.css(O.UNIFORM, hs[k], hs[k], np.stack([recs[i] for i in idx]), None,
+                                O.Config(*cfgs[k]), "x")
+        assert prc == 0 and len(O.fields_equal(res[idx], want)) == 0, k
+    assert info["guided"] == 1 and info["searched"] > 0 and info["slow"] > 0, info
