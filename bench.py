@@ -22,8 +22,7 @@ Reported (one JSON line, rank 0):
              candidate against the measured lop3 rate), above 1 where the guided
              search excludes candidates without forming them;
   roofline_dem  the same figures on the capped DEM stress (random detectors
-             of the 120 x 720 DEM, W = 3, cap 64), at the default and at a tuned
-             light budget;
+             of the 120 x 720 DEM, W = 3, cap 64);
   cpu_baseline  the upstream CPU search algorithm (its C restatement in oracle/,
              or the upstream library itself where it was built) on all host cores.
 
@@ -32,9 +31,11 @@ Reported (one JSON line, rank 0):
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import math
 import os
+import re
 import subprocess
 import sys
 import tempfile
@@ -446,9 +447,31 @@ def run_ours(args):
     return out
 
 
-# DRAM bytes (read + write) of one chunk_kernel launch on the headline batch, from an ncu
-# --set full capture (profiles/chunk_kernel.md).
-HEADLINE_TRAFFIC = 9.527808e6
+# Counts of one chunk_kernel launch each, from ncu --set full captures of these very batches: DRAM
+# bytes (read + write) on the headline batch and on the 192 stress shots, warp instructions
+# on the stress shots and on the 8192 DEM stress shots; and the digest of the kernel's sources
+# they were taken with, so that a line says whether they are this build's.
+CAPTURED_SOURCES = "11c32b3faf304e70"
+HEADLINE_TRAFFIC = 9.530624e6
+STRESS_TRAFFIC = 147712.0
+STRESS_INSTRUCTIONS = 559105
+DEM_STRESS_INSTRUCTIONS = 10085559
+CHUNK_SOURCES = ("grand_chunk.cuh", "grand_common.h", "grand_decode_plain.cu", "grand_device.cuh",
+                 "grand_front.cuh", "grand_guided.cuh", "grand_guided_tables.h", "grand_kernels.cuh",
+                 "grand_plan.h")
+
+
+def chunk_sources():
+    """Digest of what the chunk kernel is built from, comments and blank space left out."""
+    h = hashlib.sha256()
+    for name in CHUNK_SOURCES:
+        with open(os.path.join(ROOT, "library_s_grand_gb300", "csrc", name), encoding="utf-8") as f:
+            h.update(" ".join(re.sub(r"//[^\n]*", "", f.read()).split()).encode())
+    return h.hexdigest()[:16]
+
+
+def counts_of_this_build():
+    return chunk_sources() == CAPTURED_SOURCES
 
 
 def hbm_peak():
@@ -470,17 +493,13 @@ def hbm_streaming(code, dec_ms):
     return {"kernel": "chunk_kernel", "achieved": gbs, "peak": peak, "unit": "GB/s",
             "frac": gbs / peak, "peak_source": src + " copy bandwidth (MEASURED_PEAKS.json)",
             "algorithmic_bytes_per_launch": SHOTS * per_shot, "traffic": HEADLINE_TRAFFIC,
-            "traffic_unit": "bytes per launch (ncu)", "decode_ms": dec_ms,
+            "traffic_unit": "bytes per launch (ncu)", "counts_of_this_build": counts_of_this_build(),
+            "decode_ms": dec_ms,
             "what": "bytes per launch: int32 error records (4m per shot) + 72-byte results"}
 
 
 STRESS_SHOTS = 192
 SKETCH_OPS_PER_CANDIDATE = 1.5  # an enumerating search by column sketches: XOR + half a 3-way min
-# One chunk_kernel launch on the 192 stress shots and on the 8192 DEM stress shots, from ncu
-# --set full captures (profiles/chunk_kernel.md): DRAM bytes and warp instructions.
-STRESS_TRAFFIC = 142080.0
-STRESS_INSTRUCTIONS = 556033
-DEM_STRESS_INSTRUCTIONS = 10054839
 ISSUE_PER_SM_CLOCK = 4  # one warp instruction per scheduler
 SM_CLOCK_HZ = 2.07e9  # the GB300's maximum SM clock (the runs' median clock, bench `clocks`)
 
@@ -539,7 +558,7 @@ def stress_roofline(torch, lib, dev, sp):
             "kernel": "chunk_kernel",
             "workload": f"{n} random-syndrome shots of BB[[144,12,12]], W=4, exhaustive "
                         f"({cands} candidates, 3 threshold iterations)",
-            "instructions": STRESS_INSTRUCTIONS,
+            "instructions": STRESS_INSTRUCTIONS, "counts_of_this_build": counts_of_this_build(),
             "instructions_source": "smsp__inst_executed.sum (ncu capture of the same shots)",
             "search_ms": search_ms, "candidates_per_s": rate,
             "frac_sketch_convention": rate * SKETCH_OPS_PER_CANDIDATE / peak,
@@ -571,7 +590,7 @@ def dem_stress_case(torch, lib, dev, n=STRESS_DEM_SHOTS):
 
 def dem_stress_roofline(torch, lib, dev, sp):
     """Chunk kernel on the capped DEM stress, with the figures of stress_roofline."""
-    from library_s_grand_gb300 import autotune, capi
+    from library_s_grand_gb300 import capi
     n = STRESS_DEM_SHOTS
     wl, eng, d_rec, d_res = dem_stress_case(torch, lib, dev, n)
     cands, ops_fixed, _ = dem_stress_ops(wl.dem.h, wl.detectors, wl.W, wl.cap)
@@ -589,12 +608,6 @@ def dem_stress_roofline(torch, lib, dev, sp):
         return float(np.median(times[1:])), eng.launch_stats(sp)
 
     search_ms, stats = timed()
-    # the same shots with the light budget tuned for them (the guided search only counts
-    # the shots past it)
-    best, table = autotune.tune(eng, "dem-stress", n, d_rec.data_ptr(), d_res.data_ptr(), sp,
-                                use_cache=False, grid=[(l, 4, 0) for l in (10, 12, 14, 16)])
-    tuned_ms, tuned_stats = timed()
-    eng.set_tuning()
     peak = eng.int_peak()
     rate = cands / (search_ms * 1e-3)
     words = math.ceil(wl.dem.n / 32)
@@ -602,7 +615,7 @@ def dem_stress_roofline(torch, lib, dev, sp):
     achieved = DEM_STRESS_INSTRUCTIONS / (search_ms * 1e-3)
     return {"bound": "issue", "achieved": achieved / 1e9, "peak": issue / 1e9,
             "unit": "G warp instructions/s", "frac": achieved / issue, "kernel": "chunk_kernel",
-            "instructions": DEM_STRESS_INSTRUCTIONS,
+            "instructions": DEM_STRESS_INSTRUCTIONS, "counts_of_this_build": counts_of_this_build(),
             "instructions_source": "smsp__inst_executed.sum (ncu capture of the same shots)",
             "workload": f"{n} random-detector shots (Bernoulli 0.36) of the 120 x 720 DEM, "
                         f"grand_decode_cln, W=3, cap 64, exhaustive ({cands} candidates)",
@@ -612,11 +625,7 @@ def dem_stress_roofline(torch, lib, dev, sp):
             "frac_word_convention": rate * (words + 1) / peak,
             "frac_fixed_convention": ops_fixed / (search_ms * 1e-3) / peak,
             "peak_source": "issue: SMs x 4 schedulers x 2.07 GHz; conventions: lop3.b32 issue rate "
-                           "measured on this GPU (grand_measure_int_peak)",
-            "tuned": {"light_log2": best[0], "search_ms": tuned_ms,
-                      "candidates_per_s": cands / (tuned_ms * 1e-3),
-                      "frac": DEM_STRESS_INSTRUCTIONS / (tuned_ms * 1e-3) / issue,
-                      "past_light_budget": int(tuned_stats[2]), "table_ms": table}}
+                           "measured on this GPU (grand_measure_int_peak)"}
 
 
 def _time_device(torch, eng, n, d_rec, d_res, sp, flush, steps, warmup, d_sc=0, d_off=0):

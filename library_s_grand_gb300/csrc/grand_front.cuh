@@ -54,7 +54,9 @@ __global__ void __launch_bounds__(kChunkWarps * 32, kChunkMinBlocks) chunk_kerne
 
   // the codes, and one load per 128-byte line of their tables and of the candidate counts
   // of small sets: the first blocks of an SM find its L1 empty, and this way the lines come
-  // together, in place of one miss after another along the search's chains
+  // together, in place of one miss after another along the search's chains (one shot of
+  // [[144]], waited for: 48.5 us, 51 without; batches of 1, 8 and 16 DEMs of 62 KB, of which
+  // every block touches the first eight's: within 0.5 us of the time without)
   {
     const int n = b.num_codes < kHotCodes ? b.num_codes : kHotCodes;
     constexpr int kWords = (int)(sizeof(HotCode) / 8);
