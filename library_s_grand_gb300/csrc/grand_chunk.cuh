@@ -500,6 +500,10 @@ __device__ __forceinline__ void write_chunk(const DevBatch &b, const HotCode *ho
       const int ci = F.code[lane], at = F.at[lane];
       const HotCode &cd = hot && ci < kHotCodes ? hot[ci] : static_cast<const HotCode &>(b.codes[ci]);
       const bool cache = at == kKept || (b.rec_cache && at >= 0 && keep_record(b, cd, F, lane, at, slot));
+      // The record's bits before the entry, for a ticket holder that reads the entry at once: without
+      // this some read an earlier round's record (6 of 10^6 shots, 5000 a batch, all heavy).
+      // (After a chunk kernel they are read by the next launch.)
+      if (cache && !b.guided) __threadfence();
       // the entry carries this launch's tag: a ticket holder that reads it knows it
       // is not a leftover of an earlier launch
       *reinterpret_cast<volatile unsigned long long *>(b.queue + base + __popc(slow & ((1u << lane) - 1u))) =

@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(kDecodeWarps * 32, kDecodeMinBlocks) decode_ke
               step = kStepShot;
               a0 = v & 0x7fffffffull;
               a1 = (v >> 31) & 1ull;  // the chunk step left the record's bits in rec_cache
+              if (a1) __threadfence();  // (written before the entry)
             } else {
               atomicOr(b.status, kStatusWaitLimit);
             }
