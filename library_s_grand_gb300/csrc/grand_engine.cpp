@@ -243,11 +243,11 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   const int max_jobs = num_shots;
   const size_t scratch_words = 64ull << 20;
   const size_t held[] = {slot->cap_jobs, slot->cap_scratch, slot->cap_small, slot->cap_deferred};
-  cudaError_t r = ensure_zeroed(&slot->d_jobs, &slot->cap_jobs, sizeof(Job) * (size_t)max_jobs);
+  cudaError_t r = ensure_zeroed(&slot->d_jobs, &slot->cap_jobs, sizeof(Job) * (size_t)max_jobs, s);
   if (r == cudaSuccess) r = ensure(&slot->d_scratch, &slot->cap_scratch, scratch_words * 4);
-  if (r == cudaSuccess) r = ensure_zeroed(&slot->d_small, &slot->cap_small, kCtlAllocBytes);
+  if (r == cudaSuccess) r = ensure_zeroed(&slot->d_small, &slot->cap_small, kCtlAllocBytes, s);
   if (r == cudaSuccess)
-    r = ensure_zeroed(&slot->d_deferred, &slot->cap_deferred, shot_buffer_bytes(num_shots));
+    r = ensure_zeroed(&slot->d_deferred, &slot->cap_deferred, shot_buffer_bytes(num_shots), s);
   // launches captured before a buffer was replaced would write where it was
   if (held[0] != slot->cap_jobs || held[1] != slot->cap_scratch || held[2] != slot->cap_small ||
       held[3] != slot->cap_deferred)

@@ -61,12 +61,11 @@ cudaError_t ensure(void **p, size_t *cap, size_t bytes) {
   return e;
 }
 
-cudaError_t ensure_zeroed(void **p, size_t *cap, size_t bytes) {
+cudaError_t ensure_zeroed(void **p, size_t *cap, size_t bytes, cudaStream_t s) {
   const bool enough = *p && *cap >= bytes;
   cudaError_t e = ensure(p, cap, bytes);
-  // (a new allocation may have the old address; done before any other stream's launch)
-  if (e == cudaSuccess && !enough) e = cudaMemset(*p, 0, *cap);
-  if (e == cudaSuccess && !enough) e = cudaStreamSynchronize(nullptr);
+  // (a new allocation may have the old address)
+  if (e == cudaSuccess && !enough) e = cudaMemsetAsync(*p, 0, *cap, s);
   return e;
 }
 
@@ -440,12 +439,12 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
     if (req.h_cost) CK(ensure(&ws->d_cost, &ws->cap_cost, sizeof(float) * N));
   }
   const int max_jobs = std::min(N, 16384);
-  CK(ensure_zeroed(&ws->d_jobs, &ws->cap_jobs, sizeof(Job) * max_jobs));
+  CK(ensure_zeroed(&ws->d_jobs, &ws->cap_jobs, sizeof(Job) * max_jobs, s));
   const size_t scratch_words = 32ull << 20;
   CK(ensure(&ws->d_scratch, &ws->cap_scratch, scratch_words * 4));
   size_t small_cap = ws->d_small ? kCtlAllocBytes : 0;
-  CK(ensure_zeroed(&ws->d_small, &small_cap, kCtlAllocBytes));
-  CK(ensure_zeroed(&ws->d_deferred, &ws->cap_deferred, shot_buffer_bytes(N)));
+  CK(ensure_zeroed(&ws->d_small, &small_cap, kCtlAllocBytes, s));
+  CK(ensure_zeroed(&ws->d_deferred, &ws->cap_deferred, shot_buffer_bytes(N), s));
 
   // Per-call host work is kept to the launches, one status read and one
   // synchronisation; events are recorded only when the caller asks for times,

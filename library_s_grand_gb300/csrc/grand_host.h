@@ -89,9 +89,9 @@ struct Workspace {
 };
 
 cudaError_t ensure(void **p, size_t *cap, size_t bytes);
-// As ensure, and a new allocation starts zeroed (buffers whose entries carry a
-// launch tag: zero is no launch's tag).
-cudaError_t ensure_zeroed(void **p, size_t *cap, size_t bytes);
+// As ensure, and a new allocation starts zeroed, on the stream of the launches that use it
+// (buffers whose entries carry a launch tag: zero is no launch's tag).
+cudaError_t ensure_zeroed(void **p, size_t *cap, size_t bytes, cudaStream_t s);
 
 // The per-shot buffer: re-run flags (int), then, 8-byte aligned, slow-queue entries (u64),
 // then, 16-byte aligned, record-cache rows (kRecCacheWords words each), as many of each
