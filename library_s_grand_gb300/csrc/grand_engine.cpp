@@ -279,7 +279,6 @@ int grand_engine_decode_device(GrandEngine *e, int num_shots, const int *d_shot_
   // record cache pays off only for records read in place from host memory)
   b.rec_cache = nullptr;
   b.epoch = (unsigned *)((char *)slot->d_small + kCtlBytes);
-  b.fast = e->tn.fast;
   b.profile = e->tn.profile;
   b.light_max_log2 = e->tn.light_max_log2;
   b.tile_k = e->tn.tile_k;

@@ -521,7 +521,6 @@ int run_batch(Context *ctx, Workspace *ws, const BatchRequest &req, BatchTiming 
   // chunk step kept instead of a second read over NVLink-C2C
   b.rec_cache = zc ? shot_rec_cache(ws->d_deferred, ws->cap_deferred) : nullptr;
   b.epoch = (unsigned *)((char *)ws->d_small + kCtlBytes);
-  b.fast = tn.fast;
   b.profile = tn.profile;
   b.light_max_log2 = tn.light_max_log2;
   b.tile_k = tn.tile_k;

@@ -196,7 +196,6 @@ cudaError_t start_slot(GrandServer *S, SrvSlot *sl) {
   b.queue = shot_queue(sl->d_deferred, shot_buffer_bytes(S->max_shots));
   b.rec_cache = in_place ? shot_rec_cache(sl->d_deferred, shot_buffer_bytes(S->max_shots)) : nullptr;
   b.epoch = (unsigned *)((char *)sl->d_small + kCtlBytes);
-  b.fast = e->tn.fast;
   b.light_max_log2 = e->tn.light_max_log2;
   b.tile_k = e->tn.tile_k;
   // each slot's decode kernel takes its share of the resident blocks, so the

@@ -225,3 +225,18 @@ def test_more_codes_than_a_block_copies(route, port, tmp_path):
                                 O.Config(*cfgs[k]), "x")
         assert prc == 0 and len(O.fields_equal(res[idx], want)) == 0, k
     assert info["guided"] == 1 and info["searched"] > 0 and info["slow"] > 0, info
+
+
+@pytest.mark.parametrize("shots", [1, 16, 17])
+def test_a_warp_for_every_shot(route, port, tmp_path, shots):
+    """Codes without tables, up to a shot per resident warp (16 on the plan's one SM): no chunk step;
+    one shot more and empty records are settled there."""
+    h = sparse(60, 120, 9, 13)
+    e = np.zeros((shots, 120), np.int32)
+    for i in range(shots):
+        e[i, :i % 3] = 1
+    cfg = (2, 256, 0, 64, 10, -1)
+    res, info = decode(route, tmp_path, [((h, 0, 1, cfg, []), {"Ho": h})], list(e), [0] * shots)
+    prc, want, _ = port.css(O.UNIFORM, h, h, e, None, O.Config(*cfg), "x")
+    assert prc == 0 and len(O.fields_equal(res, want)) == 0
+    assert info["guided"] == 0 and info["slow"] == (shots if shots <= 16 else 5), info
