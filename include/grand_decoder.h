@@ -44,7 +44,9 @@ extern "C" {
 /* Error codes beyond the upstream -1. */
 #define GRAND_ERR_INVALID   (-1) /* same cases as upstream (bad type, weight, file) */
 #define GRAND_ERR_CUDA      (-2) /* a CUDA call failed; message on stderr            */
-#define GRAND_ERR_LIMIT     (-3) /* a size is beyond what the kernels support        */
+#define GRAND_ERR_LIMIT     (-3) /* a size is beyond what the kernels support, or a shot's
+                                    search alone outgrows the scratch arena (its result is
+                                    zero, the other shots' results stand)               */
 #define GRAND_ERR_CANCELLED (-4) /* a server request was cancelled                   */
 
 /* Upstream grand_decoder.h:37-44 (24 bytes). */

@@ -82,7 +82,8 @@ constexpr int kGuidedItems = 384;       // partial sets a warp's searches hold t
 // (item, neighbour) pairs of a level past which a shot is left to the decode kernel.  Without /
 // with the rule, weight 6 on a 120 x 1000 DEM with rows of up to 58 columns (8192 shots, two
 // of them so long): 384 / 215 us; weight 4 on a 24 x 230 code (256 shots) 414 / 197.  At 4096
-// weight 4 on DEMs gets slower (8192 shots of a 60 x 720 one 119 -> 151 us).
+// weight 4 on DEMs gets slower (8192 shots of a 60 x 720 one 119 -> 151 us).  Batches that cannot
+// leave a shot pay for the test: headline 28.9 us, 28.7 without, noisy [[288]] 52.4 and 51.6.
 constexpr int kLevelPairs = 6144;
 constexpr int kHotCodes = 8;            // codes a block of the chunk kernel copies to shared memory
 constexpr int kChunkWarps = 4;          // warps per block of the chunk kernel

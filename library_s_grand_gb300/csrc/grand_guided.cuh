@@ -40,8 +40,8 @@
 // trips among them) and the instruction caches.  Most of a shot's instructions are
 // uniform -- planning, loop control, reductions -- so eight lanes take a shot and a
 // warp takes four, in step; the code is kept small: loops stay rolled, column widths
-// are a run-time choice and the rare parts are out of line.  Headline batch 28.7 us, mix of
-// 100000 shots 61, noisy [[288]] 50.5, random detectors of the 720-mechanism DEM 24.6; with
+// are a run-time choice and the rare parts are out of line.  Headline batch 28.9 us, mix of
+// 100000 shots 60, noisy [[288]] 51, random detectors of the 720-mechanism DEM 24.5; with
 // a shot per warp 43.7, 112, 88 and 34, in the decode kernel alone 82, 237, 939 and 568.
 #pragma once
 
